@@ -153,11 +153,11 @@ void heff_apply(const T* Lenv, const T* Renv, const T* WWt, const T* in, T* out,
   const ll dd = (ll)d * d;
   {
     Gemm<T> g;
-    g.M = cL; g.N = (int)(dd * cR); g.K = cL;
-    g.A = Lenv; g.lda = (ll)Dl * cL; g.sA1 = cL;
-    g.B = in; g.ldb = dd * cR; g.sB1 = 0;
-    g.C = X; g.ldc = (ll)Dl * dd * cR; g.sC1 = dd * cR;
-    g.nb1 = Dl; g.skip = skip;
+    g.M = cL * Dl; g.N = (int)(dd * cR); g.K = cL;  // rows (a, w)
+    g.A = Lenv; g.lda = cL;
+    g.B = in; g.ldb = dd * cR;
+    g.C = X; g.ldc = dd * cR;
+    g.skip = skip;
     launch_gemm(g, s);
   }
   mix_rows(X, WWt, Y, cL, cR, (int)(Dl * dd), (int)(dd * Dr), skip, s, wsp);
@@ -169,16 +169,6 @@ void heff_apply(const T* Lenv, const T* Renv, const T* WWt, const T* in, T* out,
     g.B = Renv; g.ldb = (ll)Dr * cR;
     g.C = out; g.ldc = cR;
     g.skip = skip;
-    // split K when the output tiles cannot fill the GPU; X is free again and
-    // holds Dl * cL * d^2 * cR >= splitk * cL * d^2 * cR partial products
-    const int tiles = ceil_div(g.M, GemmTile<T>::BM) * ceil_div(g.N, GemmTile<T>::BN);
-    int sk = 1;
-    while (sk < Dl && sk < 8 && tiles * sk < 2 * 148 && (ll)g.K / (sk * 2) >= 4 * GemmTile<T>::BK) sk *= 2;
-    if (sk > Dl) sk = Dl;
-    if (sk > 1) {
-      g.splitk = sk;
-      g.ws = X;
-    }
     launch_gemm(g, s);
   }
 }
@@ -188,11 +178,11 @@ void heff1_apply(const T* Lenv, const T* Renv, const T* WmixL, const T* in, T* o
                  int d, int Dl, int Dr, const int* skip, cudaStream_t s) {
   {
     Gemm<T> g;  // X[a][w][(s,e)] = sum_c L[a][w][c] A[c][(s,e)]
-    g.M = cL; g.N = d * cR; g.K = cL;
-    g.A = Lenv; g.lda = (ll)Dl * cL; g.sA1 = cL;
-    g.B = in; g.ldb = (ll)d * cR; g.sB1 = 0;
-    g.C = X; g.ldc = (ll)Dl * d * cR; g.sC1 = (ll)d * cR;
-    g.nb1 = Dl; g.skip = skip;
+    g.M = cL * Dl; g.N = d * cR; g.K = cL;
+    g.A = Lenv; g.lda = cL;
+    g.B = in; g.ldb = (ll)d * cR;
+    g.C = X; g.ldc = (ll)d * cR;
+    g.skip = skip;
     launch_gemm(g, s);
   }
   mix_rows(X, WmixL, Y, cL, cR, Dl * d, d * Dr, skip, s);  // Y[a][(t,w')][e]
@@ -204,14 +194,6 @@ void heff1_apply(const T* Lenv, const T* Renv, const T* WmixL, const T* in, T* o
     g.B = Renv; g.ldb = (ll)Dr * cR;
     g.C = out; g.ldc = cR;
     g.skip = skip;
-    const int tiles = ceil_div(g.M, GemmTile<T>::BM) * ceil_div(g.N, GemmTile<T>::BN);
-    int sk = 1;
-    while (sk < Dl && sk < 8 && tiles * sk < 2 * 148 && (ll)g.K / (sk * 2) >= 4 * GemmTile<T>::BK) sk *= 2;
-    if (sk > Dl) sk = Dl;
-    if (sk > 1) {
-      g.splitk = sk;
-      g.ws = X;  // X holds Dl * cL * d * cR >= splitk * cL * d * cR partial products
-    }
     launch_gemm(g, s);
   }
 }
@@ -235,21 +217,6 @@ double env_flops(int ci, int co, int d, int Dl, int Dr, bool cplx) {
   return cplx ? 4.0 * f : f;
 }
 
-// split the K range of an environment GEMM over CTAs when its output tiles do not fill
-// the GPU, with ws (room for ws_elems elements) as the partial-product workspace
-template <typename T>
-static void env_splitk(Gemm<T>& g, ll ws_elems, T* ws) {
-  const int tiles = ceil_div(g.M, GemmTile<T>::BM) * ceil_div(g.N, GemmTile<T>::BN);
-  int sk = 1;
-  while (sk < 8 && tiles * sk < 148 && (ll)g.K / (2 * sk) >= 4 * GemmTile<T>::BK &&
-         (ll)(2 * sk) * g.M * g.N <= ws_elems)
-    sk *= 2;
-  if (sk > 1) {
-    g.splitk = sk;
-    g.ws = ws;
-  }
-}
-
 template <typename T>
 void env_left(const T* Lenv, const T* A, const T* WmixL, T* Lnew, T* X, T* Y, int cL, int cO, int d,
               int Dl, int Dr, cudaStream_t s) {
@@ -271,9 +238,6 @@ void env_left(const T* Lenv, const T* A, const T* WmixL, T* Lnew, T* X, T* Y, in
     g.A = A; g.lda = cO;
     g.B = Y; g.ldb = (ll)Dr * cO;
     g.C = Lnew; g.ldc = (ll)Dr * cO;
-    // K split when the output tiles cannot fill the GPU; X (free again) holds the
-    // cL Dl d cO products of step 1
-    env_splitk(g, (ll)cL * Dl * d * cO, X);
     launch_gemm(g, s);
   }
 }
@@ -301,20 +265,17 @@ void env_right(const T* Renv, const T* B, const T* WmixR, T* Rnew, T* X, T* Y, i
     g.A = B; g.lda = (ll)d * cI;
     g.B = Y; g.ldb = (ll)Dl * cO;
     g.C = Rnew; g.ldc = (ll)Dl * cO;
-    env_splitk(g, (ll)cI * Dr * d * cO, X);  // X holds the cI Dr d cO products of step 1
     launch_gemm(g, s);
   }
 }
 
 template <typename T>
-void theta_form(const T* A, const T* B, T* theta, int cL, int cM, int cR, int d, cudaStream_t s, T* ws,
-                ll ws_elems) {
+void theta_form(const T* A, const T* B, T* theta, int cL, int cM, int cR, int d, cudaStream_t s) {
   Gemm<T> g;
   g.M = cL * d; g.N = d * cR; g.K = cM;
   g.A = A; g.lda = cM;
   g.B = B; g.ldb = (ll)d * cR;
   g.C = theta; g.ldc = (ll)d * cR;
-  if (ws) env_splitk(g, ws_elems, ws);
   launch_gemm(g, s);
 }
 
@@ -377,7 +338,7 @@ void build_wmix_right(const T* W, int Dl, int Dr, int d, std::vector<T>& out) {
                             cudaStream_t);                                                       \
   template void env_right<T>(const T*, const T*, const T*, T*, T*, T*, int, int, int, int, int, \
                              cudaStream_t);                                                      \
-  template void theta_form<T>(const T*, const T*, T*, int, int, int, int, cudaStream_t, T*, ll); \
+  template void theta_form<T>(const T*, const T*, T*, int, int, int, int, cudaStream_t);        \
   template void build_wwt<T>(const T*, const T*, int, int, int, int, std::vector<T>&);          \
   template void build_wmix_left<T>(const T*, int, int, int, std::vector<T>&);                   \
   template void build_wmix_right<T>(const T*, int, int, int, std::vector<T>&);

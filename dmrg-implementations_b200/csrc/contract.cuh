@@ -18,7 +18,7 @@
 namespace dmrg2 {
 
 // H_eff matvec (reference: apply_heff_two_site, dmrg2_gpu_impl.h:607-780)
-//   step 1: X[a][w][s][r][e] = sum_c L[a][w][c] theta[c][s][r][e]      (Dl batches)
+//   step 1: X[a][w][s][r][e] = sum_c L[a][w][c] theta[c][s][r][e]      (one GEMM, rows (a, w))
 //   step 2: Y[a][p][q][n][e] = sum_{w,s,r} WWt[(p,q,n)][(w,s,r)] X[a][w][s][r][e]  (cL batches)
 //   step 3: out[a][p][q][f]  = sum_{n,e} Y[a][p][q][n][e] R[f][n][e]  (one GEMM, K = Dr*cR)
 //
@@ -72,9 +72,7 @@ void env_right(const T* Renv, const T* B, const T* WmixR, T* Rnew, T* X, T* Y, i
 
 // theta = A_i . A_{i+1} (reference: form_theta_two_site, dmrg2_gpu_impl.h:583-600)
 template <typename T>
-// theta = A B; ws (ws_elems elements, optional) lets a GEMM with few output tiles split K
-void theta_form(const T* A, const T* B, T* theta, int cL, int cM, int cR, int d, cudaStream_t s, T* ws = nullptr,
-                ll ws_elems = 0);
+void theta_form(const T* A, const T* B, T* theta, int cL, int cM, int cR, int d, cudaStream_t s);
 
 // host-side MPO preprocessing (reference: set_mpo / precompute_fused_mpo, dmrg2_gpu_impl.h:436-576)
 template <typename T>

@@ -482,7 +482,7 @@ class Engine final : public EngineBase {
     const int cL = dims_[bs], cM = dims_[bs + 1], cR = dims_[bs + 2];
     const ll m = (ll)cL * d_, nc = (ll)d_ * cR;
     row_scale<T>(mps_[bs + 1], V, cM, nc, l.svdX, false, l.st);  // diag(V) psi_R
-    theta_form(mps_[bs], l.svdX, l.theta, cL, cM, cR, d_, l.st, l.X, xs_);
+    theta_form(mps_[bs], l.svdX, l.theta, cL, cM, cR, d_, l.st);
     const double e = lanczos(bs, m * nc, ss);
     DMRG2_CUDA(cudaEventRecord(l.ev_c, l.st));
     DMRG2_CUDA(cudaMemcpyAsync(l.svdX, l.theta, sizeof(T) * (size_t)(m * nc), cudaMemcpyDeviceToDevice, l.st));
@@ -733,7 +733,7 @@ class Engine final : public EngineBase {
   double optimize_bond(int i, char dir, int chi, SweepStats& ss) {
     const int cL = dims_[i], cM = dims_[i + 1], cR = dims_[i + 2];
     const ll n = (ll)cL * d_ * d_ * cR;
-    theta_form(mps_[i], mps_[i + 1], ln().theta, cL, cM, cR, d_, ln().st, ln().X, xs_);
+    theta_form(mps_[i], mps_[i + 1], ln().theta, cL, cM, cR, d_, ln().st);
     double e = lanczos(i, n, ss);
     svd_split(i, dir, chi, ss);
     if (dir == 'R')

@@ -1,4 +1,6 @@
 // Host launcher and instantiations of the DMMA GEMM.
+#include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -114,41 +116,11 @@ bool test_unsignalled_waits() {
   return on;
 }
 
-template <typename T>
-__global__ void splitk_reduce_kernel(const T* __restrict__ ws, int ns, int M, int N, double ar,
-                                     double ai, double br, double bi, T* __restrict__ C, ll ldc,
-                                     const int* skip) {
-  if (skip && *((volatile const int*)skip)) return;
-  const ll tot = (ll)M * N;
-  const T alpha = ST<T>::make(ar, ai), beta = ST<T>::make(br, bi);
-  const bool use_beta = (br != 0.0 || bi != 0.0);
-  for (ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (ll)gridDim.x * blockDim.x) {
-    T acc = ws[t];
-    for (int z = 1; z < ns; ++z) acc = acc + ws[(ll)z * tot + t];
-    const ll m = t / N, n = t % N;
-    T* c = C + m * ldc + n;
-    T v = ST<T>::mul(alpha, acc);
-    if (use_beta) v = v + ST<T>::mul(beta, *c);
-    *c = v;
-  }
-}
-
-template <typename T>
-static void splitk_reduce(const T* ws, int ns, int M, int N, T alpha, T beta, T* C, ll ldc,
-                          const int* skip, cudaStream_t st) {
-  ll tot = (ll)M * N;
-  ll g = (tot + 255) / 256;
-  if (g > 148 * 8) g = 148 * 8;
-  splitk_reduce_kernel<T><<<(int)(g < 1 ? 1 : g), 256, 0, st>>>(ws, ns, M, N, ST<T>::re(alpha), ST<T>::im(alpha),
-                                                          ST<T>::re(beta), ST<T>::im(beta), C, ldc, skip);
-  DMRG2_CHECK_LAUNCH();
-}
-
-template <typename T, typename G, bool TA, bool TB, bool CA>
+template <typename T, typename G, bool TA, bool TB, bool CA, bool VA, bool VB>
 static void launch_impl(const Gemm<T>& d, int splitk, cudaStream_t st) {
   using S = GemmSmem<T, G, TA, TB>;
   static std::atomic<unsigned long long> attr{0};  // per instantiation, per device
-  set_smem_attr_once(attr, (const void*)gemm_kernel<T, G, TA, TB, CA>, (int)S::BYTES);
+  set_smem_attr_once(attr, (const void*)gemm_kernel<T, G, TA, TB, CA, VA, VB>, (int)S::BYTES);
   GemmArgs a;
   a.M = d.M; a.N = d.N; a.K = d.K;
   a.A = d.A; a.lda = d.lda; a.sA1 = d.sA1; a.sA2 = d.sA2;
@@ -158,76 +130,146 @@ static void launch_impl(const Gemm<T>& d, int splitk, cudaStream_t st) {
   a.alpha_re = ST<T>::re(d.alpha); a.alpha_im = ST<T>::im(d.alpha);
   a.beta_re = ST<T>::re(d.beta); a.beta_im = ST<T>::im(d.beta);
   a.skip = d.skip;
+  a.Cin = d.Cin;
   a.kchunk = 0;
   a.kcluster = 0;
-  if (splitk > 1) {
-    const int chunk = ceil_div(ceil_div(d.K, splitk), G::BK) * G::BK;
-    const int nsplit = ceil_div(d.K, chunk);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ceil_div(d.N, G::BN), ceil_div(d.M, G::BM), d.nb1 * d.nb2);
+  cfg.blockDim = dim3(G::THREADS);
+  cfg.dynamicSmemBytes = S::BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  constexpr int BK = S::TileA::BK;
+  const int chunk = ceil_div(ceil_div(d.K, splitk), BK) * BK;
+  const int nsplit = ceil_div(d.K, chunk);
+  if (nsplit > 1) {
+    // the slices of a tile form one cluster and are summed in it, in slice order: no
+    // workspace, no second launch
     a.kchunk = chunk;
+    a.kcluster = nsplit;
     a.sA1 = a.sA2 = a.sB1 = a.sB2 = a.sC1 = a.sC2 = 0;
     a.nb2 = 1;
-    if (nsplit > 1 && nsplit <= 8) {
-      // the slices of a tile form one cluster and are summed in it: no workspace, no
-      // second launch, the same summation order as the reduction kernel
-      a.kcluster = nsplit;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(ceil_div(d.N, G::BN), ceil_div(d.M, G::BM), nsplit);
-      cfg.blockDim = dim3(G::THREADS);
-      cfg.dynamicSmemBytes = S::BYTES;
-      cfg.stream = st;
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = 1;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = nsplit;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      DMRG2_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<T, G, TA, TB, CA>, a));
-      DMRG2_CHECK_LAUNCH();
-      return;
-    }
-    if (nsplit > 8) {
-      // more slices than a portable cluster: partial products per K slice into ws[z]
-      // (M x N, ld N), then one reduction
-      if (!d.ws) throw std::runtime_error("gemm: more than 8 K slices need a workspace");
-      a.C = d.ws; a.ldc = d.N; a.sC1 = (ll)d.M * d.N; a.sC2 = 0;
-      a.alpha_re = 1.0; a.alpha_im = 0.0; a.beta_re = 0.0; a.beta_im = 0.0;
-      dim3 grid(ceil_div(d.N, G::BN), ceil_div(d.M, G::BM), nsplit);
-      gemm_kernel<T, G, TA, TB, CA><<<grid, G::THREADS, S::BYTES, st>>>(a);
-      DMRG2_CHECK_LAUNCH();
-      splitk_reduce<T>(d.ws, nsplit, d.M, d.N, d.alpha, d.beta, d.C, d.ldc, d.skip, st);
-      return;
-    }
-    a.kchunk = 0;  // one slice
+    cfg.gridDim.z = nsplit;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = nsplit;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
   }
-  dim3 grid(ceil_div(d.N, G::BN), ceil_div(d.M, G::BM), d.nb1 * d.nb2);
-  gemm_kernel<T, G, TA, TB, CA><<<grid, G::THREADS, S::BYTES, st>>>(a);
+  DMRG2_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<T, G, TA, TB, CA, VA, VB>, a));
   DMRG2_CHECK_LAUNCH();
+}
+
+// whether every row of an operand starts on 16 bytes
+template <typename T>
+static bool rows16(const T* p, ll ld, ll s1, ll s2) {
+  return sizeof(T) == 16 || (((ld | s1 | s2) & 1) == 0 && ((uintptr_t)p & 15) == 0);
+}
+
+template <typename T, typename G, bool TA, bool TB, bool CA>
+static void launch_vec(const Gemm<T>& d, int splitk, cudaStream_t st) {
+  if constexpr (ST<T>::cplx) {
+    launch_impl<T, G, TA, TB, CA, true, true>(d, splitk, st);
+  } else {
+    const bool va = rows16(d.A, d.lda, d.sA1, d.sA2), vb = rows16(d.B, d.ldb, d.sB1, d.sB2);
+    if (va && vb) launch_impl<T, G, TA, TB, CA, true, true>(d, splitk, st);
+    else if (va) launch_impl<T, G, TA, TB, CA, true, false>(d, splitk, st);
+    else if (vb) launch_impl<T, G, TA, TB, CA, false, true>(d, splitk, st);
+    else launch_impl<T, G, TA, TB, CA, false, false>(d, splitk, st);
+  }
 }
 
 template <typename T, typename G>
 static void dispatch(const Gemm<T>& d, int splitk, cudaStream_t st) {
   const bool ca = ST<T>::cplx && d.ca;
-  if (!d.ta && !d.tb && !ca) return launch_impl<T, G, false, false, false>(d, splitk, st);
-  if (!d.ta && d.tb && !ca) return launch_impl<T, G, false, true, false>(d, splitk, st);
-  if (d.ta && !d.tb && !ca) return launch_impl<T, G, true, false, false>(d, splitk, st);
-  if (d.ta && d.tb && !ca) return launch_impl<T, G, true, true, false>(d, splitk, st);
+  if (!d.ta && !d.tb && !ca) return launch_vec<T, G, false, false, false>(d, splitk, st);
+  if (!d.ta && d.tb && !ca) return launch_vec<T, G, false, true, false>(d, splitk, st);
+  if (d.ta && !d.tb && !ca) return launch_vec<T, G, true, false, false>(d, splitk, st);
+  if (d.ta && d.tb && !ca) return launch_vec<T, G, true, true, false>(d, splitk, st);
   if constexpr (ST<T>::cplx) {
-    if (!d.ta && !d.tb) return launch_impl<T, G, false, false, true>(d, splitk, st);
-    if (!d.ta && d.tb) return launch_impl<T, G, false, true, true>(d, splitk, st);
-    if (d.ta && !d.tb) return launch_impl<T, G, true, false, true>(d, splitk, st);
-    return launch_impl<T, G, true, true, true>(d, splitk, st);
+    if (!d.ta && !d.tb) return launch_vec<T, G, false, false, true>(d, splitk, st);
+    if (!d.ta && d.tb) return launch_vec<T, G, false, true, true>(d, splitk, st);
+    if (d.ta && !d.tb) return launch_vec<T, G, true, false, true>(d, splitk, st);
+    return launch_vec<T, G, true, true, true>(d, splitk, st);
   }
 }
 
+namespace {
+struct GemmChoice {
+  int tile;    // index into the tiles of the scalar type (launch_choice)
+  int splitk;  // K slices (a cluster of at most 8)
+};
+
+// Tile and K split by a model of the busiest SM. It runs q = ceil(CTAs / 148) tiles of
+// BM BN K / splitk multiply-adds; the tensor pipe takes 64 (16 complex) a cycle, but only with
+// enough warps resident to cover the latency of a warp's dependent multiply-adds: the
+// measured share of the rate is 0.62 with 4 warps on the SM, 0.82 with 8, 0.86 with 12, 0.90
+// with 16 and 0.92 beyond (L2-resident operands, K from 64 to 1280). A split costs about 1600
+// cycles per CTA of the SM (cluster barrier, exchange of partial tiles); an operand whose rows
+// do not start on 16 bytes about 8 cycles per 32 values (twice the copies, half the bytes). Measured against
+// the model's choice, M x N x K: 1280 x 1024 x 256 (64 x 64 tiles: 2.16 CTAs an SM run as
+// three, 35.2 us; 64 x 32 28.9; 32 x 32 26.9), 1024 x 256 x 1280 (64 x 64 tiles in 5 slices
+// 37.1; 4 slices 30.0; 32 x 32 unsplit 28.9), 512 x 128 x 640 (64 x 64 in 8 slices 12.4;
+// 32 x 32 unsplit 14.5, in 4 slices 8.4), 320 x 256 x 64 (64 x 64 6.4; 32 x 32 4.3).
+struct TileModel {
+  int bm, bn;
+  int occ;  // CTAs an SM holds (four warps each)
+};
+constexpr TileModel TILES_D[] = {{64, 64, 3}, {64, 32, 4}, {32, 32, 6}};
+constexpr TileModel TILES_Z[] = {{64, 32, 4}, {32, 32, 6}};
+
+template <typename T>
+GemmChoice choose(const Gemm<T>& d) {
+  constexpr double share[] = {0.62, 0.82, 0.86, 0.90, 0.92, 0.92};
+  const TileModel* tiles = ST<T>::cplx ? TILES_Z : TILES_D;
+  const int nt = ST<T>::cplx ? 2 : 3;
+  const double rate = ST<T>::cplx ? 16.0 : 64.0;
+  const int bk = ST<T>::cplx ? 8 : 16;
+  const int nb = d.nb1 * d.nb2;
+  const double narrow_a = rows16(d.A, d.lda, d.sA1, d.sA2) ? 0.0 : 8.0 / 32;
+  const double narrow_b = rows16(d.B, d.ldb, d.sB1, d.sB2) ? 0.0 : 8.0 / 32;
+  GemmChoice best{0, 1};
+  double best_t = 1e300;
+  for (int t = 0; t < nt; ++t) {
+    const double out = (double)ceil_div(d.M, tiles[t].bm) * ceil_div(d.N, tiles[t].bn) * nb;
+    for (int sk = 1; sk <= (nb == 1 ? 8 : 1); ++sk) {
+      if (sk > 1 && ceil_div(d.K, sk) < 2 * bk) break;  // at least two k tiles per slice
+      const int kc = ceil_div(ceil_div(d.K, sk), bk) * bk, ns = ceil_div(d.K, kc);
+      if (ns < sk) continue;
+      const double q = std::ceil(out * ns / 148.0);
+      const double f = share[std::min((int)std::min(q, 6.0), tiles[t].occ) - 1];
+      const double time = q * (tiles[t].bm * tiles[t].bn * (double)kc / rate / f + (ns > 1 ? 1600.0 : 0.0) +
+                               kc * (narrow_a * tiles[t].bm + narrow_b * tiles[t].bn));
+      if (time < best_t) {
+        best_t = time;
+        best = {t, ns};
+      }
+    }
+  }
+  return best;
+}
+
+template <typename T>
+void launch_choice(const Gemm<T>& d, const GemmChoice& c, cudaStream_t st) {
+  if constexpr (ST<T>::cplx) {
+    if (c.tile == 0) dispatch<T, TileZ64>(d, c.splitk, st);
+    else dispatch<T, TileZ32>(d, c.splitk, st);
+  } else {
+    if (c.tile == 0) dispatch<T, TileD64>(d, c.splitk, st);
+    else if (c.tile == 1) dispatch<T, TileD64x32>(d, c.splitk, st);
+    else dispatch<T, TileD32>(d, c.splitk, st);
+  }
+}
+}  // namespace
+
 // ---------------------------------------------------------------- autotuner
-// A single real GEMM of at least TUNE_MIN_FLOP is run in each configuration (64 x 64
-// tiles with 1, 2, 4 or 8 K slices reduced in a cluster; 32 x 32 tiles with 1, 2 or 4)
+// A single real GEMM of at least TUNE_MIN_FLOP is run in each configuration (every tile
+// with 1, 2, 4 or 8 K slices)
 // the first time its shape (transposes, M, N, K) occurs in the process, on the caller's
 // stream and operands, writing into a scratch output (never the caller's C, no skip
 // flag); the fastest by CUDA events serves every later GEMM of that shape. Smaller GEMMs
-// are latency-bound and keep the default (64 x 64 tiles, the caller's K split): their
-// many distinct shapes (chain ends, bond-dimension ramps) would cost more to time than
+// are latency-bound and keep the model's choice: their many distinct shapes (chain ends, bond-dimension ramps) would cost more to time than
 // a configuration can save. The tuning is off unless DMRG2_GEMM_TUNE=1: measured on the
 // L=100, chi=256 sweep it gains 2% on steady sweeps but loses 10% on a run that starts
 // from a fresh engine (the choices timed in isolation, on L2-resident operands, do not
@@ -245,17 +287,13 @@ struct TuneKeyHash {
     return h ^ (size_t)(k.ta * 2 + k.tb) ^ ((size_t)k.dev << 40);
   }
 };
-struct TuneChoice {
-  int tile;   // 0: TileD64, 1: TileD32
-  int splitk;
-};
 constexpr double TUNE_MIN_FLOP = 1e8;
 std::mutex& tune_mutex() {
   static std::mutex m;
   return m;
 }
-std::unordered_map<TuneKey, TuneChoice, TuneKeyHash>& tune_cache() {
-  static auto* c = new std::unordered_map<TuneKey, TuneChoice, TuneKeyHash>();
+std::unordered_map<TuneKey, GemmChoice, TuneKeyHash>& tune_cache() {
+  static auto* c = new std::unordered_map<TuneKey, GemmChoice, TuneKeyHash>();
   return *c;
 }
 }  // namespace
@@ -269,7 +307,7 @@ bool tune_enabled() {
 }
 
 namespace {
-TuneChoice tuned(const Gemm<double>& d, cudaStream_t st) {
+GemmChoice tuned(const Gemm<double>& d, cudaStream_t st) {
   int dev = 0;
   DMRG2_CUDA(cudaGetDevice(&dev));
   const TuneKey key{d.ta ? 1 : 0, d.tb ? 1 : 0, d.M, d.N, d.K, dev};
@@ -278,21 +316,20 @@ TuneChoice tuned(const Gemm<double>& d, cudaStream_t st) {
   if (it != tune_cache().end()) return it->second;
   Gemm<double> t = d;
   t.skip = nullptr;
+  t.Cin = nullptr;
+  t.beta = 0.0;
   t.ldc = d.N;
   t.sC1 = t.sC2 = 0;
   t.C = (double*)dev_alloc(sizeof(double) * (size_t)d.M * d.N);
   cudaEvent_t e0, e1;
   DMRG2_CUDA(cudaEventCreate(&e0));
   DMRG2_CUDA(cudaEventCreate(&e1));
-  TuneChoice best{0, 1};
+  GemmChoice best{0, 1};
   float best_ms = 1e30f;
-  for (int tile = 0; tile < 2; ++tile)
-    for (int sk = 1; sk <= (tile == 0 ? 8 : 4); sk *= 2) {
+  for (int tile = 0; tile < 3; ++tile)
+    for (int sk = 1; sk <= 8; sk *= 2) {
       if (sk > 1 && d.K < 32 * sk) continue;  // at least two k-tiles per slice
-      auto run = [&]() {
-        if (tile == 0) dispatch<double, TileD64>(t, sk, st);
-        else dispatch<double, TileD32>(t, sk, st);
-      };
+      auto run = [&]() { launch_choice<double>(t, {tile, sk}, st); };
       run();  // first launch: attributes, instruction cache
       DMRG2_CUDA(cudaEventRecord(e0, st));
       for (int r = 0; r < 2; ++r) run();
@@ -317,16 +354,14 @@ template <typename T>
 void launch_gemm(const Gemm<T>& d, cudaStream_t st) {
   if (d.M <= 0 || d.N <= 0 || d.nb1 * d.nb2 <= 0) return;
   if (d.nb1 * d.nb2 > 65535) throw std::runtime_error("gemm: batch count exceeds 65535");
-  if (d.splitk > 1 && d.nb1 * d.nb2 != 1) throw std::runtime_error("gemm: split-K needs a single GEMM");
+  if (d.Cin && d.nb1 * d.nb2 != 1) throw std::runtime_error("gemm: a separate Cin needs a single GEMM");
   if (ceil_div(d.M, TileD32::BM) > 65535) throw std::runtime_error("gemm: M too large");
   if constexpr (!ST<T>::cplx) {
     if (d.nb1 * d.nb2 == 1 && 2.0 * d.M * d.N * d.K >= TUNE_MIN_FLOP && tune_enabled()) {
-      const TuneChoice c = tuned(d, st);
-      if (c.tile == 1) return dispatch<T, TileD32>(d, c.splitk, st);
-      return dispatch<T, TileD64>(d, c.splitk, st);
+      return launch_choice<T>(d, tuned(d, st), st);
     }
   }
-  dispatch<T, GemmTile<T>>(d, d.splitk, st);
+  launch_choice<T>(d, choose<T>(d), st);
 }
 
 template void launch_gemm<double>(const Gemm<double>&, cudaStream_t);

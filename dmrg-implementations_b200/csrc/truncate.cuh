@@ -129,14 +129,6 @@ SvdOut eig_split(EigWork<T>& W, const T* theta, int m, int nt, char dir, int chi
   constexpr double gtol_rel = 1e-14;  // groups: neighbours within 1e-14 lambda_max
   tridiag_eigvecs(W.d, W.e, n, K, W.lam, W.out, W.Z, W.scr, gtol_rel, s);
   group_mgs(W.Z, n, K, W.lam, W.out, gtol_rel, s);
-  // Newton-Schulz GEMMs have K x K (or n x K) outputs, a few 64 x 64 tiles at chi = 256:
-  // split their long dimension over CTAs, partials in the (otherwise idle) scratch area
-  const size_t scr_len = (size_t)5 * W.nmax * W.Kmax;
-  auto split_for = [&](int M, int N, int Kd) {
-    int sk = std::min(8, std::max(1, Kd / 64));
-    while (sk > 1 && (size_t)sk * M * N > scr_len) --sk;
-    return sk;
-  };
   // Newton-Schulz polar step Z <- Z (3I - Z^T Z) / 2; an orthogonality error e becomes
   // ~1.5 e^2 per iteration, and iterations after convergence only launch kernels that
   // return at once
@@ -148,8 +140,6 @@ SvdOut eig_split(EigWork<T>& W, const T* theta, int m, int nt, char dir, int chi
     g1.B = W.Z; g1.ldb = K;
     g1.C = W.S; g1.ldc = K;
     g1.skip = &W.out->ns_done;
-    g1.splitk = split_for(K, K, n);
-    g1.ws = W.scr;
     launch_gemm(g1, s);
     ns_check(W.S, K, W.out, 4e-16 * (double)n, W.part, W.counter, s);
     DMRG2_CUDA(cudaMemcpyAsync(W.Z2, W.Z, sizeof(double) * (size_t)n * K, cudaMemcpyDeviceToDevice, s));
@@ -160,8 +150,6 @@ SvdOut eig_split(EigWork<T>& W, const T* theta, int m, int nt, char dir, int chi
     g2.C = W.Z2; g2.ldc = K;
     g2.alpha = -0.5; g2.beta = 1.5;
     g2.skip = &W.out->ns_done;
-    g2.splitk = split_for(n, K, K);
-    g2.ws = W.scr;
     launch_gemm(g2, s);
     std::swap(W.Z, W.Z2);
   };
@@ -270,7 +258,6 @@ struct WstWork {
   double* Yc = nullptr;  // qmax x kmax, the other half of each Newton-Schulz step
   double* S = nullptr;   // Gram matrix, then its tiled Cholesky factor (np x np, np = chol_padded(kmax))
   double* cpart = nullptr;  // column sums of squares per row chunk
-  double* ws = nullptr;  // split-K partial products: 8 x qmax x kmax
   double* nrm = nullptr; // |theta|^2, |kept factor|^2
   double* part = nullptr;
   unsigned* counter = nullptr;
@@ -310,7 +297,6 @@ struct WstWork {
     const size_t np = (size_t)chol_padded(kmax);
     S = (double*)alloc(sizeof(double) * np * np);
     cpart = (double*)alloc(sizeof(double) * (size_t)COLNORM_MAX_CHUNKS * kmax);
-    ws = (double*)alloc(sizeof(double) * 8 * qk);
     nrm = (double*)alloc(sizeof(double) * 4);
     part = (double*)alloc(sizeof(double) * 64);
     counter = (unsigned*)alloc(sizeof(unsigned) * 4);
@@ -339,7 +325,7 @@ inline size_t wst_bytes(ll qmax, ll kmax) {
   qmax = std::max<ll>(qmax, 1);
   kmax = std::max<ll>(std::min<ll>(kmax, CHOL_MAX), 1);
   const ll np = chol_padded((int)kmax);
-  return sizeof(double) * (size_t)(14 * qmax * kmax + np * np + COLNORM_MAX_CHUNKS * kmax + 4 + 64) +
+  return sizeof(double) * (size_t)(6 * qmax * kmax + np * np + COLNORM_MAX_CHUNKS * kmax + 4 + 64) +
          sizeof(unsigned) * 4 + sizeof(int) * 4 + sizeof(SvdOut);
 }
 
@@ -350,14 +336,6 @@ inline bool wst_debug() {
     return e && e[0] == '1';
   }();
   return on;
-}
-
-// K split so that a GEMM with few output tiles still spreads over the GPU
-inline int wst_splitk(int M, int N, int K) {
-  const int tiles = ceil_div(M, GemmTile<double>::BM) * ceil_div(N, GemmTile<double>::BN);
-  int sk = 1;
-  while (sk < 8 && tiles * sk < 148 && K / (2 * sk) >= 64) sk *= 2;
-  return sk;
 }
 
 // How many power half-steps a warm split runs:
@@ -389,7 +367,7 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
     *W.h_out = o0;
     DMRG2_CUDA(cudaMemcpyAsync(W.out, W.h_out, sizeof(SvdOut), cudaMemcpyHostToDevice, s));
   }
-  // C (M x N) = alpha op(A) op(B) + beta C, K split over CTAs when the output is small
+  // C (M x N) = alpha op(A) op(B) + beta C
   auto mul = [&](bool ta, const double* A, ll lda, int M, int N, int Kd, const double* B, ll ldb, bool tb,
                  double* C, ll ldc, double alpha, double beta, const int* skip) {
     Gemm<double> g;
@@ -400,8 +378,6 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
     g.C = C; g.ldc = ldc;
     g.alpha = alpha; g.beta = beta;
     g.skip = skip;
-    g.splitk = wst_splitk(M, N, Kd);
-    g.ws = W.ws;
     launch_gemm(g, s);
   };
   const int* done = &W.out->ns_done;

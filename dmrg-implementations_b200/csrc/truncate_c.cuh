@@ -32,7 +32,6 @@ struct WstWorkC {
   double* Z3 = nullptr;
   double* S = nullptr;   // Gram matrix, then its tiled factor (np x np, np = chol_padded(2 kmax))
   double* cpart = nullptr;
-  double* ws = nullptr;  // split-K partial products: 32 qmax kmax doubles
   double* nrm = nullptr;
   double* part = nullptr;
   unsigned* counter = nullptr;
@@ -63,7 +62,6 @@ struct WstWorkC {
     const size_t np = (size_t)chol_padded(2 * kmax);
     S = (double*)alloc(sizeof(double) * np * np);
     cpart = (double*)alloc(sizeof(double) * (size_t)COLNORM_MAX_CHUNKS * 2 * kmax);
-    ws = (double*)alloc(sizeof(double) * 32 * qk);
     nrm = (double*)alloc(sizeof(double) * 4);
     part = (double*)alloc(sizeof(double) * 64);
     counter = (unsigned*)alloc(sizeof(unsigned) * 4);
@@ -93,7 +91,7 @@ inline size_t wstc_bytes(ll qmax, ll kmax) {
   const ll qk = qmax * kmax;
   const ll np = chol_padded((int)(2 * kmax));
   return sizeof(zc) * (size_t)(2 * qk) +
-         sizeof(double) * (size_t)(12 * qk + np * np + COLNORM_MAX_CHUNKS * 2 * kmax + 32 * qk + 4 + 64) +
+         sizeof(double) * (size_t)(12 * qk + np * np + COLNORM_MAX_CHUNKS * 2 * kmax + 4 + 64) +
          sizeof(unsigned) * 4 + sizeof(int) * 4 + sizeof(SvdOut);
 }
 
@@ -122,8 +120,6 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
     g.A = A; g.lda = lda;
     g.B = B; g.ldb = ldb;
     g.C = C; g.ldc = ldc;
-    g.splitk = wst_splitk(M, N, Kd);
-    g.ws = (zc*)W.ws;
     launch_gemm(g, s);
   };
   // real C = alpha op(A) op(B) + beta C on the embeddings
@@ -137,8 +133,6 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
     g.C = C; g.ldc = ldc;
     g.alpha = alpha; g.beta = beta;
     g.skip = skip;
-    g.splitk = wst_splitk(M, N, Kd);
-    g.ws = W.ws;
     launch_gemm(g, s);
   };
   const int k2 = 2 * k;
