@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 namespace dmrg2 {
 
@@ -110,6 +111,38 @@ bool test_unsignalled_waits();
 // uses the memory (owners synchronise their stream first).
 void* dev_alloc(size_t bytes);
 void dev_free(void* p);
+
+// Several buffers in one dev_alloc: every buffer is asked for first (add), then carved in 256-byte
+// aligned slices (commit). An allocation and its wait cost about 10 us; a truncation's or a
+// Lanczos solve's workspace has a dozen buffers.
+class DevSlab {
+ public:
+  template <typename P>
+  void add(P*& p, size_t bytes) {
+    items_.push_back({(void**)&p, bytes});
+  }
+  // returns the block to free with dev_free
+  void* commit() {
+    size_t total = 0;
+    for (const Item& i : items_) total += round(i.bytes);
+    char* base = (char*)dev_alloc(total);
+    size_t off = 0;
+    for (const Item& i : items_) {
+      *i.p = base + off;
+      off += round(i.bytes);
+    }
+    items_.clear();
+    return base;
+  }
+
+ private:
+  struct Item {
+    void** p;
+    size_t bytes;
+  };
+  static size_t round(size_t b) { return ((b ? b : 1) + 255) & ~(size_t)255; }
+  std::vector<Item> items_;
+};
 
 // Page-locked host memory from a process-wide cache of blocks in power-of-two size
 // classes: a block is page-locked once and reused, never handed back to the driver

@@ -1141,7 +1141,7 @@ class Engine final : public EngineBase {
     l.svdout = (SvdOut*)al(sizeof(SvdOut));
     l.jctl = (JacobiCtl*)al(sizeof(JacobiCtl));
     l.dscal = (double*)al(sizeof(double) * 16);
-    l.red.nblk = vec_blocks(nmax_);
+    l.red.nblk = red_blocks(nmax_);
     l.red.part = (double*)al(sizeof(double) * (size_t)l.red.nblk * 2 * (KRYLOV_CAP + 2));
     l.red.counter = (unsigned*)al(sizeof(unsigned) * 4);
     DMRG2_CUDA(cudaMemset(l.red.counter, 0, sizeof(unsigned) * 4));
@@ -1220,7 +1220,7 @@ size_t engine_footprint(const EngineConfig& c, const std::vector<int>& Dl, const
   for (int i = 0; i < L; ++i) qmax = std::max(qmax, (ll)d * cap[i + 1]);
   b += 2 * el(nmax) + el(qmax * qmax) + el(chi * chi);
   const int kcap = std::min(std::max(c.krylov_max, 2), KRYLOV_CAP);
-  const ll nblk = vec_blocks(nmax);
+  const ll nblk = red_blocks(nmax);
   b += sb * ((size_t)kcap + 2) * (size_t)nmax + sizeof(LanczosDev) + sizeof(double) * (size_t)nblk * 2 * (KRYLOV_CAP + 2);
   {
     const size_t nn = (size_t)qmax, kk = (size_t)std::max<ll>(std::min<ll>(chi, qmax), 1);

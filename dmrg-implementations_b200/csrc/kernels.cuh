@@ -24,9 +24,17 @@ struct LanczosDev {
   int kmax;
   int j;                               // Krylov index of the device-looped solve's current step
   int guard;                           // loop bodies run so far (bounds the device loop)
-  unsigned seed_in;                    // the device-looped solve's seed (copied in per solve)
   unsigned long long t_mark;           // %globaltimer when the current matvec was issued
   unsigned long long mv_ns;            // matvec time accumulated by the device-looped solve
+  unsigned bar[8];                     // grid barrier counters of the fused step, start and Ritz kernels
+};
+
+// What the host needs of a finished solve, in page-locked host memory (the last kernel of
+// the solve writes it; valid once the stream has run it).
+struct LanczosHost {
+  double e_cur;
+  unsigned long long mv_ns;
+  int done, converged, n_iter, guard;
 };
 
 // Reduction scratch shared by the vector kernels.
@@ -36,33 +44,35 @@ struct RedScratch {
   int nblk = 0;
 };
 
+constexpr int STEP_BLOCKS = 148;  // blocks of a cooperative Lanczos step (one per SM)
 int vec_blocks(ll n);
+// blocks' worth of partial sums (2 (KRYLOV_CAP + 2) each) RedScratch::part holds for vectors
+// of up to n elements: the streaming passes', or the fused step's two sets
+int red_blocks(ll n);
 
 // w <- H v is done by the caller; these kernels implement one Lanczos step.
-template <typename T>
-void lz_dots(const T* V, int nv, ll n, const T* w, LanczosDev* st, RedScratch& r, cudaStream_t s);
-template <typename T>
-void lz_update_dots(const T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, cudaStream_t s);
-template <typename T>
-void lz_update_norm_check(const T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, int j,
-                          int kmax, cudaStream_t s);
-template <typename T>
-void lz_normalize_next(T* vnext, const T* w, ll n, LanczosDev* st, cudaStream_t s);
-// start: nrm(theta) -> (random fill if ~0) -> v0 = theta/|theta| (also into cur when given)
+// start: nrm(theta) -> (random fill if ~0) -> v0 = theta/|theta| (also into cur when given);
+// seed_host, when given, is page-locked host memory that holds the seed (read only where the
+// random fill is needed)
 template <typename T>
 void lz_start(T* theta, T* v0, ll n, LanczosDev* st, RedScratch& r, unsigned seed, double tol,
-              int kmax, cudaStream_t s, T* cur = nullptr, const unsigned* seed_dev = nullptr);
+              int kmax, cudaStream_t s, T* cur = nullptr, const unsigned* seed_host = nullptr);
+// Krylov step nv (w = H v_(nv-1)): w orthogonalised against v_0 .. v_(nv-1), alpha, beta and the
+// stop rule, v_nv = w / |w| into V when nv < kmax, and the done flag into host_done
+// (page-locked; valid once the stream has run the step). One launch where the vectors fit
+// the fused kernel, the streaming passes (which overwrite w) beyond.
+template <typename T>
+void lz_step(T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, int kmax, int* host_done, cudaStream_t s);
 // The same step with the Krylov index read on the device (st->j), for a loop that runs
-// without the host: the three passes over w = H v_j, then v_(j+1) into V and into cur
-// (the matvec's fixed input).
+// without the host: v_(j+1) also into cur (the matvec's fixed input); it ends one body of
+// the device loop, advancing st->j and setting the loop condition of h to "not done and
+// fewer than kmax bodies run".
 template <typename T>
-void lz_step_dev(const T* V, ll n, T* w, T* cur, LanczosDev* st, RedScratch& r, int kmax, cudaStream_t s);
-// Ends one body of the device loop: advances st->j and sets the loop condition to
-// "not done and fewer than kmax bodies run".
-void lz_loop_next(LanczosDev* st, cudaGraphConditionalHandle h, int kmax, cudaStream_t s);
-// Ritz vector out = sum_i ritz_i V_i, normalised.
+void lz_step_dev(T* V, ll n, T* w, T* cur, LanczosDev* st, RedScratch& r, int kmax, cudaGraphConditionalHandle h,
+                 cudaStream_t s);
+// Ritz vector out = sum_i ritz_i V_i, normalised, and the solve's report into host.
 template <typename T>
-void lz_ritz(const T* V, ll n, T* out, LanczosDev* st, RedScratch& r, cudaStream_t s);
+void lz_ritz(const T* V, ll n, T* out, LanczosDev* st, RedScratch& r, LanczosHost* host, cudaStream_t s);
 
 // ---------------------------------------------------------------- SVD
 struct JacobiCtl {
@@ -83,6 +93,7 @@ struct SvdOut {
   int jacobi_sweeps;
   int jacobi_err;
   int ns_done;      // eigenvector block already orthonormal (Newton-Schulz steps skipped)
+  int ns_near;      // one Newton-Schulz step makes it so (its deviation squared is below the tolerance)
 };
 
 template <typename T>
@@ -124,6 +135,9 @@ void apply_q(const T* R, ll ld, const T* tau, int n, const double* Z, int K, con
              T* Tb, cudaStream_t s, bool wy_ready = false);
 void ns_check(const double* S, int K, SvdOut* out, double tol, double* part, unsigned* counter,
               cudaStream_t s);
+// Up to `iters` Newton-Schulz steps of Z (n x K) in one launch, with ns_check's flag; false, with
+// nothing launched, for blocks beyond 128 x 64
+bool ns_small(double* Z, int n, int K, SvdOut* out, double tol, int iters, cudaStream_t s);
 // k from the eigenvalues: min(chi_max, K, #lam above max(cutoff^2 (x lam_max if relative),
 // floor_rel lam_max)); eigenvalues at or below floor_rel lam_max are rounding noise
 constexpr double EIG_NOISE_FLOOR = 16.0 * 2.2e-16;
@@ -133,6 +147,20 @@ template <typename T>
 void copy_cols_conj(const T* in, ll ldi, int rows, int k, T* out, cudaStream_t s);
 template <typename T>
 void transpose_conj(const T* in, ll ldi, int rows, int k, T* out, cudaStream_t s);
+
+// ---------------------------------------------------------------- warm-started split
+// What the host needs of a split, in page-locked host memory.
+struct SplitHost {
+  double theta2, kept2;  // |theta|^2, |kept factor|^2
+  int failed;            // an orthonormalisation gave up or the polish did not converge
+};
+// status <- 0, *out <- {k}
+void split_begin(int* status, SvdOut* out, int k, cudaStream_t s);
+// |theta|^2 and |kept|^2, and the split's report into host (one launch; the last block of the
+// grid sums the partials in block order and writes the report)
+template <typename T>
+void split_finish(const T* theta, ll nt, const T* kept, ll nk, const int* status, const SvdOut* out, SplitHost* host,
+                  RedScratch& r, cudaStream_t s);
 
 // ---------------------------------------------------------------- misc
 template <typename T>

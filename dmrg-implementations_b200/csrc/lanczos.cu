@@ -6,14 +6,23 @@
 // iteration that read every Krylov vector with coalesced loads, reduce with
 // warp shuffles, and finalise in the last block to arrive (no host sync). The
 // last block of the third kernel also solves the tridiagonal eigenproblem for
-// its lowest eigenvalue (Sturm-sequence multisection), applies the |dE| stop
+// its lowest eigenvalue (multisection on the leading minors), applies the |dE| stop
 // rule and, once done, computes the Ritz coefficients by inverse iteration, so
-// the host never copies alpha/beta back.
+// the host never copies alpha/beta back. Vectors that fit the fused step kernel's
+// shared memory (every n below about 1.8M doubles) take one launch per Krylov step
+// instead (lz_step_kernel).
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+#include "gemm.cuh"
 #include "kernels.cuh"
 
 namespace dmrg2 {
 
 static constexpr int MAX_CHUNK = 2048;
+
+int red_blocks(ll n) { return std::max(vec_blocks(n), 2 * STEP_BLOCKS); }
 
 int vec_blocks(ll n) {
   ll nb = (n + VEC_THREADS - 1) / VEC_THREADS;
@@ -62,88 +71,89 @@ __device__ inline bool arrive_last(unsigned* counter, unsigned nblk) {
 // ----------------------------------------------------------------------------
 // tridiagonal helpers (block-wide / single thread)
 // ----------------------------------------------------------------------------
-// 1/a from the hardware estimate and two Newton-Raphson steps y <- y + y (1 - a y)
-__device__ inline double rcp_refined(double a) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  double r = fma(-a, y, 1.0);
-  y = fma(y, r, y);
-  r = fma(-a, y, 1.0);
-  return fma(y, r, y);
-}
-
-__device__ inline int sturm_count(const double* a, const double* b, int k, double x, double pivmin) {
-  double q = a[0] - x;
-  int c = 0;
-  if (fabs(q) < pivmin) q = -pivmin;
-  if (q < 0) ++c;
-  for (int i = 1; i < k; ++i) {
-    q = (a[i] - x) - b[i - 1] * b[i - 1] * rcp_refined(q);
-    if (fabs(q) < pivmin) q = -pivmin;
-    if (q < 0) ++c;
+// Lowest eigenvalue of the symmetric tridiagonal (a, b) of order k <= KRYLOV_CAP, a and b in
+// shared memory; hint is the lowest eigenvalue of the leading block of order k - 1 (unused for
+// k = 1). One warp; every lane gets the result. sa, sb: KRYLOV_CAP + 8 doubles of shared memory each.
+//
+// Multisection with two trial points per lane. x lies below the lowest eigenvalue exactly
+// when every leading principal minor of T - x is positive, so a trial is the minors'
+// recurrence p_i = (a_i - x) p_(i-1) - b_(i-1)^2 p_(i-2) and one sign test per step: one
+// multiply and one fused multiply-add on the dependent chain, no division. T is scaled by a
+// power of two to entries of at most 1 and the pair (p_i, p_(i-1)) is rescaled by a power of
+// two before it can underflow, so the signs are those of the unscaled recurrence. One warp with
+// two chains a lane just hides the chain's latency; a block of 512 trial points instead is
+// bound by the FP64 pipe (12,300 cycles at k = 10, 23,100 at k = 25). The trial points
+// are ordered, so the count of positive ones is the position of the eigenvalue.
+// Bracket: interlacing gives lambda_k <= hint, Weyl's bound
+// lambda_k >= min(hint, a_k) - |b_(k-1)|; the slack covers the rounding in hint.
+__device__ double tridiag_lowest(const double* a, const double* b, int k, double hint, double* sa, double* sb) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  if (k == 1) return a[0];
+  double mx = 0.0, lo = 1e300, hi = 1e300;
+  bool bad = false;  // a NaN or infinity (fmax and fmin would drop a NaN)
+  for (int i = lane; i < k; i += 32) {
+    bad = bad || !isfinite(a[i]) || (i < k - 1 && !isfinite(b[i]));
+    const double l = i > 0 ? fabs(b[i - 1]) : 0.0, r = i < k - 1 ? fabs(b[i]) : 0.0;
+    mx = fmax(mx, fabs(a[i]) + l + r);
+    lo = fmin(lo, a[i] - l - r);
+    hi = fmin(hi, a[i]);
   }
-  return c;
-}
-
-// Lowest eigenvalue of the symmetric tridiagonal (a, b) of order k. All threads
-// of the block must call; the result is returned to every thread. When hint is
-// finite, the bracket starts at [hint - 2|b_{k-2}| - tiny, hint]: by Cauchy
-// interlacing the lowest eigenvalue of T_k is at most that of T_{k-1} (hint),
-// and by Weyl's bound it is at least hint - |b_{k-2}| - |a_{k-1} - ...| which the
-// Gershgorin check below still guards.
-__device__ double tridiag_lowest(const double* a, const double* b, int k, double hint) {
-  __shared__ double lo_s, hi_s, piv_s;
-  __shared__ int tmin;
-  const int NT = blockDim.x;
-  if (threadIdx.x == 0) {
-    double lo = 1e300, hi = -1e300, bm = 0.0;
-    for (int i = 0; i < k; ++i) {
-      double r = (i > 0 ? fabs(b[i - 1]) : 0.0) + (i < k - 1 ? fabs(b[i]) : 0.0);
-      lo = fmin(lo, a[i] - r);
-      hi = fmax(hi, a[i] + r);
-      if (i < k - 1) bm = fmax(bm, b[i] * b[i]);
-    }
-    double w = fmax(hi - lo, 1e-300);
-    lo_s = lo - 1e-14 * w;
-    hi_s = hi + 1e-14 * w;
-    piv_s = 1e-300 * fmax(1.0, bm);
-    if (k >= 2 && isfinite(hint) && hint < 1e299) {
-      // tight bracket: [hint - 2 |b_{k-2}| - slack, hint + slack], verified by counts below
-      double slack = 1e-12 * fmax(fabs(hint), 1e-300) + 1e-300;
-      double tlo = hint - 2.0 * fabs(b[k - 2]) - slack, thi = hint + slack;
-      int clo = sturm_count(a, b, k, tlo, piv_s), chi = sturm_count(a, b, k, thi, piv_s);
-      if (clo == 0 && chi >= 1) {
-        lo_s = tlo;
-        hi_s = thi;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    mx = fmax(mx, __shfl_xor_sync(FULL, mx, o));
+    lo = fmin(lo, __shfl_xor_sync(FULL, lo, o));
+    hi = fmin(hi, __shfl_xor_sync(FULL, hi, o));
+  }
+  if (__any_sync(FULL, bad)) return nan("");
+  if (!(mx > 0.0)) return 0.0;
+  if (isfinite(hint) && fabs(hint) < 1e299) {
+    lo = fmax(lo, fmin(hint, a[k - 1]) - fabs(b[k - 2]));
+    hi = fmin(hi, hint);
+  }
+  int e = 0;
+  frexp(mx, &e);
+  // (sb[i] belongs to step i; steps beyond k - 1 up to a whole group of 8 keep every sign: the
+  // trial points are below 4 after the scaling)
+  const int kp = ((k + 6) / 8) * 8 + 1;
+  for (int i = lane; i < kp; i += 32) {
+    sa[i] = i < k ? ldexp(a[i], -e) : 8.0;
+    const double bi = (i > 0 && i < k) ? ldexp(b[i - 1], -e) : 0.0;
+    sb[i] = -bi * bi;
+  }
+  lo = ldexp(lo, -e) - 4e-15;
+  hi = ldexp(hi, -e) + 4e-15;
+  __syncwarp();
+  for (int round = 0; round < 16; ++round) {
+    const double step = (hi - lo) * (1.0 / 65.0);
+    const double x0 = fma(step, (double)(lane + 1), lo), x1 = fma(step, (double)(lane + 33), lo);
+    double m0 = 1.0, m1 = 1.0, p0 = sa[0] - x0, p1 = sa[0] - x1;
+    bool pos0 = p0 > 0.0, pos1 = p1 > 0.0;
+    for (int i0 = 1; i0 < kp; i0 += 8) {
+      double ai[8], bi[8];  // loaded ahead of the chain
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        ai[u] = sa[i0 + u];
+        bi[u] = sb[i0 + u];
       }
-    }
-  }
-  __syncthreads();
-  for (int round = 0; round < 12; ++round) {
-    double lo = lo_s, hi = hi_s;
-    double x = lo + (hi - lo) * (double)(threadIdx.x + 1) / (double)(NT + 1);
-    int c = sturm_count(a, b, k, x, piv_s);
-    if (threadIdx.x == 0) tmin = NT;
-    __syncthreads();
-    if (c >= 1) atomicMin(&tmin, (int)threadIdx.x);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int t = tmin;
-      double step = (hi - lo) / (double)(NT + 1);
-      if (t == NT) {
-        lo_s = lo + step * NT;
-      } else {
-        hi_s = lo + step * (t + 1);
-        lo_s = lo + step * t;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const double q0 = fma(ai[u] - x0, p0, bi[u] * m0), q1 = fma(ai[u] - x1, p1, bi[u] * m1);
+        m0 = p0; p0 = q0;
+        m1 = p1; p1 = q1;
+        pos0 = pos0 && (p0 > 0.0);
+        pos1 = pos1 && (p1 > 0.0);
       }
+      if (fmax(fabs(p0), fabs(m0)) < 0x1p-300) { p0 *= 0x1p+300; m0 *= 0x1p+300; }
+      if (fmax(fabs(p1), fabs(m1)) < 0x1p-300) { p1 *= 0x1p+300; m1 *= 0x1p+300; }
     }
-    __syncthreads();
-    double l2 = lo_s, h2 = hi_s;
-    if (h2 - l2 <= 4e-16 * fmax(fabs(l2), fabs(h2)) + 1e-300) break;
+    const int n = __popc(__ballot_sync(FULL, pos0)) + __popc(__ballot_sync(FULL, pos1));
+    const double l2 = n > 0 ? fma(step, (double)n, lo) : lo;
+    if (n < 64) hi = fma(step, (double)(n + 1), lo);
+    lo = l2;
+    if (hi - lo <= 4e-16 * fmax(fabs(lo), fabs(hi)) + 1e-300) break;
   }
-  double r = 0.5 * (lo_s + hi_s);
-  __syncthreads();
-  return r;
+  return ldexp(0.5 * (lo + hi), e);
 }
 
 // Eigenvector of the tridiagonal (a, b) for eigenvalue lam by inverse iteration
@@ -213,6 +223,479 @@ __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
+}
+
+// The end of a Krylov step (the first warp of a block): the lowest Ritz value of the k-step
+// matrix (a, b) (shared memory), the stop rule and, once done, the Ritz coefficients. Returns
+// whether the solve is done.
+struct StepState {
+  double a[KRYLOV_CAP], b[KRYLOV_CAP], y[KRYLOV_CAP], work[5 * KRYLOV_CAP];
+};
+__device__ bool lz_finish_step(LanczosDev* st, StepState& sh, int k, int kmax, double e_prev, double tol) {
+  const double lam = tridiag_lowest(sh.a, sh.b, k, e_prev, sh.work, sh.work + 2 * KRYLOV_CAP);
+  const bool conv = (k >= 3) && (fabs(lam - e_prev) < tol);
+  const bool brk = sh.b[k - 1] < 1e-14;
+  const bool done = conv || brk || k >= kmax;
+  __syncwarp();  // the work area is free again
+  if (threadIdx.x == 0) {
+    st->e_cur = lam;
+    st->e_prev = lam;
+    if (done) {
+      st->converged = (conv || brk) ? 1 : 0;
+      st->n_iter = k;
+      tridiag_vector(sh.a, sh.b, k, lam, sh.y, sh.work);
+      for (int i = 0; i < k; ++i) st->ritz[i] = sh.y[i];
+      __threadfence();
+      st->done = 1;
+    }
+  }
+  return done;
+}
+
+// ----------------------------------------------------------------------------
+// one Krylov step in one launch
+// ----------------------------------------------------------------------------
+// A step's vectors live in the L2 (2.1 MB each at chi = 256), so the passes above are bound
+// by their latency: three launches, each with a grid-wide last-block reduction that the next
+// one waits for, then a normalisation and a loop kernel. Here one grid keeps its slice of w in
+// shared memory through the whole step and meets at two barriers:
+//   coef0 = V^H w | w -= V coef0, coef1 = V^H w, |w|^2 | w -= V coef1, v_(j+1) = w / |w|
+// (the same classical Gram-Schmidt, applied twice). The norm after the second projection
+// follows from the one before it, |w'|^2 - |coef1|^2 (V is orthonormal to rounding, coef1 is
+// the rounding left by the first projection), so no third barrier is needed, and block 0
+// solves the tridiagonal problem while the others finish their slices. Every block sums the
+// partial products itself, in the same fixed order.
+// The barrier: up to LS_CLUSTER blocks are one thread-block cluster (hardware barrier);
+// beyond, a cooperative launch of one block per SM with a counter barrier (bounded).
+// The staged basis is read four times a step, so a slice costs one pass over the L2.
+// Per step at chi = 256 (n = 262,144, 3 Krylov vectors) 31 us in five launches before and
+// 15 us now; in a 12-site chain at chi = 64 (n <= 16,384) 33 us before, 16 us now.
+constexpr int LS_THREADS = 512;
+constexpr int LS_WARPS = LS_THREADS / 32;
+constexpr int LS_CLUSTER = 16;
+constexpr int LS_PUSH = 32;                    // values exchanged through the cluster's shared memory at most
+constexpr size_t LS_SMEM_W = 96 * 1024;        // slice of w per block at most
+// w and the staged basis per block: one block per SM of the cooperative grid; a cluster leaves room
+// for a second block, since the clusters of concurrent solves share the SMs
+constexpr size_t LS_SMEM_GRID = 176 * 1024, LS_SMEM_CLUSTER = 72 * 1024;
+constexpr long long LS_SPIN = 1ll << 22;       // barrier polls before a block gives up (seconds)
+
+struct StepGrid {
+  int blocks = 0;  // 0: the vector does not fit, the streaming passes run
+  int chunk = 0;
+  bool cluster = false;
+};
+
+template <typename T>
+static StepGrid step_grid(ll n) {
+  // slices of 512 elements (one per thread) until 16 blocks are reached, which a cluster holds up
+  // to 2048 elements each; then one block per SM
+  StepGrid g;
+  const ll cl_max = 2048 / (ll)(sizeof(T) / sizeof(double));
+  ll nb = (n + LS_THREADS - 1) / LS_THREADS;
+  g.cluster = n <= LS_CLUSTER * cl_max;
+  const ll cap = g.cluster ? LS_CLUSTER : STEP_BLOCKS;
+  if (nb > cap) nb = cap;
+  const ll ch = ((n + nb - 1) / nb + 1) & ~1ll;  // even: 16-byte slices
+  if (ch * (ll)sizeof(T) > (ll)LS_SMEM_W) return g;
+  g.blocks = (int)nb;
+  g.chunk = (int)ch;
+  return g;
+}
+
+__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// all blocks of the grid meet; false when the bounded wait ran out
+template <bool CL>
+__device__ __forceinline__ bool step_barrier(unsigned* bar) {
+  if constexpr (CL) {
+    cooperative_groups::this_cluster().sync();
+    return true;
+  } else {
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+      long long it = 0;
+      while (ld_acquire_gpu(bar) < gridDim.x && ++it < LS_SPIN) {
+      }
+      ok = it < LS_SPIN;
+    }
+    return __syncthreads_and(ok ? 1 : 0) != 0;
+  }
+}
+
+// warp sums of eight values per lane, out[0 .. cnt-1]: the sums share their shuffles (nine instead
+// of forty; the value index follows lane bits 4, 3 and 2)
+__device__ __forceinline__ void warp_sum8(double (&v)[8], int lane, double* out, int cnt) {
+  const bool h = lane & 16, g = lane & 8, f = lane & 4;
+  double a[4], b[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) a[i] = (h ? v[4 + i] : v[i]) + __shfl_xor_sync(0xffffffffu, h ? v[i] : v[4 + i], 16);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) b[i] = (g ? a[2 + i] : a[i]) + __shfl_xor_sync(0xffffffffu, g ? a[i] : a[2 + i], 8);
+  double c = (f ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, f ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  c += __shfl_xor_sync(0xffffffffu, c, 1);
+  const int idx = (h ? 4 : 0) + (g ? 2 : 0) + (f ? 1 : 0);
+  if ((lane & 3) == 0 && idx < cnt) out[idx] = c;
+}
+
+// A block's slice of the Krylov basis: the first nc vectors staged in shared memory (they are
+// read four times in a step), the others read from the L2.
+template <typename T>
+struct BasisSlice {
+  const T* sm;  // [nc][chunk]
+  int nc, chunk;
+  const T* g;   // vector i at g + i n
+  ll n;
+};
+
+// <v_i, ws> for u < m vectors from i0 (stride ld), this thread's elements, into acc
+template <typename T, int U, bool FULL>
+__device__ __forceinline__ void dots_group(const T* v0, ll ld, int m, const T* ws, int len, double (&acc)[8]) {
+  constexpr bool CPLX = ST<T>::cplx;
+#pragma unroll 2
+  for (int x = threadIdx.x; x < len; x += LS_THREADS) {
+    const T wv = ws[x];
+    T v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = (FULL || u < m) ? v0[u * ld + x] : ST<T>::zero();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const T p = ST<T>::cmul(v[u], wv);
+      if constexpr (CPLX) {
+        acc[2 * u] += p.re;
+        acc[2 * u + 1] += p.im;
+      } else {
+        acc[u] += p;
+      }
+    }
+  }
+}
+
+// per-warp sums of <v_i, ws>, i < nv (c = i, or 2 i and 2 i + 1 for complex data), into
+// wsum[warp][c]
+template <typename T>
+__device__ __forceinline__ void slice_dots(const BasisSlice<T>& V, int nv, const T* ws, int len, double* wsum,
+                                           int wpitch) {
+  constexpr bool CPLX = ST<T>::cplx;
+  constexpr int U = CPLX ? 4 : 8;  // the vectors of one eight-value reduction
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i0 = 0; i0 < nv;) {
+    double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const bool in_sm = i0 < V.nc;
+    const int m = min(U, (in_sm ? V.nc : nv) - i0);
+    if (in_sm) {
+      const T* v0 = V.sm + i0 * V.chunk;
+      if (m == U) dots_group<T, U, true>(v0, V.chunk, m, ws, len, acc);
+      else dots_group<T, U, false>(v0, V.chunk, m, ws, len, acc);
+    } else {
+      const T* v0 = V.g + (ll)i0 * V.n;
+      if (m == U) dots_group<T, U, true>(v0, V.n, m, ws, len, acc);
+      else dots_group<T, U, false>(v0, V.n, m, ws, len, acc);
+    }
+    warp_sum8(acc, lane, wsum + warp * wpitch + (CPLX ? 2 * i0 : i0), CPLX ? 2 * m : m);
+    i0 += m;
+  }
+}
+
+// ws -= sum_i c_i v_i on this thread's elements; returns its share of |ws|^2
+template <typename T>
+__device__ __forceinline__ double slice_update(const BasisSlice<T>& V, int nv, T* ws, int len, const double* c) {
+  constexpr bool CPLX = ST<T>::cplx;
+  auto coef = [&](int i) {
+    if constexpr (CPLX) return mkz(c[2 * i], c[2 * i + 1]);
+    else return c[i];
+  };
+  double ww = 0.0;
+  for (int x = threadIdx.x; x < len; x += LS_THREADS) {
+    T v = ws[x];
+    int i = 0;
+#pragma unroll 4
+    for (; i < V.nc; ++i) v = v - ST<T>::mul(coef(i), V.sm[i * V.chunk + x]);
+#pragma unroll 8
+    for (; i < nv; ++i) v = v - ST<T>::mul(coef(i), V.g[(ll)i * V.n + x]);
+    ws[x] = v;
+    ww += ST<T>::abs2(v);
+  }
+  return ww;
+}
+
+// The grid's sums of `ncoef` values from each block's per-warp sums, into dst (shared memory,
+// every block, the same order everywhere). A cluster with few values pushes them into every
+// block's shared memory (xch: LS_CLUSTER x ncoef there) ahead of the hardware barrier; otherwise they
+// go through part[c][block] and the grid barrier. Returns false when a bounded wait ran out.
+template <bool CL>
+__device__ __forceinline__ bool exchange_sums(const double* wsum, int wpitch, int ncoef, double* part, unsigned* bar,
+                                              double* xch, double* dst) {
+  const int tid = threadIdx.x, lane = tid & 31, nblk = gridDim.x;
+  const bool push = CL && ncoef <= LS_PUSH;
+  __syncthreads();
+  for (int c = tid; c < ncoef; c += LS_THREADS) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < LS_WARPS; ++w) s += wsum[w * wpitch + c];
+    if (push) {
+      cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+      for (int b = 0; b < nblk; ++b) cl.map_shared_rank(xch, b)[blockIdx.x * ncoef + c] = s;
+    } else {
+      part[(ll)c * nblk + blockIdx.x] = s;
+    }
+  }
+  const bool ok = step_barrier<CL>(bar);
+  if (push) {
+    for (int c = tid; c < ncoef; c += LS_THREADS) {
+      double s = 0.0;
+      for (int b = 0; b < nblk; ++b) s += xch[b * ncoef + c];
+      dst[c] = s;
+    }
+  } else {
+    for (int c = tid >> 5; c < ncoef; c += LS_WARPS) {
+      double s = 0.0;
+      for (int b = lane; b < nblk; b += 32) s += __ldcg(part + (ll)c * nblk + b);
+      s = warp_sum(s);
+      if (lane == 0) dst[c] = s;
+    }
+  }
+  __syncthreads();
+  return ok;
+}
+
+// asynchronous copy of `count` elements from global to shared memory (committed by the caller);
+// vec: both are 16-byte aligned
+template <typename T>
+__device__ __forceinline__ void copy_async(T* dst, const T* src, int count, bool vec) {
+  if (vec && sizeof(T) == 8) {
+    for (int x = 2 * threadIdx.x; x + 1 < count; x += 2 * LS_THREADS) cp_async_16(dst + x, src + x, true);
+    if ((count & 1) && threadIdx.x == 0) cp_async_8(dst + count - 1, src + count - 1, true);
+  } else {
+    for (int x = threadIdx.x; x < count; x += LS_THREADS) {
+      if constexpr (sizeof(T) == 16) cp_async_16(dst + x, src + x, true);
+      else cp_async_8(dst + x, src + x, true);
+    }
+  }
+}
+
+// loop != 0: the device-looped solve (the Krylov index is st->j, cur gets v_(j+1), the matvec's
+// time since st->t_mark is added to st->mv_ns, and block 0 advances the index and sets the
+// loop condition of handle h); else nv = j + 1 is given and host_done, when given, gets the
+// done flag (page-locked host memory). ncache: vectors of the basis staged in shared memory.
+template <typename T, bool CL>
+__global__ void __launch_bounds__(LS_THREADS, 1)
+    lz_step_kernel(T* V, int nv, ll n, const T* w, T* cur, LanczosDev* st, double* part, int kmax, int chunk,
+                   int ncache, int loop, cudaGraphConditionalHandle h, volatile int* host_done) {
+  extern __shared__ __align__(16) unsigned char ls_smem[];
+  __shared__ StepState sh;
+  __shared__ double csum[2 * KRYLOV_CAP + 1];
+  __shared__ double xch[CL ? 2 * LS_CLUSTER * LS_PUSH : 1];
+  constexpr int CV = ST<T>::cplx ? 2 : 1;
+  const int tid = threadIdx.x;
+  const bool lead = blockIdx.x == 0;
+  // one thread per block reads the state (every warp of 148 blocks reading these words took 2.6 us:
+  // they are one L2 line), all fields in one round trip
+  __shared__ int s_j, s_guard, s_done;
+  __shared__ double s_eprev, s_tol;
+  if (tid == 0) {
+    s_done = *((volatile int*)&st->done);
+    s_j = *((volatile int*)&st->j);
+    s_guard = *((volatile int*)&st->guard);
+    s_eprev = *((volatile double*)&st->e_prev);
+    s_tol = *((volatile double*)&st->tol);
+  }
+  __syncthreads();
+  const int j = s_j, guard = s_guard;
+  if (s_done) {  // set by an earlier launch only: the same for every block
+    if (lead && tid == 0) {
+      if (host_done) *host_done = 1;
+      if (loop) cudaGraphSetConditional(h, 0u);
+    }
+    return;
+  }
+  if (loop) {
+    nv = j + 1;
+    if (lead && tid == 0) st->mv_ns += global_ns() - st->t_mark;
+  }
+  const int nc = CV * nv, wpitch = nc + 1;
+  const ll x0 = (ll)blockIdx.x * chunk;
+  const int len = (int)max((ll)0, min((ll)chunk, n - x0));
+  T* ws = reinterpret_cast<T*>(ls_smem);
+  T* vs = ws + chunk;                                                // [ncache][chunk]
+  double* wsum = reinterpret_cast<double*>(vs + (ll)ncache * chunk);  // LS_WARPS x wpitch
+  const BasisSlice<T> B{vs, min(nv, ncache), chunk, V + x0, n};
+  {
+    const bool vec = ((n | chunk) & 1) == 0;  // slices and vectors start on 16 bytes
+    copy_async(ws, w + x0, len, vec);
+    for (int i = 0; i < B.nc; ++i) copy_async(vs + i * chunk, V + (ll)i * n + x0, len, vec);
+    cp_async_commit();
+  }
+  if (lead)
+    for (int i = tid; i < nv - 1; i += LS_THREADS) {
+      sh.a[i] = st->alpha[i];
+      sh.b[i] = st->beta[i];
+    }
+  if (lead && tid == 0 && !CL) {  // before anyone passes the first barrier
+    volatile unsigned* bar = st->bar;
+    bar[1] = bar[2] = bar[3] = 0u;  // the last step's, and the start's
+  }
+  if (CL) cooperative_groups::this_cluster().sync();  // the peers run: their shared memory may be written
+  cp_async_wait<0>();
+  __syncthreads();
+  slice_dots<T>(B, nv, ws, len, wsum, wpitch);
+  bool ok = exchange_sums<CL>(wsum, wpitch, nc, part, &st->bar[0], xch, csum);
+  const double a0 = csum[CV * (nv - 1)];
+  {
+    const double ww = warp_sum(slice_update<T>(B, nv, ws, len, csum));
+    slice_dots<T>(B, nv, ws, len, wsum, wpitch);
+    if ((tid & 31) == 0) wsum[(tid >> 5) * wpitch + nc] = ww;
+  }
+  ok = exchange_sums<CL>(wsum, wpitch, nc + 1, part + (ll)nc * gridDim.x, &st->bar[1],
+                         xch + (CL ? LS_CLUSTER * LS_PUSH : 0), csum) && ok;
+  double c2 = 0.0;
+  for (int c = 0; c < nc; ++c) c2 += csum[c] * csum[c];
+  const double nrm2 = fmax(csum[nc] - c2, 0.0);
+  if (nv < kmax) {
+    slice_update<T>(B, nv, ws, len, csum);
+    const double inv = nrm2 > 0.0 ? 1.0 / sqrt(nrm2) : 0.0;
+    T* vn = V + (ll)nv * n + x0;
+    for (int x = tid; x < len; x += LS_THREADS) {
+      const T v = ST<T>::scale(inv, ws[x]);
+      vn[x] = v;
+      if (cur) cur[x0 + x] = v;
+    }
+  }
+  if (!lead || tid >= 32) return;
+  const double beta = sqrt(nrm2);
+  if (tid == 0) {
+    sh.a[nv - 1] = st->alpha[nv - 1] = a0 + csum[CV * (nv - 1)];
+    sh.b[nv - 1] = st->beta[nv - 1] = beta;
+    st->nrm2 = nrm2;
+    if (!CL) *((volatile unsigned*)&st->bar[0]) = 0u;  // everyone is past the first barrier
+    if (!ok) {  // a barrier gave up: end the solve without a result
+      st->n_iter = 0;
+      st->done = 1;
+    }
+  }
+  __syncwarp();
+  const bool done = ok ? lz_finish_step(st, sh, nv, kmax, s_eprev, s_tol) : true;
+  if (tid == 0) {
+    if (host_done) *host_done = done ? 1 : 0;
+    if (loop) {
+      st->guard = guard + 1;
+      if (!done) st->j = j + 1;
+      st->t_mark = global_ns();
+      cudaGraphSetConditional(h, (!done && guard + 1 < kmax) ? 1u : 0u);
+    }
+  }
+}
+
+__device__ inline double hash_uniform(unsigned long long x) {
+  x += 0x9E3779B97F4A7C15ull;
+  x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
+  x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
+  x ^= x >> 31;
+  return (double)(x >> 11) * (1.0 / 9007199254740992.0) * 2.0 - 1.0;
+}
+
+// start of a solve: |theta|^2 (theta replaced by a seeded random vector where it is ~0 or not a
+// number), the solver state, v_0 = theta / |theta| into V and cur
+template <typename T, bool CL>
+__global__ void __launch_bounds__(LS_THREADS, 1)
+    lz_start_kernel(T* theta, T* v0, T* cur, ll n, LanczosDev* st, double* part, unsigned seed,
+                    const unsigned* seed_host, double tol, int kmax, int chunk) {
+  __shared__ double wsum[LS_WARPS], xch_s[2][LS_CLUSTER], tot;
+  const int tid = threadIdx.x;
+  const bool lead = blockIdx.x == 0;
+  if (CL) cooperative_groups::this_cluster().sync();  // the peers run: their shared memory may be written
+  const ll x0 = (ll)blockIdx.x * chunk;
+  const int len = (int)max((ll)0, min((ll)chunk, n - x0));
+  auto norm = [&](double* p, unsigned* bar, double* xch) {
+    double ww = 0.0;
+    for (int x = tid; x < len; x += LS_THREADS) ww += ST<T>::abs2(theta[x0 + x]);
+    ww = warp_sum(ww);
+    if ((tid & 31) == 0) wsum[tid >> 5] = ww;
+    return exchange_sums<CL>(wsum, 1, 1, p, bar, xch, &tot);
+  };
+  if (lead && tid == 0 && !CL) *((volatile unsigned*)&st->bar[4]) = 0u;  // the last solve's
+  bool ok = norm(part, &st->bar[2], xch_s[0]);
+  const bool tiny = !(tot >= 1e-28);
+  if (tiny) {
+    if (seed_host) seed = *((volatile const unsigned*)seed_host);
+    for (int e = tid; e < len; e += LS_THREADS) {
+      const ll x = x0 + e;
+      const double r = hash_uniform(((unsigned long long)seed << 32) ^ (unsigned long long)(2 * x));
+      const double i = ST<T>::cplx ? hash_uniform(((unsigned long long)seed << 32) ^ (2 * x + 1)) : 0.0;
+      theta[x] = ST<T>::make(r, i);
+    }
+    __syncthreads();  // tot is read by every thread before the second sum replaces it
+    ok = norm(part + gridDim.x, &st->bar[3], xch_s[1]) && ok;
+  }
+  const double inv = 1.0 / sqrt(tot);
+  for (int x = tid; x < len; x += LS_THREADS) {
+    const T v = ST<T>::scale(inv, theta[x0 + x]);
+    v0[x0 + x] = v;
+    if (cur) cur[x0 + x] = v;
+  }
+  if (lead && tid == 0) {
+    st->nrm2 = tot;
+    st->randomized = tiny ? 1 : 0;
+    st->done = ok ? 0 : 1;
+    st->converged = 0;
+    st->n_iter = 0;
+    st->e_prev = 1e300;
+    st->e_cur = 0.0;
+    st->tol = tol;
+    st->kmax = kmax;
+    st->j = 0;
+    st->guard = 0;
+    st->t_mark = global_ns();
+    st->mv_ns = 0ull;
+  }
+}
+
+__device__ __forceinline__ void lz_report(const LanczosDev* st, LanczosHost* host) {
+  volatile LanczosHost* h = host;
+  h->e_cur = st->e_cur;
+  h->mv_ns = st->mv_ns;
+  h->done = st->done;
+  h->converged = st->converged;
+  h->n_iter = st->n_iter;
+  h->guard = st->guard;
+}
+__global__ void lz_report_kernel(const LanczosDev* st, LanczosHost* host) { lz_report(st, host); }
+
+// end of a solve: out = sum_i ritz_i v_i, normalised, and the report to the host
+template <typename T, bool CL>
+__global__ void __launch_bounds__(LS_THREADS, 1)
+    lz_ritz_norm_kernel(const T* V, ll n, T* out, LanczosDev* st, double* part, LanczosHost* host, int chunk) {
+  extern __shared__ __align__(16) unsigned char ls_smem[];
+  __shared__ double r[KRYLOV_CAP], wsum[LS_WARPS], xch[LS_CLUSTER], tot;
+  const int tid = threadIdx.x, k = st->n_iter;
+  if (CL) cooperative_groups::this_cluster().sync();  // the peers run: their shared memory may be written
+  if (blockIdx.x == gridDim.x - 1 && tid == 0) lz_report(st, host);
+  T* ws = reinterpret_cast<T*>(ls_smem);
+  const ll x0 = (ll)blockIdx.x * chunk;
+  const int len = (int)max((ll)0, min((ll)chunk, n - x0));
+  for (int i = tid; i < k; i += LS_THREADS) r[i] = st->ritz[i];
+  __syncthreads();
+  double ww = 0.0;
+  for (int x = tid; x < len; x += LS_THREADS) {
+    T acc = ST<T>::zero();
+#pragma unroll 4
+    for (int i = 0; i < k; ++i) acc = acc + ST<T>::scale(r[i], V[(ll)i * n + x0 + x]);
+    ws[x] = acc;
+    ww += ST<T>::abs2(acc);
+  }
+  ww = warp_sum(ww);
+  if ((tid & 31) == 0) wsum[tid >> 5] = ww;
+  exchange_sums<CL>(wsum, 1, 1, part, &st->bar[4], xch, &tot);
+  const double inv = tot > 0.0 ? 1.0 / sqrt(tot) : 0.0;
+  for (int x = tid; x < len; x += LS_THREADS) out[x0 + x] = ST<T>::scale(inv, ws[x]);
+  if (blockIdx.x == 0 && tid == 0) st->nrm2 = tot;
 }
 
 // ----------------------------------------------------------------------------
@@ -304,30 +787,15 @@ __global__ void __launch_bounds__(VEC_THREADS)
   } else if (PHASE == 1) {
     if (threadIdx.x == 0) st->alpha[j] += st->coef[2 * j];
   } else {
-    __shared__ int done_s;
-    __shared__ double tv_work[5 * KRYLOV_CAP];
-    if (threadIdx.x == 0) {
-      double b = sqrt(fmax(st->nrm2, 0.0));
-      st->beta[j] = b;
+    __shared__ StepState sh;
+    if (threadIdx.x == 0) st->beta[j] = sqrt(fmax(st->nrm2, 0.0));
+    __syncthreads();
+    for (int i = threadIdx.x; i <= j; i += blockDim.x) {
+      sh.a[i] = st->alpha[i];
+      sh.b[i] = st->beta[i];
     }
     __syncthreads();
-    const int k = j + 1;
-    double lam = tridiag_lowest(st->alpha, st->beta, k, st->e_prev);
-    if (threadIdx.x == 0) {
-      st->e_cur = lam;
-      bool conv = (k >= 3) && (fabs(lam - st->e_prev) < st->tol);
-      bool brk = st->beta[j] < 1e-14;
-      bool full = (k >= kmax);
-      st->e_prev = lam;
-      done_s = (conv || brk || full) ? 1 : 0;
-      if (done_s) {
-        st->converged = (conv || brk) ? 1 : 0;
-        st->n_iter = k;
-        tridiag_vector(st->alpha, st->beta, k, lam, st->ritz, tv_work);
-        __threadfence();
-        st->done = 1;
-      }
-    }
+    if (threadIdx.x < 32) lz_finish_step(st, sh, j + 1, kmax, st->e_prev, st->tol);
   }
   if (threadIdx.x == 0) *counter = 0u;
 }
@@ -389,21 +857,13 @@ __global__ void norm2_kernel(const T* __restrict__ x, ll n, double* out, double*
   }
 }
 
-__device__ inline double hash_uniform(unsigned long long x) {
-  x += 0x9E3779B97F4A7C15ull;
-  x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
-  x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
-  x ^= x >> 31;
-  return (double)(x >> 11) * (1.0 / 9007199254740992.0) * 2.0 - 1.0;
-}
-
 // reset solver state; if |theta| is ~0, replace theta by a seeded random vector
 template <typename T>
 __global__ void lz_reset_kernel(T* theta, ll n, LanczosDev* st, unsigned seed, double tol, int kmax,
-                                const unsigned* seed_dev) {
-  if (seed_dev) seed = *seed_dev;
+                                const unsigned* seed_host) {
   const bool tiny = !(st->nrm2 >= 1e-28);
   if (tiny) {
+    if (seed_host) seed = *((volatile const unsigned*)seed_host);
     for (ll x = (ll)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (ll)gridDim.x * blockDim.x) {
       double r = hash_uniform(((unsigned long long)seed << 32) ^ (unsigned long long)(2 * x));
       double i = ST<T>::cplx ? hash_uniform(((unsigned long long)seed << 32) ^ (2 * x + 1)) : 0.0;
@@ -467,30 +927,62 @@ static int grid_for(ll n) {
   return (int)g;
 }
 
-template <typename T>
-void lz_dots(const T* V, int nv, ll n, const T* w, LanczosDev* st, RedScratch& r, cudaStream_t s) {
-  lz_pass_kernel<T, 0><<<vec_blocks(n), VEC_THREADS, 0, s>>>(V, nv, n, const_cast<T*>(w), st,
-                                                             r.part, r.counter, 0);
+namespace {
+// launches a kernel of the fused step on grid g: one cluster, or cooperatively
+template <typename K, typename... A>
+void launch_step(K kernel, std::atomic<unsigned long long>& attr, std::atomic<unsigned long long>& attr_c,
+                 const StepGrid& g, size_t smem, cudaStream_t s, A... args) {
+  // (g.cluster is the same in every launch of one kernel instantiation)
+  const size_t smem_max = (g.cluster ? LS_SMEM_CLUSTER : LS_SMEM_GRID) + sizeof(double) * LS_WARPS * (2 * KRYLOV_CAP + 1);
+  set_smem_attr_once(attr, (const void*)kernel, (int)smem_max);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(g.blocks);
+  cfg.blockDim = dim3(LS_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  if (g.cluster) {
+    func_attr_once(attr_c, (const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = g.blocks;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  }
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  DMRG2_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
   DMRG2_CHECK_LAUNCH();
 }
-template <typename T>
-void lz_update_dots(const T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, cudaStream_t s) {
-  lz_pass_kernel<T, 1><<<vec_blocks(n), VEC_THREADS, 0, s>>>(V, nv, n, w, st, r.part, r.counter, 0);
-  DMRG2_CHECK_LAUNCH();
+
+template <typename T, bool CL>
+void step_launch(const StepGrid& g, T* V, int nv, ll n, const T* w, T* cur, LanczosDev* st, RedScratch& r, int kmax,
+                 int loop, cudaGraphConditionalHandle h, int* host_done, cudaStream_t s) {
+  static std::atomic<unsigned long long> attr{0}, attr_c{0};
+  const int nvm = loop ? kmax : nv, nc = (ST<T>::cplx ? 2 : 1) * nvm;
+  const size_t row = sizeof(T) * (size_t)g.chunk, cap = g.cluster ? LS_SMEM_CLUSTER : LS_SMEM_GRID;
+  const int ncache = cap > row ? (int)std::min<size_t>((cap - row) / row, (size_t)nvm) : 0;
+  const size_t smem = row * (size_t)(1 + ncache) + sizeof(double) * (size_t)LS_WARPS * (nc + 1);
+  launch_step(lz_step_kernel<T, CL>, attr, attr_c, g, smem, s, V, nv, n, w, cur, st, r.part, kmax, g.chunk,
+              ncache, loop, h, (volatile int*)host_done);
 }
-template <typename T>
-void lz_update_norm_check(const T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, int j,
-                          int kmax, cudaStream_t s) {
-  (void)j;
-  lz_pass_kernel<T, 2><<<vec_blocks(n), VEC_THREADS, 0, s>>>(V, nv, n, w, st, r.part, r.counter,
-                                                             kmax);
-  DMRG2_CHECK_LAUNCH();
+template <typename T, bool CL>
+void start_launch(const StepGrid& g, T* theta, T* v0, T* cur, ll n, LanczosDev* st, RedScratch& r, unsigned seed,
+                  const unsigned* seed_host, double tol, int kmax, cudaStream_t s) {
+  static std::atomic<unsigned long long> attr{0}, attr_c{0};
+  launch_step(lz_start_kernel<T, CL>, attr, attr_c, g, 0, s, theta, v0, cur, n, st, r.part, seed, seed_host, tol, kmax,
+              g.chunk);
 }
-template <typename T>
-void lz_normalize_next(T* vnext, const T* w, ll n, LanczosDev* st, cudaStream_t s) {
-  lz_normalize_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(vnext, w, n, st);
-  DMRG2_CHECK_LAUNCH();
+template <typename T, bool CL>
+void ritz_launch(const StepGrid& g, const T* V, ll n, T* out, LanczosDev* st, RedScratch& r, LanczosHost* host,
+                 cudaStream_t s) {
+  static std::atomic<unsigned long long> attr{0}, attr_c{0};
+  launch_step(lz_ritz_norm_kernel<T, CL>, attr, attr_c, g, sizeof(T) * (size_t)g.chunk, s, V, n, out, st, r.part,
+              host, g.chunk);
 }
+}  // namespace
 
 template <typename T>
 void norm2(const T* x, ll n, double* out_dev, RedScratch& r, cudaStream_t s) {
@@ -502,38 +994,131 @@ void norm2(const T* x, ll n, double* out_dev, RedScratch& r, cudaStream_t s) {
 
 template <typename T>
 void lz_start(T* theta, T* v0, ll n, LanczosDev* st, RedScratch& r, unsigned seed, double tol,
-              int kmax, cudaStream_t s, T* cur, const unsigned* seed_dev) {
+              int kmax, cudaStream_t s, T* cur, const unsigned* seed_host) {
+  const StepGrid g = step_grid<T>(n);
+  if (g.blocks && g.cluster) return start_launch<T, true>(g, theta, v0, cur, n, st, r, seed, seed_host, tol, kmax, s);
+  if (g.blocks) return start_launch<T, false>(g, theta, v0, cur, n, st, r, seed, seed_host, tol, kmax, s);
   norm2<T>(theta, n, &st->nrm2, r, s);
-  lz_reset_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(theta, n, st, seed, tol, kmax, seed_dev);
+  lz_reset_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(theta, n, st, seed, tol, kmax, seed_host);
   DMRG2_CHECK_LAUNCH();
   norm2<T>(theta, n, &st->nrm2, r, s);
   lz_v0_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(theta, v0, n, st, cur);
   DMRG2_CHECK_LAUNCH();
 }
 
+namespace {
+// the streaming passes, for vectors beyond the fused step (nv < 0: read from st->j)
 template <typename T>
-void lz_step_dev(const T* V, ll n, T* w, T* cur, LanczosDev* st, RedScratch& r, int kmax, cudaStream_t s) {
-  lz_pass_kernel<T, 0><<<vec_blocks(n), VEC_THREADS, 0, s>>>(V, -1, n, w, st, r.part, r.counter, 0);
+void step_passes(T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, int kmax, cudaStream_t s) {
+  lz_pass_kernel<T, 0><<<vec_blocks(n), VEC_THREADS, 0, s>>>(V, nv, n, w, st, r.part, r.counter, 0);
   DMRG2_CHECK_LAUNCH();
-  lz_pass_kernel<T, 1><<<vec_blocks(n), VEC_THREADS, 0, s>>>(V, -1, n, w, st, r.part, r.counter, 0);
+  lz_pass_kernel<T, 1><<<vec_blocks(n), VEC_THREADS, 0, s>>>(V, nv, n, w, st, r.part, r.counter, 0);
   DMRG2_CHECK_LAUNCH();
-  lz_pass_kernel<T, 2><<<vec_blocks(n), VEC_THREADS, 0, s>>>(V, -1, n, w, st, r.part, r.counter, kmax);
-  DMRG2_CHECK_LAUNCH();
-  lz_normalize_dev_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(const_cast<T*>(V), cur, w, n, st);
+  lz_pass_kernel<T, 2><<<vec_blocks(n), VEC_THREADS, 0, s>>>(V, nv, n, w, st, r.part, r.counter, kmax);
   DMRG2_CHECK_LAUNCH();
 }
+}  // namespace
 
-void lz_loop_next(LanczosDev* st, cudaGraphConditionalHandle h, int kmax, cudaStream_t s) {
+template <typename T>
+void lz_step(T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, int kmax, int* host_done, cudaStream_t s) {
+  const StepGrid g = step_grid<T>(n);
+  if (g.blocks && g.cluster)
+    return step_launch<T, true>(g, V, nv, n, w, nullptr, st, r, kmax, 0, cudaGraphConditionalHandle{}, host_done, s);
+  if (g.blocks)
+    return step_launch<T, false>(g, V, nv, n, w, nullptr, st, r, kmax, 0, cudaGraphConditionalHandle{}, host_done, s);
+  step_passes<T>(V, nv, n, w, st, r, kmax, s);
+  if (nv < kmax) {
+    lz_normalize_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(V + (ll)nv * n, w, n, st);
+    DMRG2_CHECK_LAUNCH();
+  }
+  DMRG2_CUDA(cudaMemcpyAsync(host_done, &st->done, sizeof(int), cudaMemcpyDeviceToHost, s));
+}
+
+template <typename T>
+void lz_step_dev(T* V, ll n, T* w, T* cur, LanczosDev* st, RedScratch& r, int kmax, cudaGraphConditionalHandle h,
+                 cudaStream_t s) {
+  const StepGrid g = step_grid<T>(n);
+  if (g.blocks && g.cluster) return step_launch<T, true>(g, V, 0, n, w, cur, st, r, kmax, 1, h, nullptr, s);
+  if (g.blocks) return step_launch<T, false>(g, V, 0, n, w, cur, st, r, kmax, 1, h, nullptr, s);
+  step_passes<T>(V, -1, n, w, st, r, kmax, s);
+  lz_normalize_dev_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(V, cur, w, n, st);
+  DMRG2_CHECK_LAUNCH();
   lz_loop_next_kernel<<<1, 1, 0, s>>>(st, h, kmax);
   DMRG2_CHECK_LAUNCH();
 }
 
 template <typename T>
-void lz_ritz(const T* V, ll n, T* out, LanczosDev* st, RedScratch& r, cudaStream_t s) {
+void lz_ritz(const T* V, ll n, T* out, LanczosDev* st, RedScratch& r, LanczosHost* host, cudaStream_t s) {
+  const StepGrid g = step_grid<T>(n);
+  if (g.blocks && g.cluster) return ritz_launch<T, true>(g, V, n, out, st, r, host, s);
+  if (g.blocks) return ritz_launch<T, false>(g, V, n, out, st, r, host, s);
   lz_ritz_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(V, n, out, st);
   DMRG2_CHECK_LAUNCH();
   norm2<T>(out, n, &st->nrm2, r, s);
   scale_by_inv_sqrt_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(out, n, &st->nrm2);
+  DMRG2_CHECK_LAUNCH();
+  lz_report_kernel<<<1, 1, 0, s>>>(st, host);
+  DMRG2_CHECK_LAUNCH();
+}
+
+// The end of a warm-started split. As two norm kernels and three copies to the host this took
+// about 20 us of a bond (five latency-bound operations); the last block's report to
+// page-locked memory needs no copy.
+template <typename T>
+__global__ void __launch_bounds__(512)
+    split_finish_kernel(const T* __restrict__ theta, ll nt, const T* __restrict__ kept, ll nk,
+                        const int* status, const SvdOut* out, SplitHost* host, double* part, unsigned* counter) {
+  __shared__ double red[32];
+  const ll step = (ll)gridDim.x * blockDim.x, t0 = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+  double a = 0.0, b = 0.0;
+#pragma unroll 4
+  for (ll i = t0; i < nt; i += step) a += ST<T>::abs2(theta[i]);
+#pragma unroll 4
+  for (ll i = t0; i < nk; i += step) b += ST<T>::abs2(kept[i]);
+  a = block_sum(a, red);
+  b = block_sum(b, red);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = a;
+    part[gridDim.x + blockIdx.x] = b;
+  }
+  if (!arrive_last(counter, gridDim.x)) return;
+  if (threadIdx.x < 32) {  // fixed order: lane l adds blocks l, l+32, ..., then a shuffle tree
+    double s = 0.0, t = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += 32) {
+      s += __ldcg(part + i);
+      t += __ldcg(part + gridDim.x + i);
+    }
+    s = warp_sum(s);
+    t = warp_sum(t);
+    if (threadIdx.x == 0) {
+      volatile SplitHost* h = host;
+      h->theta2 = s;
+      h->kept2 = t;
+      h->failed = (*status || !(out->ns_done || out->ns_near)) ? 1 : 0;
+      *counter = 0u;
+    }
+  }
+}
+
+__global__ void split_begin_kernel(int* status, SvdOut* out, int k) {
+  SvdOut o{};
+  o.k = k;
+  *out = o;
+  *status = 0;
+}
+
+void split_begin(int* status, SvdOut* out, int k, cudaStream_t s) {
+  split_begin_kernel<<<1, 1, 0, s>>>(status, out, k);
+  DMRG2_CHECK_LAUNCH();
+}
+
+template <typename T>
+void split_finish(const T* theta, ll nt, const T* kept, ll nk, const int* status, const SvdOut* out, SplitHost* host,
+                  RedScratch& r, cudaStream_t s) {
+  // four elements of theta per thread, at most one block per SM (the sums of their partials are
+  // the serial end of the kernel)
+  const int g = (int)std::max<ll>(1, std::min<ll>(std::min(STEP_BLOCKS, r.nblk / 2), (nt + 2047) / 2048));
+  split_finish_kernel<T><<<g, 512, 0, s>>>(theta, nt, kept, nk, status, out, host, r.part, r.counter);
   DMRG2_CHECK_LAUNCH();
 }
 
@@ -544,15 +1129,14 @@ void scale_inplace(T* x, ll n, const double* nrm2_dev, cudaStream_t s) {
 }
 
 #define INST(T)                                                                                   \
-  template void lz_dots<T>(const T*, int, ll, const T*, LanczosDev*, RedScratch&, cudaStream_t); \
-  template void lz_update_dots<T>(const T*, int, ll, T*, LanczosDev*, RedScratch&, cudaStream_t);\
-  template void lz_update_norm_check<T>(const T*, int, ll, T*, LanczosDev*, RedScratch&, int, int,\
-                                        cudaStream_t);                                            \
-  template void lz_normalize_next<T>(T*, const T*, ll, LanczosDev*, cudaStream_t);                \
   template void lz_start<T>(T*, T*, ll, LanczosDev*, RedScratch&, unsigned, double, int,      \
                             cudaStream_t, T*, const unsigned*);                                   \
-  template void lz_step_dev<T>(const T*, ll, T*, T*, LanczosDev*, RedScratch&, int, cudaStream_t); \
-  template void lz_ritz<T>(const T*, ll, T*, LanczosDev*, RedScratch&, cudaStream_t);             \
+  template void lz_step<T>(T*, int, ll, T*, LanczosDev*, RedScratch&, int, int*, cudaStream_t);   \
+  template void lz_step_dev<T>(T*, ll, T*, T*, LanczosDev*, RedScratch&, int,                     \
+                               cudaGraphConditionalHandle, cudaStream_t);                         \
+  template void lz_ritz<T>(const T*, ll, T*, LanczosDev*, RedScratch&, LanczosHost*, cudaStream_t); \
+  template void split_finish<T>(const T*, ll, const T*, ll, const int*, const SvdOut*, SplitHost*, \
+                                RedScratch&, cudaStream_t);                                       \
   template void norm2<T>(const T*, ll, double*, RedScratch&, cudaStream_t);                       \
   template void scale_inplace<T>(T*, ll, const double*, cudaStream_t);
 INST(double)

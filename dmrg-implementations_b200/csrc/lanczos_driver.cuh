@@ -7,14 +7,12 @@
 //    no-op launches are issued after convergence;
 //  - device-looped: one CUDA graph per matvec identity (operator shapes and the fixed
 //    buffers it reads and writes) holds the whole solve: the start (norms, reset, first
-//    vector), a conditional WHILE node whose body is one Krylov step (matvec, the three
-//    vector passes, the normalisation, and a one-thread kernel that advances the index
-//    and ends the loop on convergence or after kmax bodies), then the Ritz vector and a
-//    copy of the solver state to pinned host memory. The host copies in a seed, launches
-//    the graph once per restart and waits once; no flags cross to the host between steps
-//    and no no-op steps are issued. A call site opts in by passing a key; solves run
-//    host-driven until a key is met the second time, when the solve is followed by the
-//    capture (graphs.cuh holds the cache).
+//    vector), a conditional WHILE node whose body is one Krylov step (matvec, then the
+//    step kernel, which also advances the index and ends the loop on convergence or after
+//    kmax bodies), then the Ritz vector, with the solver's report into pinned host memory.
+//    The host writes a seed there, launches the graph once per restart and waits once; no flags cross to the host between steps and no no-op steps are issued. A call
+//    site opts in by passing a key; solves run host-driven until a key is met the second
+//    time, when the solve is followed by the capture (graphs.cuh holds the cache).
 #pragma once
 
 #include <algorithm>
@@ -50,37 +48,34 @@ struct LanczosWork {
   LanczosDev* st = nullptr;
   RedScratch red;
   int* h_flags = nullptr;
-  LanczosDev* h_st = nullptr;
-  unsigned* h_seed = nullptr;  // the device-looped solve's seed, copied to st->seed_in
+  LanczosHost* h_st = nullptr;  // the solve's report (pinned, written by its last kernel)
+  unsigned* h_seed = nullptr;   // the device-looped solve's seed (pinned, read by its first kernel)
   std::vector<cudaEvent_t> ev_poll, ev_mv;
   std::vector<void*> owned;
 
-  void init(int kcap_, ll nmax) {
+  // timing: the host-driven form measures its matvecs (an event pair per Krylov step)
+  void init(int kcap_, ll nmax, bool timing = true) {
     graphs.cap = LZ_GRAPH_CAP;
     graphs.name = "lanczos";
     kcap = std::min(kcap_, KRYLOV_CAP);
-    krylov = (T*)alloc(sizeof(T) * (size_t)kcap * std::max<ll>(nmax, 1));
-    w = (T*)alloc(sizeof(T) * (size_t)std::max<ll>(nmax, 1));
-    cur = (T*)alloc(sizeof(T) * (size_t)std::max<ll>(nmax, 1));
-    st = (LanczosDev*)alloc(sizeof(LanczosDev));
-    red.nblk = vec_blocks(nmax);
-    red.part = (double*)alloc(sizeof(double) * (size_t)red.nblk * 2 * (KRYLOV_CAP + 2));
-    red.counter = (unsigned*)alloc(sizeof(unsigned) * 4);
+    red.nblk = red_blocks(nmax);
+    DevSlab slab;
+    slab.add(krylov, sizeof(T) * (size_t)kcap * std::max<ll>(nmax, 1));
+    slab.add(w, sizeof(T) * (size_t)std::max<ll>(nmax, 1));
+    slab.add(cur, sizeof(T) * (size_t)std::max<ll>(nmax, 1));
+    slab.add(st, sizeof(LanczosDev));
+    slab.add(red.part, sizeof(double) * (size_t)red.nblk * 2 * (KRYLOV_CAP + 2));
+    slab.add(red.counter, sizeof(unsigned) * 4);
+    owned.push_back(slab.commit());
     DMRG2_CUDA(cudaMemset(red.counter, 0, sizeof(unsigned) * 4));
     DMRG2_CUDA(cudaMemset(st, 0, sizeof(LanczosDev)));
     h_flags = (int*)host_pinned(sizeof(int) * POLL_RING);
-    h_st = (LanczosDev*)host_pinned(sizeof(LanczosDev));
+    h_st = (LanczosHost*)host_pinned(sizeof(LanczosHost));
     h_seed = (unsigned*)host_pinned(sizeof(unsigned));
     ev_poll.resize(POLL_RING);
     for (auto& e : ev_poll) DMRG2_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    ev_mv.resize(2 * KRYLOV_CAP);
+    ev_mv.resize(timing ? 2 * (size_t)kcap : 0);
     for (auto& e : ev_mv) DMRG2_CUDA(cudaEventCreate(&e));
-  }
-  void* alloc(size_t b) {
-    void* p = nullptr;
-    p = dev_alloc(b);
-    owned.push_back(p);
-    return p;
   }
   size_t bytes(ll nmax) const {
     return sizeof(T) * ((size_t)kcap + 2) * (size_t)nmax + sizeof(LanczosDev) +
@@ -113,14 +108,14 @@ struct LanczosResult {
 };
 
 // Captures one solve of W's buffers and this matvec into G (nothing runs): the start
-// (norms, reset with the seed read from st->seed_in, first vector), the WHILE node over
-// the Krylov steps, the Ritz vector and the copy of the solver state to W.h_st.
+// (norm, first vector), the WHILE node over the Krylov steps, the Ritz vector with the
+// report to W.h_st.
 template <typename T>
 void lz_build_graph(LanczosWork<T>& W, GraphEntry& G, T* theta, ll n, int kmax, double tol,
                     const std::function<void(const T*, T*, const int*)>& matvec, cudaStream_t s) {
   DMRG2_CUDA(cudaGraphCreate(&G.g, 0));
   G.fixed = capture_to_graph(s, G.g, [&]() {
-    lz_start(theta, W.krylov, n, W.st, W.red, 0u, tol, kmax, s, W.cur, &W.st->seed_in);
+    lz_start(theta, W.krylov, n, W.st, W.red, 0u, tol, kmax, s, W.cur, W.h_seed);
   });
   const cudaGraphNode_t start = graph_leaf(G.g);
   cudaGraphConditionalHandle h;
@@ -134,14 +129,12 @@ void lz_build_graph(LanczosWork<T>& W, GraphEntry& G, T* theta, ll n, int kmax, 
   DMRG2_CUDA(cudaGraphAddNode(&loop, G.g, &start, 1, &p));
   G.launches = capture_to_graph(s, p.conditional.phGraph_out[0], [&]() {
     matvec(W.cur, W.w, &W.st->done);
-    lz_step_dev(W.krylov, n, W.w, W.cur, W.st, W.red, kmax, s);
-    lz_loop_next(W.st, h, kmax, s);
+    lz_step_dev(W.krylov, n, W.w, W.cur, W.st, W.red, kmax, h, s);
   });
   G.fixed += capture_to_graph(
       s, G.g,
       [&]() {
-        lz_ritz(W.krylov, n, theta, W.st, W.red, s);
-        DMRG2_CUDA(cudaMemcpyAsync(W.h_st, W.st, sizeof(LanczosDev), cudaMemcpyDeviceToHost, s));
+        lz_ritz(W.krylov, n, theta, W.st, W.red, W.h_st, s);
       },
       &loop);
   graph_instantiate(W.graphs, G);
@@ -157,6 +150,7 @@ LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, d
                             const std::function<void(const T*, T*, const int*)>& matvec,
                             cudaStream_t s, const LzKey* key = nullptr) {
   LanczosResult res;
+  const bool timed = !W.ev_mv.empty();
   const int kmax = (int)std::min<ll>(std::min(krylov_max, W.kcap), n);
   if (kmax < 1) throw std::runtime_error("lanczos: empty problem");
   GraphEntry* G = nullptr;
@@ -178,15 +172,20 @@ LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, d
       build = true;
     }
   }
+  auto check_done = [&]() {
+    if (W.h_st->done && W.h_st->n_iter >= 1) return;
+    // (a grid barrier that gave up leaves its counters behind)
+    DMRG2_CUDA(cudaMemsetAsync(W.st, 0, sizeof(LanczosDev), s));
+    throw std::runtime_error("Lanczos did not terminate");
+  };
   for (int rs = 0; rs <= max_restarts; ++rs) {
     if (G && G->ex) {
-      // the pinned seed is read by this copy before the host writes it again (the wait below)
+      // the solve reads the pinned seed before the host writes it again (the wait below)
       *W.h_seed = seed + 104729u * (unsigned)rs;
-      DMRG2_CUDA(cudaMemcpyAsync(&W.st->seed_in, W.h_seed, sizeof(unsigned), cudaMemcpyHostToDevice, s));
       DMRG2_CUDA(cudaGraphLaunch(G->ex, s));
       W.graphs.replays += 1;
       DMRG2_CUDA(cudaStreamSynchronize(s));
-      if (!W.h_st->done || W.h_st->n_iter < 1) throw std::runtime_error("Lanczos did not terminate");
+      check_done();
       const int bodies = W.h_st->guard;
       launch_counter() += bodies * G->launches + G->fixed;
       thread_launches() += bodies * G->launches + G->fixed;
@@ -208,23 +207,18 @@ LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, d
         if (W.h_flags[jj % LanczosWork<T>::POLL_RING]) break;
       }
       T* vj = W.krylov + (ll)j * n;
-      DMRG2_CUDA(cudaEventRecord(W.ev_mv[2 * j], s));
+      if (timed) DMRG2_CUDA(cudaEventRecord(W.ev_mv[2 * j], s));
       matvec(vj, W.w, &W.st->done);
-      DMRG2_CUDA(cudaEventRecord(W.ev_mv[2 * j + 1], s));
-      lz_dots(W.krylov, j + 1, n, W.w, W.st, W.red, s);
-      lz_update_dots(W.krylov, j + 1, n, W.w, W.st, W.red, s);
-      lz_update_norm_check(W.krylov, j + 1, n, W.w, W.st, W.red, j, kmax, s);
-      if (j + 1 < kmax) lz_normalize_next(W.krylov + (ll)(j + 1) * n, W.w, n, W.st, s);
-      DMRG2_CUDA(cudaMemcpyAsync(&W.h_flags[j % LanczosWork<T>::POLL_RING], &W.st->done,
-                                 sizeof(int), cudaMemcpyDeviceToHost, s));
+      if (timed) DMRG2_CUDA(cudaEventRecord(W.ev_mv[2 * j + 1], s));
+      lz_step(W.krylov, j + 1, n, W.w, W.st, W.red, kmax, &W.h_flags[j % LanczosWork<T>::POLL_RING], s);
       DMRG2_CUDA(cudaEventRecord(W.ev_poll[j % LanczosWork<T>::POLL_RING], s));
       issued = j + 1;
     }
-    DMRG2_CUDA(cudaMemcpyAsync(W.h_st, W.st, sizeof(LanczosDev), cudaMemcpyDeviceToHost, s));
+    lz_ritz(W.krylov, n, theta, W.st, W.red, W.h_st, s);
     DMRG2_CUDA(cudaStreamSynchronize(s));
-    if (!W.h_st->done || W.h_st->n_iter < 1) throw std::runtime_error("Lanczos did not terminate");
+    check_done();
     const int used = std::min(issued, W.h_st->n_iter);
-    for (int j = 0; j < used; ++j) {
+    for (int j = 0; timed && j < used; ++j) {
       float ms = 0.f;
       DMRG2_CUDA(cudaEventElapsedTime(&ms, W.ev_mv[2 * j], W.ev_mv[2 * j + 1]));
       res.matvec_s += ms * 1e-3;
@@ -232,7 +226,6 @@ LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, d
     res.matvecs += used;
     res.iters += W.h_st->n_iter;
     res.energy = W.h_st->e_cur;
-    lz_ritz(W.krylov, n, theta, W.st, W.red, s);
     res.converged = W.h_st->converged;
     if (res.converged) break;
   }
