@@ -1,4 +1,5 @@
 #include "contract.cuh"
+#include "heff_small.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -151,6 +152,7 @@ template <typename T>
 void heff_apply(const T* Lenv, const T* Renv, const T* WWt, const T* in, T* out, T* X, T* Y, int cL,
                 int cR, int d, int Dl, int Dr, const int* skip, cudaStream_t s, const T* wsp) {
   const ll dd = (ll)d * d;
+  if (heff_small(Lenv, Renv, WWt, in, out, cL, cR, (int)dd, Dl, Dr, skip, s)) return;
   {
     Gemm<T> g;
     g.M = cL * Dl; g.N = (int)(dd * cR); g.K = cL;  // rows (a, w)
@@ -176,6 +178,7 @@ void heff_apply(const T* Lenv, const T* Renv, const T* WWt, const T* in, T* out,
 template <typename T>
 void heff1_apply(const T* Lenv, const T* Renv, const T* WmixL, const T* in, T* out, T* X, T* Y, int cL, int cR,
                  int d, int Dl, int Dr, const int* skip, cudaStream_t s) {
+  if (heff_small(Lenv, Renv, WmixL, in, out, cL, cR, d, Dl, Dr, skip, s)) return;
   {
     Gemm<T> g;  // X[a][w][(s,e)] = sum_c L[a][w][c] A[c][(s,e)]
     g.M = cL * Dl; g.N = d * cR; g.K = cL;
