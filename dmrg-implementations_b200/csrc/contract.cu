@@ -81,6 +81,53 @@ __global__ void __launch_bounds__(MIX_SPARSE_NT)
   }
 }
 
+// The same mixing for up to MIX_WIDE_K inputs (complex chains with d^2 D = 100, say): a CTA takes
+// one a and 32 columns e, stages all Kin inputs of them in shared memory, and its warps walk the
+// rows of W (nonzeros read through L1, the same for every lane). Bandwidth-bound on L2: X read
+// once, Y written once, and no work for W's zeros, which as a dense product on the tensor
+// cores cost 28% of a Josephson matvec's flops (187 of 10,000 entries are nonzero there).
+constexpr int MIX_WIDE_NT = 256;
+constexpr int MIX_WIDE_NNZ = 768;  // nonzeros staged in shared memory (more are read through L1)
+template <typename T>
+__global__ void __launch_bounds__(MIX_WIDE_NT)
+    mpo_mix_wide_kernel(const T* __restrict__ X, const T* __restrict__ val, const int* __restrict__ rowp,
+                        T* __restrict__ Y, int Kin, int Kout, int cR, ll sX, ll sY, const int* skip) {
+  if (skip && *((volatile const int*)skip)) return;
+  extern __shared__ __align__(16) unsigned char mix_smem[];
+  T* xs = reinterpret_cast<T*>(mix_smem);  // [Kin][32]
+  __shared__ T vs[MIX_WIDE_NNZ];
+  __shared__ int cs[MIX_WIDE_NNZ], rp[MIX_WIDE_K + 1];
+  constexpr int W = MIX_WIDE_NT / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e = blockIdx.x * 32 + lane;
+  const bool in = e < cR;
+  const T* xa = X + blockIdx.y * sX + e;
+  T* ya = Y + blockIdx.y * sY + e;
+  const int* col = rowp + Kout + 1;
+#pragma unroll 8
+  for (int k = warp; k < Kin; k += W) xs[k * 32 + lane] = in ? xa[(ll)k * cR] : ST<T>::zero();
+  for (int i = threadIdx.x; i <= Kout; i += MIX_WIDE_NT) rp[i] = rowp[i];
+  // (the slots behind the last nonzero exist: the block holds Kin Kout of them)
+  const int st = min(MIX_WIDE_NNZ, Kin * Kout);
+  for (int i = threadIdx.x; i < st; i += MIX_WIDE_NT) {
+    cs[i] = col[i] * 32;
+    vs[i] = val[i];
+  }
+  __syncthreads();
+  const bool staged = rp[Kout] <= MIX_WIDE_NNZ;
+  for (int o = warp; o < Kout; o += W) {
+    const int j0 = rp[o], j1 = rp[o + 1];
+    T acc = ST<T>::zero();
+    if (staged) {
+      for (int j = j0; j < j1; ++j) acc = acc + ST<T>::mul(vs[j], xs[cs[j] + lane]);
+    } else {
+#pragma unroll 4
+      for (int j = j0; j < j1; ++j) acc = acc + ST<T>::mul(val[j], xs[col[j] * 32 + lane]);
+    }
+    if (in) ya[(ll)o * cR] = acc;
+  }
+}
+
 template <typename T>
 int wwt_sparse_block(std::vector<T>& w, int Kin, int Kout) {
   const ll kk = (ll)Kin * Kout;
@@ -119,6 +166,14 @@ static void mix_rows(const T* X, const T* W, T* Y, int cL, int cR, int Kin, int 
     mpo_mix_sparse_kernel<T><<<grid, MIX_SPARSE_NT, 0, s>>>(X, wsp, (const int*)(wsp + kk), Y, Kin, Kout, cR,
                                                             (ll)Kin * cR, (ll)Kout * cR, skip);
     DMRG2_CHECK_LAUNCH();
+  } else if (wsp && Kin <= MIX_WIDE_K && Kout <= MIX_WIDE_K && cL <= 65535) {
+    const ll kk = (ll)Kin * Kout;
+    static std::atomic<unsigned long long> attr{0};
+    set_smem_attr_once(attr, (const void*)mpo_mix_wide_kernel<T>, (int)(sizeof(T) * MIX_WIDE_K * 32));
+    dim3 grid(ceil_div(cR, 32), cL);
+    mpo_mix_wide_kernel<T><<<grid, MIX_WIDE_NT, sizeof(T) * (size_t)Kin * 32, s>>>(X, wsp, (const int*)(wsp + kk), Y, Kin, Kout,
+                                                                           cR, (ll)Kin * cR, (ll)Kout * cR, skip);
+    DMRG2_CHECK_LAUNCH();
   } else if (Kin <= 32 && Kout <= 32 && cL <= 65535) {
     dim3 grid(ceil_div(cR, 128), cL);
     mpo_mix_kernel<T, 32><<<grid, 128, 0, s>>>(X, W, Y, Kin, Kout, cR, (ll)Kin * cR, (ll)Kout * cR, skip);
@@ -150,7 +205,7 @@ void heff_apply_split(const T* Lenv, const T* Renv, const T* WWt, const T* in, T
 
 template <typename T>
 void heff_apply(const T* Lenv, const T* Renv, const T* WWt, const T* in, T* out, T* X, T* Y, int cL,
-                int cR, int d, int Dl, int Dr, const int* skip, cudaStream_t s, const T* wsp) {
+                int cR, int d, int Dl, int Dr, const int* skip, cudaStream_t s, const T* wsp, const int* dense) {
   const ll dd = (ll)d * d;
   if (heff_small(Lenv, Renv, WWt, in, out, cL, cR, (int)dd, Dl, Dr, skip, s)) return;
   {
@@ -162,7 +217,12 @@ void heff_apply(const T* Lenv, const T* Renv, const T* WWt, const T* in, T* out,
     g.skip = skip;
     launch_gemm(g, s);
   }
-  mix_rows(X, WWt, Y, cL, cR, (int)(Dl * dd), (int)(dd * Dr), skip, s, wsp);
+  if (wsp && dense) {  // which form serves is known on the device only; the other one returns at once
+    mix_rows(X, WWt, Y, cL, cR, (int)(Dl * dd), (int)(dd * Dr), dense, s, wsp);
+    mix_rows<T>(X, WWt, Y, cL, cR, (int)(Dl * dd), (int)(dd * Dr), dense + 1, s);
+  } else {
+    mix_rows(X, WWt, Y, cL, cR, (int)(Dl * dd), (int)(dd * Dr), skip, s, wsp);
+  }
   {
     Gemm<T> g;
     g.tb = true;
@@ -331,7 +391,7 @@ void build_wmix_right(const T* W, int Dl, int Dr, int d, std::vector<T>& out) {
 
 #define INST(T)                                                                                 \
   template void heff_apply<T>(const T*, const T*, const T*, const T*, T*, T*, T*, int, int, int, \
-                              int, int, const int*, cudaStream_t, const T*);                     \
+                              int, int, const int*, cudaStream_t, const T*, const int*);         \
   template int wwt_sparse_block<T>(std::vector<T>&, int, int);                                  \
   template void heff1_apply<T>(const T*, const T*, const T*, const T*, T*, T*, T*, int, int, int,  \
                                int, int, const int*, cudaStream_t);                              \

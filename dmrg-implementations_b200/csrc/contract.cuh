@@ -23,10 +23,15 @@ namespace dmrg2 {
 //   step 3: out[a][p][q][f]  = sum_{n,e} Y[a][p][q][n][e] R[f][n][e]  (one GEMM, K = Dr*cR)
 //
 // wsp, when given, is the nonzero form of WWt (wwt_sparse_block below): step 2 then sums
-// only the nonzero entries, in the same column order, so the result is the same.
+// only the nonzero entries, in the same column order, so the result is the same. dense, when
+// given with it, points to two device flags (W is dense, W is not): step 2 takes the form
+// they say (a caller whose W is only on the device; skip must be null).
 template <typename T>
 void heff_apply(const T* Lenv, const T* Renv, const T* WWt, const T* in, T* out, T* X, T* Y, int cL,
-                int cR, int d, int Dl, int Dr, const int* skip, cudaStream_t s, const T* wsp = nullptr);
+                int cR, int d, int Dl, int Dr, const int* skip, cudaStream_t s, const T* wsp = nullptr,
+                const int* dense = nullptr);
+
+constexpr int MIX_WIDE_K = 128;  // largest d^2 D the nonzero form of the mixing serves
 
 // The fused two-site MPO of a bond as the engine stores it, one block: the dense Kout x Kin
 // matrix WWt, then its nonzeros row by row (Kout x Kin slots for values), then, as ints, the

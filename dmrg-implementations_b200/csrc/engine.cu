@@ -166,7 +166,7 @@ class Engine final : public EngineBase {
     for (int i = 0; i + 1 < L_; ++i) {
       const int Kin = Dl[i] * d_ * d_, Kout = d_ * d_ * Dr[i + 1];
       const int nnz = wwt_sparse_block(hww[i], Kin, Kout);
-      wwt_sparse_[i] = (!mix_dense && 2 * (ll)nnz <= (ll)Kin * Kout && Kin <= 32 && Kout <= 32) ? 1 : 0;
+      wwt_sparse_[i] = (!mix_dense && 2 * (ll)nnz <= (ll)Kin * Kout && Kin <= MIX_WIDE_K && Kout <= MIX_WIDE_K) ? 1 : 0;
     }
     // contraction scratch
     ll xs = 1;

@@ -123,6 +123,60 @@ __global__ void wwt_kernel(const T* __restrict__ WL, const T* __restrict__ WR, T
   out[i] = acc;
 }
 
+// The nonzero form of the dense W (Kout x Kin, both <= MIX_WIDE_K) in wwt_sparse_block's layout, by one
+// CTA: all rows read at once into registers, row counts, their prefix sums, then columns and
+// values; flags[0] = W is dense (more than half its entries are nonzero), flags[1] = it is not.
+template <typename T>
+__global__ void __launch_bounds__(1024) wwt_nonzeros_kernel(const T* __restrict__ W, T* __restrict__ val,
+                                                            int* __restrict__ rowp, int Kin, int Kout, int* flags) {
+  constexpr int R = MIX_WIDE_K / 32;  // rows per warp, column groups per row
+  __shared__ int cnt[MIX_WIDE_K];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned mask[R][R];
+#pragma unroll
+  for (int h = 0; h < R; ++h) {
+    const int o = warp + 32 * h;
+    T v[R];
+#pragma unroll
+    for (int g = 0; g < R; ++g) v[g] = (o < Kout && 32 * g + lane < Kin) ? W[(ll)o * Kin + 32 * g + lane] : ST<T>::zero();
+    int n = 0;
+#pragma unroll
+    for (int g = 0; g < R; ++g) {
+      mask[h][g] = __ballot_sync(0xffffffffu, ST<T>::abs2(v[g]) != 0.0);
+      n += __popc(mask[h][g]);
+    }
+    if (lane == 0) cnt[o] = n;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < R; ++h) {
+    const int o = warp + 32 * h;
+    if (o >= Kout) break;
+    int pos = 0;
+    for (int i = lane; i < o; i += 32) pos += cnt[i];
+    for (int s = 16; s > 0; s >>= 1) pos += __shfl_xor_sync(0xffffffffu, pos, s);
+    if (lane == 0) {
+      rowp[o] = pos;
+      if (o == Kout - 1) {
+        const int nnz = pos + cnt[o];
+        rowp[Kout] = nnz;
+        flags[0] = 2 * nnz > Kin * Kout ? 1 : 0;
+        flags[1] = 1 - flags[0];
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < R; ++g) {
+      const unsigned m = mask[h][g];
+      if ((m >> lane) & 1u) {
+        const int j = pos + __popc(m & ((1u << lane) - 1u)), k = 32 * g + lane;
+        val[j] = W[(ll)o * Kin + k];
+        rowp[Kout + 1 + j] = k;
+      }
+      pos += __popc(m);
+    }
+  }
+}
+
 }  // namespace
 
 size_t heff_noalloc_scratch_bytes(int cL, int cR, int d, int Dl, int Dr, size_t scalar_bytes) {
@@ -164,6 +218,26 @@ void heff_noalloc(int cL, int cR, int d, int Dl, int Dm, int Dr, const T* L, con
   const ll entries = dd * Dr * Dl * dd;
   wwt_kernel<T><<<(unsigned)((entries + 255) / 256), 256, 0, s>>>(WL, WR, WWt, Dl, Dm, Dr, d);
   DMRG2_CHECK_LAUNCH();
+  // A large mixing step goes over W's nonzeros, where the scratch has room for that form beside
+  // the rest (its size does not count against the caller's limit). Building it and the launch that
+  // returns at once cost about 6 us, the mixing then its traffic; the batched GEMM on the dense
+  // W runs at about 25 TFLOP/s of its padded size. Josephson, d = 5 (us per matvec, nonzeros /
+  // dense): 64 x 64 49 / 46, 96 x 96 91 / 107, 128 x 128 155 / 181. At most 32 inputs the
+  // dense kernel is as fast.
+  const int Kin = (int)(Dl * dd), Kout = (int)(dd * Dr);
+  const size_t sp_b = round256((size_t)wwt_block_elems(Kin, Kout, sizeof(T)) * sizeof(T)) + 256;
+  const double dense_us = 2e6 * (ST<T>::cplx ? 4.0 : 1.0) * cL * (double)cR * (ceil_div(Kout, 32) * 32.0) * Kin / 25e12;
+  const double nonzero_us = 6.0 + 1e6 * sizeof(T) * (double)cL * cR * (Kin + Kout) / 4e12;
+  if ((Kin > 32 || Kout > 32) && Kin <= MIX_WIDE_K && Kout <= MIX_WIDE_K && need + sp_b <= NOALLOC_SCRATCH_BYTES &&
+      dense_us > nonzero_us) {
+    T* val = (T*)(base + wwt_b + 2 * xs_b);
+    int* rowp = (int*)(val + (ll)Kin * Kout);
+    int* flags = (int*)(base + wwt_b + 2 * xs_b + sp_b - 256);
+    wwt_nonzeros_kernel<T><<<1, 1024, 0, s>>>(WWt, val, rowp, Kin, Kout, flags);
+    DMRG2_CHECK_LAUNCH();
+    heff_apply<T>(L, R, WWt, theta, out, X, Y, cL, cR, d, Dl, Dr, nullptr, s, val, flags);
+    return;
+  }
   heff_apply<T>(L, R, WWt, theta, out, X, Y, cL, cR, d, Dl, Dr, nullptr, s);
 }
 
