@@ -11,11 +11,11 @@
 // the peer's shared memory. A published tile is never written again, and nothing is
 // copied asynchronously, so the only exit condition is the final cluster barrier
 // (no CTA leaves while a peer may still read it). Per tile column t:
-//   P  CTA r > t: L_rt = A_rt X_tt^T with X_tt = L_tt^{-1} from CTA t (rows split
-//      over the 8 warps);
+//   P  CTA r > t: L_rt = A_rt X_tt^T with X_tt = L_tt^{-1}, whose fragments every warp reads
+//      straight from CTA t (one 16 x 8 piece per warp, FP64 tensor cores);
 //   T  CTA r > t: A_rj -= L_rt L_jt^T for the peers' tiles t < j < r (one warp per
-//      tile, the peer tile staged in that warp's buffer) and the lower part of the
-//      diagonal tile j = r (rows split over the warps);
+//      tile, the fragments of L_jt straight from CTA j) and the diagonal tile j = r (one 16 x 8
+//      piece per warp);
 //   D  CTA t, once its row is updated: in-register Cholesky of the diagonal tile
 //      (one warp, lane = row; the chain of pivots is the critical path), then X_tt by
 //      forward substitution (lane = column), then the counter says "row complete".
@@ -23,6 +23,12 @@
 // wider updates of the rows further down overlap with it. A poll that runs out marks
 // the result invalid (status) and the CTA carries on with what it has, so every CTA
 // reaches the final barrier.
+// The pivots of D go in blocks of 8 columns: inside a block a pivot's column reaches the others
+// by shuffles, behind it the finished 8 columns update the rest of the tile through shared
+// memory as one rank-8 product. Shuffling every column to all 31 others instead put ~265
+// cycles of issue between two pivots (35 us of a factor at k = 256).
+// Per factor at k = 256: 89.6 us before (fused multiply-add loops for P and T on staged
+// copies, 32-column shuffles in D), 67.6 us now.
 //
 // trsm_rows_kernel: Y = Z L^{-T}, 16 rows of Z per CTA, column block by column block:
 // Y_b = (Z_b - sum_{j<b} Y_j L_bj^T) X_bb^T on the FP64 tensor cores (DMMA), the tiles
@@ -39,7 +45,7 @@ namespace dmrg2 {
 namespace {
 
 constexpr int NB = CHOL_NB;
-constexpr int TP = NB + 1;           // padded tile row in shared memory (conflict-free columns)
+constexpr int TP = NB + 3;           // padded tile row: conflict-free down a column, two-way for fragments
 constexpr int TT = NB * TP;          // doubles per padded tile
 constexpr int CT_THREADS = 256;      // 8 warps
 constexpr int CT_WARPS = CT_THREADS / 32;
@@ -61,58 +67,105 @@ __device__ inline bool wait_tiles(const int* peer_done, int need) {
 }
 
 // column J of the in-register Cholesky of one diagonal tile (lane i holds row i) with a
-// reciprocal square root per pivot, then the columns after it; compile-time J keeps
-// every index of a[] static
+// reciprocal square root per pivot, then the columns after it (those of its block of 8 at
+// once, the rest at the block's end from blk, [NB][8] in shared memory); compile-time J keeps
+// every index of a[] static. Entries above the diagonal are left undefined.
 template <int J>
 __device__ __forceinline__ void tile_chol_col(double (&a)[NB], int lane, double piv_min, double piv_sub, bool& bad,
-                                              double* rd) {
+                                              double* rd, double* blk) {
+  constexpr int B0 = J & ~7, BE = B0 + 8;
   double piv = __shfl_sync(0xffffffffu, a[J], J);
   if (!(piv > piv_min)) {  // also catches NaN
     bad = true;
     piv = piv_sub;
   }
   const double r = rsqrt(piv);
-  if (lane == J) {
-    a[J] = piv * r;
-    rd[J] = r;
-  } else if (lane > J) {
-    a[J] *= r;
-  }
+  if (lane == J) rd[J] = r;
+  a[J] = (lane == J ? piv : a[J]) * r;
 #pragma unroll
-  for (int c = J + 1; c < NB; ++c) {
+  for (int c = J + 1; c < BE; ++c) {
     const double lc = __shfl_sync(0xffffffffu, a[J], c);
-    if (lane >= c) a[c] -= a[J] * lc;
+    a[c] -= a[J] * lc;
   }
-  if constexpr (J + 1 < NB) tile_chol_col<J + 1>(a, lane, piv_min, piv_sub, bad, rd);
+  if constexpr (J + 1 == BE && BE < NB) {
+    double2* row = reinterpret_cast<double2*>(blk + lane * 8);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) row[q] = make_double2(a[B0 + 2 * q], a[B0 + 2 * q + 1]);
+    __syncwarp();
+#pragma unroll
+    for (int c = BE; c < NB; ++c) {
+      const double2* l = reinterpret_cast<const double2*>(blk + c * 8);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double2 v = l[q];
+        a[c] -= a[B0 + 2 * q] * v.x;
+        a[c] -= a[B0 + 2 * q + 1] * v.y;
+      }
+    }
+    __syncwarp();
+  }
+  if constexpr (J + 1 < NB) tile_chol_col<J + 1>(a, lane, piv_min, piv_sub, bad, rd, blk);
+}
+
+// acc += sign * A B^T for 16 rows of A and 8 rows of B, k = 0 .. NB-1; b[k step][2]: the
+// fragments of B (row g of the 8, columns 8 k + t and 8 k + t + 4)
+__device__ __forceinline__ void piece_mma(double (&acc)[4], const double* A, double sign, const double (&b)[NB / 8][2],
+                                          int gq, int tq) {
+#pragma unroll
+  for (int k = 0; k < NB / 8; ++k) {
+    const double* p = A + gq * TP + 8 * k + tq;
+    dmma16x8x8(acc, sign * p[0], sign * p[8 * TP], sign * p[4], sign * p[8 * TP + 4], b[k][0], b[k][1]);
+  }
+}
+__device__ __forceinline__ void load_frag(double (&b)[NB / 8][2], const double* B, int gq, int tq) {
+#pragma unroll
+  for (int k = 0; k < NB / 8; ++k) {
+    b[k][0] = B[gq * TP + 8 * k + tq];
+    b[k][1] = B[gq * TP + 8 * k + tq + 4];
+  }
 }
 
 template <int C>
 __global__ void __launch_bounds__(CT_THREADS, 1)
     chol_tiles_kernel(const double* __restrict__ G, int k, int nb, ll ldg, double* __restrict__ LX, ll ldx,
-                      int* __restrict__ status, double rel_tol, double shift_rel) {
+                      int* __restrict__ status, double rel_tol, double shift_rel, double* __restrict__ dscale) {
   cg::cluster_group cluster = cg::this_cluster();
   const int r = (int)cluster.block_rank();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
+  const int pr = (warp >> 2) * 16, pc = (warp & 3) * 8;  // this warp's 16 x 8 piece of a tile
   extern __shared__ __align__(16) double ctsm[];
   double* Lt = ctsm;                 // [C] tiles of block row r: A_rj, turned into L_rj
   double* Xr = Lt + C * TT;          // X_rr = L_rr^{-1} (zeros above the diagonal)
-  double* Xs = Xr + TT;              // X_tt of the tile column being solved, staged
-  double* Ws = Xs + TT;              // [CT_WARPS] a peer's L_jt, staged per warp
-  double* Rd = Ws + CT_WARPS * TT;   // 1 / diag of L_rr
+  double* blk = Xr + TT;             // [NB][8] finished columns of D's current block
+  double* Rd = blk + NB * 8;         // 1 / diag of L_rr
   __shared__ int done_s;             // tiles of this block row that are final (read by peers)
   __shared__ int fail_s;
   __shared__ double tr_s, dmax_s;
+  __shared__ double ds[CHOL_MAX];    // scale of each column
   auto T_ = [](double* base, int t) { return base + t * TT; };
 
   if (tid == 0) {
     done_s = 0;
     fail_s = 0;
   }
+  bool bad = false;
+  for (int i = tid; i < k; i += CT_THREADS) {
+    double sc = 1.0;
+    if (dscale) {
+      const double g = G[(ll)i * ldg + i];
+      const bool ok = g > 0.0 && isfinite(g);
+      sc = ok ? rsqrt(g) : 0.0;
+      bad = bad || !ok;
+      if (r == 0) dscale[i] = sc;
+    }
+    ds[i] = sc;
+  }
+  __syncthreads();
   // trace and largest diagonal entry of G (every CTA reads them from global memory)
   if (warp == 0) {
     double m = 0.0, tr = 0.0;
     for (int i = lane; i < k; i += 32) {
-      const double a = G[(ll)i * ldg + i];
+      const double a = G[(ll)i * ldg + i] * ds[i] * ds[i];
       m = fmax(m, a);
       tr += a;
     }
@@ -136,7 +189,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
         const int row = e >> 5, col = e & 31;
         const int gi = r * NB + row, gj = j * NB + col;
         double v;
-        if (gi < k && gj < k) v = (j < r || col <= row) ? G[(ll)gi * ldg + gj] + (gi == gj ? shift : 0.0) : 0.0;
+        if (gi < k && gj < k) v = (j < r || col <= row) ? G[(ll)gi * ldg + gj] * ds[gi] * ds[gj] + (gi == gj ? shift : 0.0) : 0.0;
         else v = (gi == gj) ? 1.0 : 0.0;
         T_(Lt, j)[row * TP + col] = v;
       }
@@ -144,77 +197,54 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
   // or writes LX (which may be the buffer G is in)
   cluster.sync();
 
-  bool bad = false;
   if (r < nb) {
     for (int t = 0; t < r; ++t) {
-      // ---- P: L_rt = A_rt X_tt^T once CTA t has published X_tt (its row complete); one
-      // thread polls (the peer's shared memory serves its critical factorisation meanwhile)
-      // and the CTA barrier passes what it acquired on to the other threads
-      if (tid == 0 && !wait_tiles(cluster.map_shared_rank(&done_s, t), t + 1)) fail_s = 1;
-      __syncthreads();
+      // ---- P: L_rt = A_rt X_tt^T once CTA t has published X_tt (its row complete)
+      if (lane == 0 && !wait_tiles(cluster.map_shared_rank(&done_s, t), t + 1)) fail_s = 1;
+      __syncwarp();  // lane 0 acquired the tile for the warp
+      double* Art = T_(Lt, t);
       {
-        const double* Xp = cluster.map_shared_rank(Xr, t);
-        for (int e = tid; e < NB * NB; e += CT_THREADS) Xs[(e >> 5) * TP + (e & 31)] = Xp[(e >> 5) * TP + (e & 31)];
-      }
-      __syncthreads();
-      {
-        double* Art = T_(Lt, t);
-        double o[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-        for (int s = 0; s < NB; ++s) {
-          const double xv = Xs[lane * TP + s];  // X_tt[c = lane][s]
+        double b[NB / 8][2], o[4] = {0.0, 0.0, 0.0, 0.0};
+        load_frag(b, cluster.map_shared_rank(Xr, t) + pc * TP, gq, tq);
+        piece_mma(o, Art + pr * TP, 1.0, b, gq, tq);
+        __syncthreads();  // the tile is read before it is overwritten
 #pragma unroll
-          for (int u = 0; u < 4; ++u) o[u] += Art[(4 * warp + u) * TP + s] * xv;
-        }
-        __syncwarp();  // the warp's rows are read before they are overwritten
-#pragma unroll
-        for (int u = 0; u < 4; ++u) Art[(4 * warp + u) * TP + lane] = o[u];
+        for (int q = 0; q < 4; ++q) Art[(pr + gq + ((q & 2) ? 8 : 0)) * TP + pc + 2 * tq + (q & 1)] = o[q];
       }
       __syncthreads();
       if (tid == 0) st_release_cluster(&done_s, t + 1);  // L_rt is final
-      // ---- T: A_rj -= L_rt L_jt^T for t < j <= r
-      const double* Lrt = T_(Lt, t);
+      // ---- T: A_rj -= L_rt L_jt^T for t < j <= r; the diagonal tile first (the next D needs it)
+      const double* Lrt = Art;
+      {
+        double* Arr = T_(Lt, r);
+        double b[NB / 8][2], o[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) o[q] = Arr[(pr + gq + ((q & 2) ? 8 : 0)) * TP + pc + 2 * tq + (q & 1)];
+        load_frag(b, Lrt + pc * TP, gq, tq);
+        piece_mma(o, Lrt + pr * TP, -1.0, b, gq, tq);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) Arr[(pr + gq + ((q & 2) ? 8 : 0)) * TP + pc + 2 * tq + (q & 1)] = o[q];
+      }
       for (int q = warp; q < r - t - 1; q += CT_WARPS) {  // the peers' tiles j = t+1 .. r-1
         const int j = t + 1 + q;
         if (lane == 0 && !wait_tiles(cluster.map_shared_rank(&done_s, j), t + 1)) fail_s = 1;
-        __syncwarp();  // lane 0 acquired the tile for the warp
-        const double* src = cluster.map_shared_rank(T_(Lt, t), j);  // L_jt in CTA j
-        double* W = T_(Ws, warp);
-        {
-          double v[NB];
-#pragma unroll
-          for (int c = 0; c < NB; ++c) v[c] = src[c * TP + lane];
-#pragma unroll
-          for (int c = 0; c < NB; ++c) W[c * TP + lane] = v[c];
-        }
         __syncwarp();
-        double x[NB], acc[NB];  // lane = row i of A_rj: acc[c] = sum_s L_rt[i][s] L_jt[c][s]
+        const double* src = cluster.map_shared_rank(T_(Lt, t), j);  // L_jt in CTA j
+        double b[4][NB / 8][2];
 #pragma unroll
-        for (int s = 0; s < NB; ++s) {
-          x[s] = Lrt[lane * TP + s];
-          acc[s] = 0.0;
-        }
-#pragma unroll
-        for (int s = 0; s < NB; ++s)
-#pragma unroll
-          for (int c = 0; c < NB; ++c) acc[c] += x[s] * W[c * TP + s];
+        for (int c = 0; c < 4; ++c) load_frag(b[c], src + 8 * c * TP, gq, tq);
         double* Arj = T_(Lt, j);
 #pragma unroll
-        for (int c = 0; c < NB; ++c) Arj[lane * TP + c] -= acc[c];
-        __syncwarp();  // W is staged again by this warp's next tile
-      }
-      {  // the diagonal tile: rows 4w .. 4w+3, lane = column, lower part only
-        double* Arr = T_(Lt, r);
-        double o[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-        for (int s = 0; s < NB; ++s) {
-          const double lv = Lrt[lane * TP + s];
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int u = 0; u < 4; ++u) o[u] += Lrt[(4 * warp + u) * TP + s] * lv;
-        }
+          for (int c = 0; c < 4; ++c) {
+            double o[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (lane <= 4 * warp + u) Arr[(4 * warp + u) * TP + lane] -= o[u];
+            for (int e = 0; e < 4; ++e) o[e] = Arj[(16 * h + gq + ((e & 2) ? 8 : 0)) * TP + 8 * c + 2 * tq + (e & 1)];
+            piece_mma(o, Lrt + 16 * h * TP, -1.0, b[c], gq, tq);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) Arj[(16 * h + gq + ((e & 2) ? 8 : 0)) * TP + 8 * c + 2 * tq + (e & 1)] = o[e];
+          }
       }
       __syncthreads();  // tile (r, t+1) and the diagonal tile are final for this column
     }
@@ -224,7 +254,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
       double a[NB];
 #pragma unroll
       for (int j = 0; j < NB; ++j) a[j] = (j <= lane) ? Lrr[lane * TP + j] : 0.0;
-      tile_chol_col<0>(a, lane, piv_min, piv_sub, bad, Rd);
+      tile_chol_col<0>(a, lane, piv_min, piv_sub, bad, Rd, blk);
 #pragma unroll
       for (int j = 0; j < NB; ++j) Lrr[lane * TP + j] = (j <= lane) ? a[j] : 0.0;
       __syncwarp();
@@ -281,7 +311,7 @@ __device__ inline void tr_stage(double* dst, const double* LX, ll ldx, int b, in
 
 __global__ void __launch_bounds__(TR_THREADS)
     trsm_rows_kernel(const double* __restrict__ Z, ll rows, int k, int nb, const double* __restrict__ LX, ll ldx,
-                     double* __restrict__ Y, const int* __restrict__ status) {
+                     double* __restrict__ Y, const int* __restrict__ status, const double* __restrict__ dscale) {
   if (*((volatile const int*)status)) return;  // the factor is not valid: the caller falls back
   extern __shared__ __align__(16) double tsm[];
   const int YP = nb * NB + 4;     // row of the finished blocks
@@ -314,7 +344,7 @@ __global__ void __launch_bounds__(TR_THREADS)
     for (int q = 0; q < 4; ++q) {
       const ll row = r0 + gq + ((q & 2) ? 8 : 0);
       const int col = c0 + (q & 1);
-      acc[q] = (row < rows && col < k) ? Z[row * k + col] : 0.0;
+      acc[q] = (row < rows && col < k) ? Z[row * k + col] * (dscale ? dscale[col] : 1.0) : 0.0;
     }
     for (int j = 0; j <= b; ++j, ++s) {
       if (j == b) {
@@ -416,14 +446,10 @@ __global__ void __launch_bounds__(256) col_scale_kernel(double* __restrict__ Y, 
     for (ll r = r0 + warp; r < r1; r += 8) Y[r * k + c] *= inv[lane];
 }
 
-__global__ void mark_unconverged_kernel(const SvdOut* out, int* status) {
-  if (!out->ns_done) *status = 1;
-}
-
 template <int C>
 void chol_tiles_launch(const double* G, int k, int nb, ll ldg, double* LX, ll ldx, int* status, double rel_tol,
-                       double shift_rel, cudaStream_t s) {
-  constexpr size_t smem = sizeof(double) * ((size_t)(C + 2 + CT_WARPS) * TT + NB);
+                       double shift_rel, double* dscale, cudaStream_t s) {
+  constexpr size_t smem = sizeof(double) * ((size_t)(C + 1) * TT + NB * 8 + NB);
   static std::atomic<unsigned long long> attr{0};
   set_smem_attr_once(attr, (const void*)chol_tiles_kernel<C>, (int)smem);
   if constexpr (C > 8) {
@@ -442,16 +468,12 @@ void chol_tiles_launch(const double* G, int k, int nb, ll ldg, double* LX, ll ld
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  DMRG2_CUDA(cudaLaunchKernelEx(&cfg, chol_tiles_kernel<C>, G, k, nb, ldg, LX, ldx, status, rel_tol, shift_rel));
+  DMRG2_CUDA(cudaLaunchKernelEx(&cfg, chol_tiles_kernel<C>, G, k, nb, ldg, LX, ldx, status, rel_tol, shift_rel,
+                                dscale));
   DMRG2_CHECK_LAUNCH();
 }
 
 }  // namespace
-
-void mark_unconverged(const SvdOut* out, int* status, cudaStream_t s) {
-  mark_unconverged_kernel<<<1, 1, 0, s>>>(out, status);
-  DMRG2_CHECK_LAUNCH();
-}
 
 void col_normalize(double* Y, ll rows, int k, double* part, int* status, cudaStream_t s) {
   if (rows < 1 || k < 1) return;
@@ -465,17 +487,17 @@ void col_normalize(double* Y, ll rows, int k, double* part, int* status, cudaStr
 }
 
 void chol_tiles(const double* G, int k, ll ldg, double* LX, ll ldx, int* status, double rel_tol, double shift_rel,
-                cudaStream_t s) {
+                cudaStream_t s, double* dscale) {
   const int np = chol_padded(k);
   if (k < 1 || np > CHOL_MAX) throw std::invalid_argument("chol_tiles: order outside 1..512");
   if (ldg < k || ldx < np) throw std::invalid_argument("chol_tiles: leading dimension too small");
   const int nb = np / NB;
-  if (nb <= 8) chol_tiles_launch<8>(G, k, nb, ldg, LX, ldx, status, rel_tol, shift_rel, s);
-  else chol_tiles_launch<16>(G, k, nb, ldg, LX, ldx, status, rel_tol, shift_rel, s);
+  if (nb <= 8) chol_tiles_launch<8>(G, k, nb, ldg, LX, ldx, status, rel_tol, shift_rel, dscale, s);
+  else chol_tiles_launch<16>(G, k, nb, ldg, LX, ldx, status, rel_tol, shift_rel, dscale, s);
 }
 
 void trsm_rows(const double* Z, ll rows, int k, const double* LX, ll ldx, double* Y, const int* status,
-               cudaStream_t s) {
+               cudaStream_t s, const double* dscale) {
   if (rows < 1) return;
   const int np = chol_padded(k);
   if (k < 1 || np > CHOL_MAX) throw std::invalid_argument("trsm_rows: order outside 1..512");
@@ -487,7 +509,7 @@ void trsm_rows(const double* Z, ll rows, int k, const double* LX, ll ldx, double
   set_smem_attr_once(attr, (const void*)trsm_rows_kernel, (int)smem_max);  // covers every order
   const ll grid = (rows + TR_R - 1) / TR_R;
   if (grid > 2147483647LL) throw std::invalid_argument("trsm_rows: too many rows");
-  trsm_rows_kernel<<<(unsigned)grid, TR_THREADS, smem, s>>>(Z, rows, k, nb, LX, ldx, Y, status);
+  trsm_rows_kernel<<<(unsigned)grid, TR_THREADS, smem, s>>>(Z, rows, k, nb, LX, ldx, Y, status, dscale);
   DMRG2_CHECK_LAUNCH();
 }
 

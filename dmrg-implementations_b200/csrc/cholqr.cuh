@@ -23,17 +23,18 @@ inline int chol_padded(int k) { return (k + CHOL_NB - 1) / CHOL_NB * CHOL_NB; }
 // then not numerically positive definite at that tolerance and LX is not valid. One
 // cluster of 8 (np <= 256) or 16 CTAs; LX may be the buffer G is in (each CTA writes
 // only the block row it read). Enqueued on s.
+// dscale (k doubles, optional): the factor is that of D G D with D = diag(G)^{-1/2}, whose diagonal
+// goes there; a zero or non-finite diagonal entry sets *status. That is the Gram matrix of unit
+// columns without a pass that scales them: trsm_rows scales as it reads.
 void chol_tiles(const double* G, int k, ll ldg, double* LX, ll ldx, int* status, double rel_tol, double shift_rel,
-                cudaStream_t s);
+                cudaStream_t s, double* dscale = nullptr);
 
 // Y = Z L^{-T} for the rows x k row-major Z (ld k) and the factor chol_tiles left in LX:
 // the orthonormal factor of CholeskyQR when L L^T = Z^T Z. Y (ld k) must not overlap Z.
 // Does nothing while *status is set.
+// dscale (optional, from chol_tiles): Z's columns are scaled by it.
 void trsm_rows(const double* Z, ll rows, int k, const double* LX, ll ldx, double* Y, const int* status,
-               cudaStream_t s);
-
-// *status = 1 unless out->ns_done (a Newton-Schulz run that did not converge)
-void mark_unconverged(const SvdOut* out, int* status, cudaStream_t s);
+               cudaStream_t s, const double* dscale = nullptr);
 
 // every column of the rows x k row-major Y scaled to unit norm (*status = 1 on a zero
 // or non-finite column); part holds COLNORM_MAX_CHUNKS x k doubles of partial sums

@@ -1320,7 +1320,10 @@ __global__ void ns_check_kernel(const double* __restrict__ S, int K, SvdOut* out
     __threadfence();
     double t = 0.0;
     for (int b = 0; b < (int)gridDim.x; ++b) t = fmax(t, part[b]);
-    if (!out->ns_done && t < tol) out->ns_done = 1;
+    if (!out->ns_done) {
+      if (t < tol) out->ns_done = 1;
+      out->ns_near = t * t < tol ? 1 : 0;
+    }
     *counter = 0u;
   }
 }

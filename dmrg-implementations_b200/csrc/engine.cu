@@ -914,7 +914,7 @@ class Engine final : public EngineBase {
     return prev_sweep_chi_ == chi && k <= chi && k <= kmax && std::min(m, nc) > k;
   }
   // |theta|^2 of the last warm split
-  double warm_fro2() const { return ST<T>::cplx ? ln().wstc.h_buf[1] : ln().wst.h_buf[1]; }
+  double warm_fro2() const { return ST<T>::cplx ? ln().wstc.h_rep->theta2 : ln().wst.h_rep->theta2; }
 
   // A bond below the cap keeps its dimension only while the weight the warm split
   // discards could all lie below the exact split's threshold (cutoff^2, or the density

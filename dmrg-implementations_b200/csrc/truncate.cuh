@@ -43,32 +43,31 @@ struct EigWork {
   size_t bytes = 0;
   std::vector<void*> owned;
 
-  void* alloc(size_t b) {
-    void* p = nullptr;
-    p = dev_alloc(std::max<size_t>(b, 16));
-    owned.push_back(p);
-    bytes += b;
-    return p;
-  }
   void init(int nmax_, int Kmax_) {
     nmax = std::max(nmax_, 1);
     Kmax = std::max(std::min(Kmax_, nmax), 1);
     const size_t nn = (size_t)nmax, kk = (size_t)Kmax;
-    G = (T*)alloc(sizeof(T) * nn * nn);
-    d = (double*)alloc(sizeof(double) * nn);
-    e = (double*)alloc(sizeof(double) * nn);
-    tau = (T*)alloc(sizeof(T) * nn);
-    lam = (double*)alloc(sizeof(double) * kk);
-    Z = (double*)alloc(sizeof(double) * nn * kk);
-    Z2 = (double*)alloc(sizeof(double) * nn * kk);
-    S = (double*)alloc(sizeof(double) * kk * kk);
-    scr = (double*)alloc(sizeof(double) * 5 * nn * kk);
-    Zg = (T*)alloc(sizeof(T) * nn * kk);
-    Tb = (T*)alloc(sizeof(T) * 256 * (nn + 1));
-    part = (double*)alloc(sizeof(double) * 64);
-    counter = (unsigned*)alloc(sizeof(unsigned) * 4);
+    DevSlab slab;
+    auto want = [&](auto*& p, size_t b) {
+      slab.add(p, b);
+      bytes += b;
+    };
+    want(G, sizeof(T) * nn * nn);
+    want(d, sizeof(double) * nn);
+    want(e, sizeof(double) * nn);
+    want(tau, sizeof(T) * nn);
+    want(lam, sizeof(double) * kk);
+    want(Z, sizeof(double) * nn * kk);
+    want(Z2, sizeof(double) * nn * kk);
+    want(S, sizeof(double) * kk * kk);
+    want(scr, sizeof(double) * 5 * nn * kk);
+    want(Zg, sizeof(T) * nn * kk);
+    want(Tb, sizeof(T) * 256 * (nn + 1));
+    want(part, sizeof(double) * 64);
+    want(counter, sizeof(unsigned) * 4);
+    want(out, sizeof(SvdOut));
+    owned.push_back(slab.commit());
     DMRG2_CUDA(cudaMemset(counter, 0, sizeof(unsigned) * 4));
-    out = (SvdOut*)alloc(sizeof(SvdOut));
     h_out = (SvdOut*)host_pinned(sizeof(SvdOut));
     DMRG2_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
     DMRG2_CUDA(cudaEventCreateWithFlags(&ev_refl, cudaEventDisableTiming));
@@ -142,13 +141,13 @@ SvdOut eig_split(EigWork<T>& W, const T* theta, int m, int nt, char dir, int chi
     g1.skip = &W.out->ns_done;
     launch_gemm(g1, s);
     ns_check(W.S, K, W.out, 4e-16 * (double)n, W.part, W.counter, s);
-    DMRG2_CUDA(cudaMemcpyAsync(W.Z2, W.Z, sizeof(double) * (size_t)n * K, cudaMemcpyDeviceToDevice, s));
     Gemm<double> g2;
     g2.M = n; g2.N = K; g2.K = K;
     g2.A = W.Z; g2.lda = K;
     g2.B = W.S; g2.ldb = K;
     g2.C = W.Z2; g2.ldc = K;
     g2.alpha = -0.5; g2.beta = 1.5;
+    g2.Cin = W.Z;  // copied to Z2 once the vectors are orthonormal
     g2.skip = &W.out->ns_done;
     launch_gemm(g2, s);
     std::swap(W.Z, W.Z2);
@@ -233,8 +232,9 @@ SvdOut eig_split(EigWork<T>& W, const T* theta, int m, int nt, char dir, int chi
 //        left = U, right = U^T theta
 //   'L': V1 = tri(theta^T A), U1 = tri(theta V1), V = tri(theta^T U1),
 //        right = V^T, left = theta V
-// tri = unit columns, then one CholeskyQR pass (Gram matrix, its tiled Cholesky factor
-// in one cluster kernel, then the row solve Z L^{-T} on the tensor cores). Why that is
+// tri = one CholeskyQR pass on unit columns (Gram matrix, its tiled Cholesky factor
+// in one cluster kernel, which scales it to unit diagonal, then the row solve Z D L^{-T}
+// on the tensor cores). Why that is
 // enough: the basis a step starts from is orthonormal, ordered by decreasing
 // singular value and close to the Schmidt basis of the bond (the exact split
 // returns Schmidt vectors, and each later warm split keeps that), so each product
@@ -255,10 +255,8 @@ SvdOut eig_split(EigWork<T>& W, const T* theta, int m, int nt, char dir, int chi
 struct WstWork {
   double* Ya = nullptr;  // qmax x kmax
   double* Yb = nullptr;
-  double* Yc = nullptr;  // qmax x kmax, the other half of each Newton-Schulz step
   double* S = nullptr;   // Gram matrix, then its tiled Cholesky factor (np x np, np = chol_padded(kmax))
-  double* cpart = nullptr;  // column sums of squares per row chunk
-  double* nrm = nullptr; // |theta|^2, |kept factor|^2
+  double* dscale = nullptr;  // 1 / norm of each column being orthonormalised
   double* part = nullptr;
   unsigned* counter = nullptr;
   int* status = nullptr;
@@ -266,44 +264,41 @@ struct WstWork {
   // with graphs: the warm factor in, and both factors out, pass through these fixed slots
   // (qmax x kmax each), so one graph serves every bond of a shape
   double *Win = nullptr, *Lout = nullptr, *Rout = nullptr;
-  double* h_buf = nullptr;  // pinned: |theta|^2, |kept|^2
-  SvdOut* h_out = nullptr;  // pinned
-  int* h_status = nullptr;  // pinned
+  SplitHost* h_rep = nullptr;  // pinned: the split's report
+  SvdOut* h_out = nullptr;  // pinned (diagnostics)
+  int* h_status = nullptr;
   int qmax = 0, kmax = 0;
   size_t bytes = 0;
   std::vector<void*> owned;
   // the launch sequence of a split, by direction, mode and shapes
   GraphCache graphs;
 
-  void* alloc(size_t b) {
-    void* p = nullptr;
-    p = dev_alloc(std::max<size_t>(b, 16));
-    owned.push_back(p);
-    bytes += b;
-    return p;
-  }
   void init(int qmax_, int kmax_) {
     graphs.cap = 2048;  // ~100 bond shapes x 2 directions x 3 modes in a chi=256 sweep of 100 sites
     graphs.name = "warm split";
     qmax = std::max(qmax_, 1);
     kmax = std::max(std::min(kmax_, CHOL_MAX), 1);
     const size_t qk = (size_t)qmax * kmax;
-    Ya = (double*)alloc(sizeof(double) * qk);
-    Yb = (double*)alloc(sizeof(double) * qk);
-    Yc = (double*)alloc(sizeof(double) * qk);
-    Win = (double*)alloc(sizeof(double) * qk);
-    Lout = (double*)alloc(sizeof(double) * qk);
-    Rout = (double*)alloc(sizeof(double) * qk);
+    DevSlab slab;
+    auto want = [&](auto*& p, size_t b) {
+      slab.add(p, b);
+      bytes += b;
+    };
+    want(Ya, sizeof(double) * qk);
+    want(Yb, sizeof(double) * qk);
+    want(Win, sizeof(double) * qk);
+    want(Lout, sizeof(double) * qk);
+    want(Rout, sizeof(double) * qk);
     const size_t np = (size_t)chol_padded(kmax);
-    S = (double*)alloc(sizeof(double) * np * np);
-    cpart = (double*)alloc(sizeof(double) * (size_t)COLNORM_MAX_CHUNKS * kmax);
-    nrm = (double*)alloc(sizeof(double) * 4);
-    part = (double*)alloc(sizeof(double) * 64);
-    counter = (unsigned*)alloc(sizeof(unsigned) * 4);
-    status = (int*)alloc(sizeof(int) * 4);
-    out = (SvdOut*)alloc(sizeof(SvdOut));
+    want(S, sizeof(double) * np * np);
+    want(dscale, sizeof(double) * (size_t)kmax);
+    want(part, sizeof(double) * 64);
+    want(counter, sizeof(unsigned) * 4);
+    want(status, sizeof(int) * 4);
+    want(out, sizeof(SvdOut));
+    owned.push_back(slab.commit());
     DMRG2_CUDA(cudaMemset(counter, 0, sizeof(unsigned) * 4));
-    h_buf = (double*)host_pinned(sizeof(double) * 4);
+    h_rep = (SplitHost*)host_pinned(sizeof(SplitHost));
     h_out = (SvdOut*)host_pinned(sizeof(SvdOut));
     h_status = (int*)host_pinned(sizeof(int));
   }
@@ -311,10 +306,10 @@ struct WstWork {
     graphs.clear();
     for (void* p : owned) dev_free(p);
     owned.clear();
-    if (h_buf) host_unpin(h_buf);
+    if (h_rep) host_unpin(h_rep);
     if (h_out) host_unpin(h_out);
     if (h_status) host_unpin(h_status);
-    h_buf = nullptr;
+    h_rep = nullptr;
     h_out = nullptr;
     h_status = nullptr;
   }
@@ -325,7 +320,7 @@ inline size_t wst_bytes(ll qmax, ll kmax) {
   qmax = std::max<ll>(qmax, 1);
   kmax = std::max<ll>(std::min<ll>(kmax, CHOL_MAX), 1);
   const ll np = chol_padded((int)kmax);
-  return sizeof(double) * (size_t)(6 * qmax * kmax + np * np + COLNORM_MAX_CHUNKS * kmax + 4 + 64) +
+  return sizeof(double) * (size_t)(5 * qmax * kmax + np * np + kmax + 64) +
          sizeof(unsigned) * 4 + sizeof(int) * 4 + sizeof(SvdOut);
 }
 
@@ -359,17 +354,11 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
                       const double* warm, double* left, double* right, double& trunc_err, cudaStream_t s,
                       WstMode mode = WST_FULL, bool allow_graph = true, cudaEvent_t ev_end = nullptr) {
   if (k > W.kmax || m > W.qmax || nt > W.qmax) throw std::runtime_error("wst_split: workspace too small");
-  if (std::max(m, nt) > 32 * COLNORM_MAX_CHUNKS) return false;  // beyond the column-scaling kernel
-  DMRG2_CUDA(cudaMemsetAsync(W.status, 0, sizeof(int), s));
-  {
-    SvdOut o0{};
-    o0.k = k;
-    *W.h_out = o0;
-    DMRG2_CUDA(cudaMemcpyAsync(W.out, W.h_out, sizeof(SvdOut), cudaMemcpyHostToDevice, s));
-  }
+  if (std::max(m, nt) > 32 * COLNORM_MAX_CHUNKS) return false;  // longer columns take the exact split
+  split_begin(W.status, W.out, k, s);
   // C (M x N) = alpha op(A) op(B) + beta C
   auto mul = [&](bool ta, const double* A, ll lda, int M, int N, int Kd, const double* B, ll ldb, bool tb,
-                 double* C, ll ldc, double alpha, double beta, const int* skip) {
+                 double* C, ll ldc, double alpha, double beta, const int* skip, const double* Cin = nullptr) {
     Gemm<double> g;
     g.ta = ta; g.tb = tb;
     g.M = M; g.N = N; g.K = Kd;
@@ -378,26 +367,17 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
     g.C = C; g.ldc = ldc;
     g.alpha = alpha; g.beta = beta;
     g.skip = skip;
+    g.Cin = Cin;
     launch_gemm(g, s);
   };
   const int* done = &W.out->ns_done;
-  // Newton-Schulz polish of the nearly orthonormal Z (rows x k): S = Z^T Z, stop once
-  // |S - 1| < tol, Z <- 1.5 Z - 0.5 Z S (iterations after convergence only launch
-  // kernels that return); a run that ends unconverged marks the split as failed. The
-  // result is left in dst.
-  auto orth = [&](double* Z, ll rows, double tol, int iters, double* dst) {
-    DMRG2_CUDA(cudaMemsetAsync(&W.out->ns_done, 0, sizeof(int), s));
-    double* a = Z;
-    double* b = (Z == W.Yc) ? dst : W.Yc;
-    for (int it = 0; it < iters; ++it) {
-      mul(true, a, k, k, k, (int)rows, a, k, false, W.S, k, 1.0, 0.0, done);
-      ns_check(W.S, k, W.out, tol, W.part, W.counter, s);
-      DMRG2_CUDA(cudaMemcpyAsync(b, a, sizeof(double) * (size_t)rows * k, cudaMemcpyDeviceToDevice, s));
-      mul(false, a, k, (int)rows, k, k, W.S, k, false, b, k, -0.5, 1.5, done);
-      std::swap(a, b);
-    }
-    mark_unconverged(W.out, W.status, s);
-    if (a != dst) DMRG2_CUDA(cudaMemcpyAsync(dst, a, sizeof(double) * (size_t)rows * k, cudaMemcpyDeviceToDevice, s));
+  // Newton-Schulz polish of the nearly orthonormal Z (rows x k) into dst: S = Z^T Z; within tol of
+  // the identity Z is copied, else dst = 1.5 Z - 0.5 Z S, whose deviation is the square of Z's
+  // (a deviation too large for one step makes the split report a failure)
+  auto orth = [&](double* Z, ll rows, double tol, double* dst) {
+    mul(true, Z, k, k, k, (int)rows, Z, k, false, W.S, k, 1.0, 0.0, nullptr);
+    ns_check(W.S, k, W.out, tol, W.part, W.counter, s);
+    mul(false, Z, k, (int)rows, k, k, W.S, k, false, dst, k, -0.5, 1.5, done, Z);
     if (wst_debug()) {
       DMRG2_CUDA(cudaMemcpyAsync(W.h_out, W.out, sizeof(SvdOut), cudaMemcpyDeviceToHost, s));
       DMRG2_CUDA(cudaMemcpyAsync(W.h_status, W.status, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -411,13 +391,12 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
                    (long long)rows, k, tol, W.h_out->ns_done, *W.h_status, e);
     }
   };
-  // Z (rows x k) <- tri(Z) into dst (dst != Z): unit columns, Gram matrix, its Cholesky factor, Z L^{-T}
+  // Z (rows x k) <- tri(Z) into dst (dst != Z): Gram matrix, Cholesky factor of its unit-diagonal form, Z D L^{-T}
   const int ldS = chol_padded(k);
   auto tri = [&](double* Z, ll rows, double* dst) {
-    col_normalize(Z, rows, k, W.cpart, W.status, s);
     mul(true, Z, k, k, k, (int)rows, Z, k, false, W.S, ldS, 1.0, 0.0, nullptr);
-    chol_tiles(W.S, k, ldS, W.S, ldS, W.status, 1e-10, 0.0, s);  // factor in place of the Gram matrix
-    trsm_rows(Z, rows, k, W.S, ldS, dst, W.status, s);
+    chol_tiles(W.S, k, ldS, W.S, ldS, W.status, 1e-10, 0.0, s, W.dscale);  // factor in place of the Gram matrix
+    trsm_rows(Z, rows, k, W.S, ldS, dst, W.status, s, W.dscale);
   };
   const bool graph = allow_graph && graphs_enabled() && !wst_debug() && s != nullptr;
   double* const left_out = left;
@@ -432,6 +411,8 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
     right = W.Rout;
   }
   auto body = [&]() {
+  const double* kept = nullptr;
+  ll nkept = 0;
   if (dir == 'R') {
     if (mode != WST_RESUME) {
       mul(false, theta, nt, m, k, nt, warm, nt, true, W.Ya, k, 1.0, 0.0, nullptr);  // theta B^T
@@ -445,9 +426,10 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
       mul(false, theta, nt, m, k, nt, W.Yb, k, false, W.Ya, k, 1.0, 0.0, nullptr); // theta V1
       tri(W.Ya, m, W.Yb);
     }
-    orth(W.Yb, m, 4e-16 * (double)m, 2, left);                                     // polish
+    orth(W.Yb, m, 4e-16 * (double)m, left);                                     // polish
     mul(true, left, k, k, nt, m, theta, nt, false, right, nt, 1.0, 0.0, nullptr);  // right = U^T theta
-    norm2(right, (ll)k * nt, W.nrm + 1, red, s);
+    kept = right;
+    nkept = (ll)k * nt;
   } else {
     if (mode != WST_RESUME) {
       mul(true, theta, nt, nt, k, m, warm, k, false, W.Ya, k, 1.0, 0.0, nullptr);  // theta^T A
@@ -461,12 +443,13 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
       mul(true, theta, nt, nt, k, m, W.Yb, k, false, W.Ya, k, 1.0, 0.0, nullptr);  // theta^T U1
       tri(W.Ya, nt, W.Yb);
     }
-    orth(W.Yb, nt, 4e-16 * (double)nt, 2, W.Ya);                                   // polish; V in Ya
+    orth(W.Yb, nt, 4e-16 * (double)nt, W.Ya);                                   // polish; V in Ya
     transpose(W.Ya, right, (ll)nt, (ll)k, s);                                      // right = V^T
     mul(false, theta, nt, m, k, nt, W.Ya, k, false, left, k, 1.0, 0.0, nullptr);   // left = theta V
-    norm2(left, (ll)m * k, W.nrm + 1, red, s);
+    kept = left;
+    nkept = (ll)m * k;
   }
-  norm2(theta, (ll)m * nt, W.nrm, red, s);
+  split_finish(theta, (ll)m * nt, kept, nkept, W.status, W.out, W.h_rep, red, s);
   };
   if (graph) {
     const GraphKey key{dir, mode, m, nt, k, (ll)theta, (ll)&W, (ll)red.part, (ll)red.counter, 0, 0, 0, 0, 0, 0, 0};
@@ -496,13 +479,10 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
     body();
   }
   if (ev_end) DMRG2_CUDA(cudaEventRecord(ev_end, s));  // the split's device work ends here
-  DMRG2_CUDA(cudaMemcpyAsync(W.h_buf + 1, W.nrm, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
-  DMRG2_CUDA(cudaMemcpyAsync(W.h_out, W.out, sizeof(SvdOut), cudaMemcpyDeviceToHost, s));
-  DMRG2_CUDA(cudaMemcpyAsync(W.h_status, W.status, sizeof(int), cudaMemcpyDeviceToHost, s));
   DMRG2_CUDA(cudaStreamSynchronize(s));
-  if (*W.h_status) return false;
-  if (!std::isfinite(W.h_buf[1]) || !std::isfinite(W.h_buf[2])) return false;
-  trunc_err = std::max(W.h_buf[1] - W.h_buf[2], 0.0);
+  const SplitHost& rep = *W.h_rep;
+  if (rep.failed || !std::isfinite(rep.theta2) || !std::isfinite(rep.kept2)) return false;
+  trunc_err = std::max(rep.theta2 - rep.kept2, 0.0);
   return true;
 }
 

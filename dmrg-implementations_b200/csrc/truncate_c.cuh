@@ -29,17 +29,13 @@ struct WstWorkC {
   zc* Yb = nullptr;
   double* Z1 = nullptr;  // real embeddings: (2 qmax) x (2 kmax) each
   double* Z2 = nullptr;
-  double* Z3 = nullptr;
   double* S = nullptr;   // Gram matrix, then its tiled factor (np x np, np = chol_padded(2 kmax))
-  double* cpart = nullptr;
-  double* nrm = nullptr;
+  double* dscale = nullptr;  // 1 / norm of each embedded column
   double* part = nullptr;
   unsigned* counter = nullptr;
   int* status = nullptr;
   SvdOut* out = nullptr;
-  double* h_buf = nullptr;  // pinned: |theta|^2, |kept|^2
-  SvdOut* h_out = nullptr;  // pinned
-  int* h_status = nullptr;  // pinned
+  SplitHost* h_rep = nullptr;  // pinned: the split's report
   int qmax = 0, kmax = 0;
   size_t bytes = 0;
   std::vector<void*> owned;
@@ -58,29 +54,21 @@ struct WstWorkC {
     Yb = (zc*)alloc(sizeof(zc) * qk);
     Z1 = (double*)alloc(sizeof(double) * 4 * qk);
     Z2 = (double*)alloc(sizeof(double) * 4 * qk);
-    Z3 = (double*)alloc(sizeof(double) * 4 * qk);
     const size_t np = (size_t)chol_padded(2 * kmax);
     S = (double*)alloc(sizeof(double) * np * np);
-    cpart = (double*)alloc(sizeof(double) * (size_t)COLNORM_MAX_CHUNKS * 2 * kmax);
-    nrm = (double*)alloc(sizeof(double) * 4);
+    dscale = (double*)alloc(sizeof(double) * 2 * (size_t)kmax);
     part = (double*)alloc(sizeof(double) * 64);
     counter = (unsigned*)alloc(sizeof(unsigned) * 4);
     status = (int*)alloc(sizeof(int) * 4);
     out = (SvdOut*)alloc(sizeof(SvdOut));
     DMRG2_CUDA(cudaMemset(counter, 0, sizeof(unsigned) * 4));
-    h_buf = (double*)host_pinned(sizeof(double) * 4);
-    h_out = (SvdOut*)host_pinned(sizeof(SvdOut));
-    h_status = (int*)host_pinned(sizeof(int));
+    h_rep = (SplitHost*)host_pinned(sizeof(SplitHost));
   }
   void release() {
     for (void* p : owned) dev_free(p);
     owned.clear();
-    if (h_buf) host_unpin(h_buf);
-    if (h_out) host_unpin(h_out);
-    if (h_status) host_unpin(h_status);
-    h_buf = nullptr;
-    h_out = nullptr;
-    h_status = nullptr;
+    if (h_rep) host_unpin(h_rep);
+    h_rep = nullptr;
   }
 };
 
@@ -91,7 +79,7 @@ inline size_t wstc_bytes(ll qmax, ll kmax) {
   const ll qk = qmax * kmax;
   const ll np = chol_padded((int)(2 * kmax));
   return sizeof(zc) * (size_t)(2 * qk) +
-         sizeof(double) * (size_t)(12 * qk + np * np + COLNORM_MAX_CHUNKS * 2 * kmax + 4 + 64) +
+         sizeof(double) * (size_t)(8 * qk + np * np + 2 * kmax + 64) +
          sizeof(unsigned) * 4 + sizeof(int) * 4 + sizeof(SvdOut);
 }
 
@@ -103,14 +91,8 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
                         const zc* warm, zc* left, zc* right, double& trunc_err, cudaStream_t s,
                         WstMode mode = WST_FULL, cudaEvent_t ev_end = nullptr) {
   if (k > W.kmax || m > W.qmax || nt > W.qmax) throw std::runtime_error("wst_split_c: workspace too small");
-  if (2 * std::max(m, nt) > 32 * COLNORM_MAX_CHUNKS) return false;  // beyond the column-scaling kernel
-  DMRG2_CUDA(cudaMemsetAsync(W.status, 0, sizeof(int), s));
-  {
-    SvdOut o0{};
-    o0.k = k;
-    *W.h_out = o0;
-    DMRG2_CUDA(cudaMemcpyAsync(W.out, W.h_out, sizeof(SvdOut), cudaMemcpyHostToDevice, s));
-  }
+  if (2 * std::max(m, nt) > 32 * COLNORM_MAX_CHUNKS) return false;  // longer columns take the exact split
+  split_begin(W.status, W.out, k, s);
   // complex C (M x N) = op(A) op(B): ta / ca transpose / conjugate A, tb transposes B
   auto mulz = [&](bool ta, bool ca, const zc* A, ll lda, int M, int N, int Kd, const zc* B, ll ldb, bool tb,
                   zc* C, ll ldc) {
@@ -124,7 +106,7 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
   };
   // real C = alpha op(A) op(B) + beta C on the embeddings
   auto mulr = [&](bool ta, const double* A, ll lda, int M, int N, int Kd, const double* B, ll ldb, double* C,
-                  ll ldc, double alpha, double beta, const int* skip) {
+                  ll ldc, double alpha, double beta, const int* skip, const double* Cin = nullptr) {
     Gemm<double> g;
     g.ta = ta;
     g.M = M; g.N = N; g.K = Kd;
@@ -133,6 +115,7 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
     g.C = C; g.ldc = ldc;
     g.alpha = alpha; g.beta = beta;
     g.skip = skip;
+    g.Cin = Cin;
     launch_gemm(g, s);
   };
   const int k2 = 2 * k;
@@ -141,31 +124,23 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
   // tiled Cholesky factor, row solve), then the even columns
   auto tri = [&](const zc* Z, ll rows, zc* dst) {
     embed_pairs(Z, rows, k, W.Z1, s);
-    col_normalize(W.Z1, 2 * rows, k2, W.cpart, W.status, s);
     mulr(true, W.Z1, k2, k2, k2, (int)(2 * rows), W.Z1, k2, W.S, ldS, 1.0, 0.0, nullptr);
-    chol_tiles(W.S, k2, ldS, W.S, ldS, W.status, 1e-10, 0.0, s);
-    trsm_rows(W.Z1, 2 * rows, k2, W.S, ldS, W.Z2, W.status, s);
+    chol_tiles(W.S, k2, ldS, W.S, ldS, W.status, 1e-10, 0.0, s, W.dscale);
+    trsm_rows(W.Z1, 2 * rows, k2, W.S, ldS, W.Z2, W.status, s, W.dscale);
     extract_pairs(W.Z2, rows, k, dst, s);
   };
-  // two Newton-Schulz steps on the embedding of Z (rows x k), result into dst; a run that
-  // ends unconverged marks the split as failed
-  const int* done = &W.out->ns_done;
+  // one Newton-Schulz step on the embedding of Z (rows x k) unless it is orthonormal already, result
+  // into dst; a deviation too large for one step makes the split report a failure
   auto polish = [&](const zc* Z, ll rows, zc* dst) {
     const ll r2 = 2 * rows;
     embed_pairs(Z, rows, k, W.Z1, s);
-    DMRG2_CUDA(cudaMemsetAsync(&W.out->ns_done, 0, sizeof(int), s));
-    double* a = W.Z1;
-    double* b = W.Z3;
-    for (int it = 0; it < 2; ++it) {
-      mulr(true, a, k2, k2, k2, (int)r2, a, k2, W.S, k2, 1.0, 0.0, done);
-      ns_check(W.S, k2, W.out, 4e-16 * (double)r2, W.part, W.counter, s);
-      DMRG2_CUDA(cudaMemcpyAsync(b, a, sizeof(double) * (size_t)r2 * k2, cudaMemcpyDeviceToDevice, s));
-      mulr(false, a, k2, (int)r2, k2, k2, W.S, k2, b, k2, -0.5, 1.5, done);
-      std::swap(a, b);
-    }
-    mark_unconverged(W.out, W.status, s);
-    extract_pairs(a, rows, k, dst, s);
+    mulr(true, W.Z1, k2, k2, k2, (int)r2, W.Z1, k2, W.S, k2, 1.0, 0.0, nullptr);
+    ns_check(W.S, k2, W.out, 4e-16 * (double)r2, W.part, W.counter, s);
+    mulr(false, W.Z1, k2, (int)r2, k2, k2, W.S, k2, W.Z2, k2, -0.5, 1.5, &W.out->ns_done, W.Z1);
+    extract_pairs(W.Z2, rows, k, dst, s);
   };
+  const zc* kept = nullptr;
+  ll nkept = 0;
   if (dir == 'R') {
     if (mode != WST_RESUME) {
       mulz(false, true, warm, nt, k, m, nt, theta, nt, true, W.Yb, m);  // conj(B) theta^T (k x m)
@@ -182,7 +157,8 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
     }
     polish(W.Yb, m, left);
     mulz(true, true, left, k, k, nt, m, theta, nt, false, right, nt);  // right = U^H theta
-    norm2(right, (ll)k * nt, W.nrm + 1, red, s);
+    kept = right;
+    nkept = (ll)k * nt;
   } else {
     if (mode != WST_RESUME) {
       mulz(true, true, theta, nt, nt, k, m, warm, k, false, W.Ya, k);  // theta^H A
@@ -199,17 +175,15 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
     polish(W.Yb, nt, W.Ya);                                              // V in Ya
     transpose_conj<zc>(W.Ya, k, nt, k, right, s);                        // right = V^H
     mulz(false, false, theta, nt, m, k, nt, W.Ya, k, false, left, k);    // left = theta V
-    norm2(left, (ll)m * k, W.nrm + 1, red, s);
+    kept = left;
+    nkept = (ll)m * k;
   }
-  norm2(theta, (ll)m * nt, W.nrm, red, s);
+  split_finish(theta, (ll)m * nt, kept, nkept, W.status, W.out, W.h_rep, red, s);
   if (ev_end) DMRG2_CUDA(cudaEventRecord(ev_end, s));
-  DMRG2_CUDA(cudaMemcpyAsync(W.h_buf + 1, W.nrm, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
-  DMRG2_CUDA(cudaMemcpyAsync(W.h_out, W.out, sizeof(SvdOut), cudaMemcpyDeviceToHost, s));
-  DMRG2_CUDA(cudaMemcpyAsync(W.h_status, W.status, sizeof(int), cudaMemcpyDeviceToHost, s));
   DMRG2_CUDA(cudaStreamSynchronize(s));
-  if (*W.h_status) return false;
-  if (!std::isfinite(W.h_buf[1]) || !std::isfinite(W.h_buf[2])) return false;
-  trunc_err = std::max(W.h_buf[1] - W.h_buf[2], 0.0);
+  const SplitHost& rep = *W.h_rep;
+  if (rep.failed || !std::isfinite(rep.theta2) || !std::isfinite(rep.kept2)) return false;
+  trunc_err = std::max(rep.theta2 - rep.kept2, 0.0);
   return true;
 }
 
