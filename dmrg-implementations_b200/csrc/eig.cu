@@ -1328,6 +1328,72 @@ __global__ void ns_check_kernel(const double* __restrict__ S, int K, SvdOut* out
   }
 }
 
+// The Newton-Schulz steps of a small block (n <= NSS_N, K <= NSS_K) in one CTA: Z in shared
+// memory, S = Z^T Z and 1.5 Z - 0.5 Z S on the FP64 tensor cores, until S deviates from 1 by
+// less than tol (over the first out->k vectors) or `iters` steps are made. One launch of 4 us per
+// product of 128 x 64 instead of three (GEMM, check, GEMM) per step, of 2 to 4 us each, which
+// at this size is all latency: three steps took 25 us of a split at n = 128, K = 64.
+constexpr int NSS_N = 128, NSS_K = 64, NSS_P = NSS_K + 4, NSS_THREADS = 256;
+__global__ void __launch_bounds__(NSS_THREADS) ns_small_kernel(double* __restrict__ Z, int n, int K, SvdOut* out,
+                                                               double tol, int iters) {
+  extern __shared__ __align__(16) double nss[];
+  double* A = nss;                  // [NSS_N][NSS_P], zeros beyond n x K
+  double* B = A + NSS_N * NSS_P;    // the next Z
+  double* S = B + NSS_N * NSS_P;    // [NSS_K][NSS_P]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
+  const int np = (n + 15) & ~15, Kp = (K + 15) & ~15, k = min(out->k, K);
+  for (int e = tid; e < np * Kp; e += NSS_THREADS) {
+    const int r = e / Kp, c = e % Kp;
+    A[r * NSS_P + c] = (r < n && c < K) ? Z[(ll)r * K + c] : 0.0;
+  }
+  __syncthreads();
+  bool done = false, moved = false;
+  for (int it = 0; it <= iters; ++it) {
+    double m = 0.0;
+    const int mt = Kp / 16, nt = Kp / 8;
+    for (int u = warp; u < mt * nt; u += NSS_THREADS / 32) {
+      const int r0 = (u / nt) * 16, c0 = (u % nt) * 8;
+      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int q = 0; q < np; q += 8) {
+        const double* p = A + (q + tq) * NSS_P;
+        dmma16x8x8(acc, p[r0 + gq], p[r0 + gq + 8], p[4 * NSS_P + r0 + gq], p[4 * NSS_P + r0 + gq + 8], p[c0 + gq],
+                   p[4 * NSS_P + c0 + gq]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = r0 + gq + ((e & 2) ? 8 : 0), c = c0 + 2 * tq + (e & 1);
+        S[r * NSS_P + c] = acc[e];
+        if (r < k && c < k) m = fmax(m, fabs(acc[e] - (r == c ? 1.0 : 0.0)));
+      }
+    }
+    done = __syncthreads_and(m < tol ? 1 : 0) != 0;
+    if (done || it == iters) break;
+    const int zt = np / 16;
+    for (int u = warp; u < zt * nt; u += NSS_THREADS / 32) {
+      const int r0 = (u / nt) * 16, c0 = (u % nt) * 8;
+      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int q = 0; q < Kp; q += 8) {
+        const double* pa = A + (r0 + gq) * NSS_P + q + tq;
+        const double* pb = S + (q + tq) * NSS_P + c0 + gq;
+        dmma16x8x8(acc, pa[0], pa[8 * NSS_P], pa[4], pa[8 * NSS_P + 4], pb[0], pb[4 * NSS_P]);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int at = (r0 + gq + ((e & 2) ? 8 : 0)) * NSS_P + c0 + 2 * tq + (e & 1);
+        B[at] = 1.5 * A[at] - 0.5 * acc[e];
+      }
+    }
+    __syncthreads();
+    double* t = A;
+    A = B;
+    B = t;
+    moved = true;
+  }
+  if (moved)
+    for (int e = tid; e < n * K; e += NSS_THREADS) Z[e] = A[(e / K) * NSS_P + e % K];
+  if (tid == 0 && done) out->ns_done = 1;
+}
+
 // ----------------------------------------------------------------------------
 // truncation decision from the eigenvalues (one CTA)
 // ----------------------------------------------------------------------------
@@ -1519,6 +1585,16 @@ void ns_check(const double* S, int K, SvdOut* out, double tol, double* part, uns
               cudaStream_t s) {
   ns_check_kernel<<<32, 256, 0, s>>>(S, K, out, tol, part, counter);
   DMRG2_CHECK_LAUNCH();
+}
+
+bool ns_small(double* Z, int n, int K, SvdOut* out, double tol, int iters, cudaStream_t s) {
+  if (n > NSS_N || K > NSS_K) return false;
+  constexpr size_t smem = sizeof(double) * (size_t)(2 * NSS_N + NSS_K) * NSS_P;
+  static std::atomic<unsigned long long> attr{0};
+  set_smem_attr_once(attr, (const void*)ns_small_kernel, (int)smem);
+  ns_small_kernel<<<1, NSS_THREADS, smem, s>>>(Z, n, K, out, tol, iters);
+  DMRG2_CHECK_LAUNCH();
+  return true;
 }
 
 void eig_truncate(const double* d, const double* lam, int n, int K, int chi_max, double cutoff,

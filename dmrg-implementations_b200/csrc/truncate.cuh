@@ -152,7 +152,9 @@ SvdOut eig_split(EigWork<T>& W, const T* theta, int m, int nt, char dir, int chi
     launch_gemm(g2, s);
     std::swap(W.Z, W.Z2);
   };
-  for (int it = 0; it < 3; ++it) ns_iteration();
+  const double ns_tol = 4e-16 * (double)n;
+  if (!ns_small(W.Z, n, K, W.out, ns_tol, 3, s))
+    for (int it = 0; it < 3; ++it) ns_iteration();
   DMRG2_CUDA(cudaStreamWaitEvent(s, W.ev_wy, 0));
   apply_q<T>(W.G, n, W.tau, n, W.Z, K, W.out, W.Zg, W.Tb, s, true);
   DMRG2_CUDA(cudaMemcpyAsync(W.h_out, W.out, sizeof(SvdOut), cudaMemcpyDeviceToHost, s));
