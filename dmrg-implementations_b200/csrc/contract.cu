@@ -15,6 +15,7 @@ template <typename T, int KM>
 __global__ void __launch_bounds__(128)
     mpo_mix_kernel(const T* __restrict__ X, const T* __restrict__ W, T* __restrict__ Y, int Kin,
                    int Kout, int cR, ll sX, ll sY, const int* skip) {
+  pdl_wait();
   if (skip && *((volatile const int*)skip)) return;
   __shared__ T Ws[KM * KM];
   for (int i = threadIdx.x; i < KM * KM; i += blockDim.x) {
@@ -49,6 +50,7 @@ template <typename T>
 __global__ void __launch_bounds__(MIX_SPARSE_NT)
     mpo_mix_sparse_kernel(const T* __restrict__ X, const T* __restrict__ val, const int* __restrict__ rowp,
                           T* __restrict__ Y, int Kin, int Kout, int cR, ll sX, ll sY, const int* skip) {
+  pdl_wait();
   if (skip && *((volatile const int*)skip)) return;
   constexpr int KM = 32, NT = MIX_SPARSE_NT;
   __shared__ int rp[KM + 1];
@@ -92,6 +94,7 @@ template <typename T>
 __global__ void __launch_bounds__(MIX_WIDE_NT)
     mpo_mix_wide_kernel(const T* __restrict__ X, const T* __restrict__ val, const int* __restrict__ rowp,
                         T* __restrict__ Y, int Kin, int Kout, int cR, ll sX, ll sY, const int* skip) {
+  pdl_wait();
   if (skip && *((volatile const int*)skip)) return;
   extern __shared__ __align__(16) unsigned char mix_smem[];
   T* xs = reinterpret_cast<T*>(mix_smem);  // [Kin][32]
@@ -163,21 +166,18 @@ static void mix_rows(const T* X, const T* W, T* Y, int cL, int cR, int Kin, int 
     // (the engine uses the nonzero form only where nnz <= Kin Kout / 2 <= MIX_SPARSE_NNZ)
     const ll kk = (ll)Kin * Kout;
     dim3 grid(ceil_div(cR, MIX_SPARSE_NT), cL);
-    mpo_mix_sparse_kernel<T><<<grid, MIX_SPARSE_NT, 0, s>>>(X, wsp, (const int*)(wsp + kk), Y, Kin, Kout, cR,
-                                                            (ll)Kin * cR, (ll)Kout * cR, skip);
-    DMRG2_CHECK_LAUNCH();
+    launch_pdl(mpo_mix_sparse_kernel<T>, grid, MIX_SPARSE_NT, 0, s, X, wsp, (const int*)(wsp + kk), Y, Kin, Kout, cR,
+               (ll)Kin * cR, (ll)Kout * cR, skip);
   } else if (wsp && Kin <= MIX_WIDE_K && Kout <= MIX_WIDE_K && cL <= 65535) {
     const ll kk = (ll)Kin * Kout;
     static std::atomic<unsigned long long> attr{0};
     set_smem_attr_once(attr, (const void*)mpo_mix_wide_kernel<T>, (int)(sizeof(T) * MIX_WIDE_K * 32));
     dim3 grid(ceil_div(cR, 32), cL);
-    mpo_mix_wide_kernel<T><<<grid, MIX_WIDE_NT, sizeof(T) * (size_t)Kin * 32, s>>>(X, wsp, (const int*)(wsp + kk), Y, Kin, Kout,
-                                                                           cR, (ll)Kin * cR, (ll)Kout * cR, skip);
-    DMRG2_CHECK_LAUNCH();
+    launch_pdl(mpo_mix_wide_kernel<T>, grid, MIX_WIDE_NT, sizeof(T) * (size_t)Kin * 32, s, X, wsp,
+               (const int*)(wsp + kk), Y, Kin, Kout, cR, (ll)Kin * cR, (ll)Kout * cR, skip);
   } else if (Kin <= 32 && Kout <= 32 && cL <= 65535) {
     dim3 grid(ceil_div(cR, 128), cL);
-    mpo_mix_kernel<T, 32><<<grid, 128, 0, s>>>(X, W, Y, Kin, Kout, cR, (ll)Kin * cR, (ll)Kout * cR, skip);
-    DMRG2_CHECK_LAUNCH();
+    launch_pdl(mpo_mix_kernel<T, 32>, grid, 128, 0, s, X, W, Y, Kin, Kout, cR, (ll)Kin * cR, (ll)Kout * cR, skip);
   } else {
     Gemm<T> g;
     g.M = Kout; g.N = cR; g.K = Kin;

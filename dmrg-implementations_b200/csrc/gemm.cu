@@ -138,7 +138,10 @@ static void launch_impl(const Gemm<T>& d, int splitk, cudaStream_t st) {
   cfg.blockDim = dim3(G::THREADS);
   cfg.dynamicSmemBytes = S::BYTES;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  at[0] = pdl_attribute();
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
   constexpr int BK = S::TileA::BK;
   const int chunk = ceil_div(ceil_div(d.K, splitk), BK) * BK;
   const int nsplit = ceil_div(d.K, chunk);
@@ -150,12 +153,11 @@ static void launch_impl(const Gemm<T>& d, int splitk, cudaStream_t st) {
     a.sA1 = a.sA2 = a.sB1 = a.sB2 = a.sC1 = a.sC2 = 0;
     a.nb2 = 1;
     cfg.gridDim.z = nsplit;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 1;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = nsplit;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 1;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = nsplit;
+    cfg.numAttrs = 2;
   }
   DMRG2_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<T, G, TA, TB, CA, VA, VB>, a));
   DMRG2_CHECK_LAUNCH();

@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(G::THREADS) gemm_kernel(GemmArgs g) {
   constexpr int MI = WM / 16, NI = WN / 8, BK = S::TileA::BK;
   constexpr bool CPLX = ST<T>::cplx;
   static_assert(CPLX || NI % 2 == 0, "column pairs");
+  pdl_wait();
   if (g.skip && *((volatile const int*)g.skip)) {
     if (g.Cin && (g.kchunk == 0 || blockIdx.z == 0)) {
       const T* src = reinterpret_cast<const T*>(g.Cin);

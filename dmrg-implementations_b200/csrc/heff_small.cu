@@ -120,6 +120,7 @@ __device__ __forceinline__ void tile_product(Acc<T> (&acc)[MT], const T* As, int
 
 template <typename T, int MT3>
 __global__ void __launch_bounds__(HS_THREADS) heff_small_kernel(HsArgs g) {
+  pdl_wait();
   if (g.skip && *((volatile const int*)g.skip)) return;  // constant during the launch: the whole cluster leaves
   cg::cluster_group cluster = cg::this_cluster();
   const int q = (int)cluster.block_rank(), C = (int)cluster.num_blocks();
@@ -298,13 +299,14 @@ void hs_launch(const HsPlan& p, const HsArgs& a, cudaStream_t s) {
   cfg.blockDim = dim3(HS_THREADS);
   cfg.dynamicSmemBytes = p.smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  at[1] = pdl_attribute();
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = p.C;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   DMRG2_CUDA(cudaLaunchKernelEx(&cfg, heff_small_kernel<T, MT3>, a));
   DMRG2_CHECK_LAUNCH();
 }

@@ -496,6 +496,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
   constexpr int CV = ST<T>::cplx ? 2 : 1;
   const int tid = threadIdx.x;
   const bool lead = blockIdx.x == 0;
+  pdl_wait();
   // one thread per block reads the state (every warp of 148 blocks reading these words took 2.6 us:
   // they are one L2 line), all fields in one round trip
   __shared__ int s_j, s_guard, s_done;
@@ -610,6 +611,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
   __shared__ double wsum[LS_WARPS], xch_s[2][LS_CLUSTER], tot;
   const int tid = threadIdx.x;
   const bool lead = blockIdx.x == 0;
+  pdl_wait();
   if (CL) cooperative_groups::this_cluster().sync();  // the peers run: their shared memory may be written
   const ll x0 = (ll)blockIdx.x * chunk;
   const int len = (int)max((ll)0, min((ll)chunk, n - x0));
@@ -674,7 +676,9 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
     lz_ritz_norm_kernel(const T* V, ll n, T* out, LanczosDev* st, double* part, LanczosHost* host, int chunk) {
   extern __shared__ __align__(16) unsigned char ls_smem[];
   __shared__ double r[KRYLOV_CAP], wsum[LS_WARPS], xch[LS_CLUSTER], tot;
-  const int tid = threadIdx.x, k = st->n_iter;
+  const int tid = threadIdx.x;
+  pdl_wait();
+  const int k = st->n_iter;
   if (CL) cooperative_groups::this_cluster().sync();  // the peers run: their shared memory may be written
   if (blockIdx.x == gridDim.x - 1 && tid == 0) lz_report(st, host);
   T* ws = reinterpret_cast<T*>(ls_smem);
@@ -940,8 +944,11 @@ void launch_step(K kernel, std::atomic<unsigned long long>& attr, std::atomic<un
   cfg.blockDim = dim3(LS_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  at[1] = pdl_attribute();
+  cfg.numAttrs = 1;
   if (g.cluster) {
+    cfg.numAttrs = 2;  // (not with the cooperative launch)
     func_attr_once(attr_c, (const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = g.blocks;
@@ -952,7 +959,6 @@ void launch_step(K kernel, std::atomic<unsigned long long>& attr, std::atomic<un
     at[0].val.cooperative = 1;
   }
   cfg.attrs = at;
-  cfg.numAttrs = 1;
   DMRG2_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
   DMRG2_CHECK_LAUNCH();
 }

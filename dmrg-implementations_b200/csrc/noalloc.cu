@@ -108,6 +108,7 @@ size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 template <typename T>
 __global__ void wwt_kernel(const T* __restrict__ WL, const T* __restrict__ WR, T* __restrict__ out,
                            int Dl, int Dm, int Dr, int d) {
+  pdl_wait();
   const ll rows = (ll)d * d * Dr, cols = (ll)Dl * d * d;
   const ll i = (ll)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * cols) return;
@@ -133,6 +134,7 @@ __global__ void __launch_bounds__(1024) wwt_nonzeros_kernel(const T* __restrict_
   __shared__ int cnt[MIX_WIDE_K];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned mask[R][R];
+  pdl_wait();
 #pragma unroll
   for (int h = 0; h < R; ++h) {
     const int o = warp + 32 * h;
@@ -216,8 +218,7 @@ void heff_noalloc(int cL, int cR, int d, int Dl, int Dm, int Dr, const T* L, con
   T* X = (T*)(base + wwt_b);
   T* Y = (T*)(base + wwt_b + xs_b);
   const ll entries = dd * Dr * Dl * dd;
-  wwt_kernel<T><<<(unsigned)((entries + 255) / 256), 256, 0, s>>>(WL, WR, WWt, Dl, Dm, Dr, d);
-  DMRG2_CHECK_LAUNCH();
+  launch_pdl(wwt_kernel<T>, (unsigned)((entries + 255) / 256), 256, 0, s, WL, WR, WWt, Dl, Dm, Dr, d);
   // A large mixing step goes over W's nonzeros, where the scratch has room for that form beside
   // the rest (its size does not count against the caller's limit). Building it and the launch that
   // returns at once cost about 6 us, the mixing then its traffic; the batched GEMM on the dense
@@ -233,8 +234,7 @@ void heff_noalloc(int cL, int cR, int d, int Dl, int Dm, int Dr, const T* L, con
     T* val = (T*)(base + wwt_b + 2 * xs_b);
     int* rowp = (int*)(val + (ll)Kin * Kout);
     int* flags = (int*)(base + wwt_b + 2 * xs_b + sp_b - 256);
-    wwt_nonzeros_kernel<T><<<1, 1024, 0, s>>>(WWt, val, rowp, Kin, Kout, flags);
-    DMRG2_CHECK_LAUNCH();
+    launch_pdl(wwt_nonzeros_kernel<T>, 1, 1024, 0, s, WWt, val, rowp, Kin, Kout, flags);
     heff_apply<T>(L, R, WWt, theta, out, X, Y, cL, cR, d, Dl, Dr, nullptr, s, val, flags);
     return;
   }
