@@ -30,6 +30,8 @@
 //      compact-WY blocks to its own slab of columns (columns are independent).
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include <cstdlib>
 
 #include "gemm.cuh"
@@ -845,13 +847,24 @@ __device__ inline double hash_unit(unsigned long long x) {
   x ^= x >> 31;
   return (double)(x >> 11) * (1.0 / 9007199254740992.0) * 2.0 - 1.0;
 }
+// 1/a from the hardware estimate and two Newton-Raphson steps y <- y + y (1 - a y); 0 and values
+// outside the estimate's range take the division
+__device__ __forceinline__ double invit_rcp(double a) {
+  const double m = fabs(a);
+  if (!(m > 1e-290 && m < 1e290)) return 1.0 / a;
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  y = fma(y, fma(-a, y, 1.0), y);
+  return fma(y, fma(-a, y, 1.0), y);
+}
 
 __global__ void tridiag_invit_kernel(const double* __restrict__ dg, const double* __restrict__ eg,
                                      int n, int K, const double* __restrict__ lam,
-                                     const SvdOut* __restrict__ tr, double* __restrict__ Z, double gtol_rel) {
+                                     const SvdOut* __restrict__ tr, double* __restrict__ Z, double gtol_rel,
+                                     int vpb) {
   extern __shared__ double dsh[];
   __shared__ double tn_s;
-  const int vpb = blockDim.x;  // one vector per thread
+  // one vector per thread, vpb of the block's 32 (or more) threads
   double* d = dsh;
   double* e = dsh + n;
   double* base = dsh + 2 * n;  // [6][n][vpb]: factors, then the iterate
@@ -860,14 +873,16 @@ __global__ void tridiag_invit_kernel(const double* __restrict__ dg, const double
     e[i] = (i < n - 1) ? eg[i] : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {  // |T|_inf once per CTA
+  if (threadIdx.x < 32) {  // |T|_inf once per CTA
     double tn = 0.0;
-    for (int i = 0; i < n; ++i) tn = fmax(tn, fabs(d[i]) + fabs(i > 0 ? e[i - 1] : 0.0) + fabs(e[i]));
-    tn_s = tn;
+    for (int i = threadIdx.x; i < n; i += 32)
+      tn = fmax(tn, fabs(d[i]) + fabs(i > 0 ? e[i - 1] : 0.0) + fabs(e[i]));
+    for (int o = 16; o > 0; o >>= 1) tn = fmax(tn, __shfl_xor_sync(0xffffffffu, tn, o));
+    if (threadIdx.x == 0) tn_s = tn;
   }
   __syncthreads();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= K) return;
+  const int j = blockIdx.x * vpb + threadIdx.x;
+  if ((int)threadIdx.x >= vpb || j >= K) return;
   if (j >= tr->k) {
     for (int i = 0; i < n; ++i) Z[(ll)i * K + j] = 0.0;
     return;
@@ -895,67 +910,89 @@ __global__ void tridiag_invit_kernel(const double* __restrict__ dg, const double
       if (fmin(gap_up, gap_dn) >= 1e4 * shift) sft = (gap_up >= gap_dn) ? lam[first] + shift : lam[last] - shift;
     }
   }
+  // Bound by the dependent chain of one row (reciprocal, product, update): the row exchange is
+  // selects on one path (lanes that differ would run both branches, each with its division),
+  // the reciprocal the hardware's estimate and two Newton steps, and the next row's entries are
+  // loaded ahead of this row's stores. At n = K = 512: 216 us with branches, a division per row
+  // and loads behind the stores, 137 us now.
   double c0 = d[0] - sft, c1 = e[0];
-  for (int i = 0; i < n - 1; ++i) {
-    const double s = e[i];
-    const double dn = d[i + 1] - sft;
-    const double en = e[i + 1];
-    if (fabs(c0) >= fabs(s)) {
-      if (fabs(c0) < tiny) c0 = (c0 < 0 ? -tiny : tiny);
-      const double r = 1.0 / c0;
-      const double m = s * r;
+  {
+    double s = e[0], dn = d[1 < n ? 1 : 0] - sft, en = e[1 < n ? 1 : 0];
+    for (int i = 0; i < n - 1; ++i) {
+      const int i1 = min(i + 1, n - 1), i2 = min(i + 2, n - 1);
+      const double s1 = e[i1], dn1 = d[i2] - sft, en1 = e[i2];
+      const bool sw = fabs(c0) < fabs(s);
+      const double cc = (!sw && fabs(c0) < tiny) ? (c0 < 0 ? -tiny : tiny) : c0;
+      const double r = invit_rcp(sw ? s : cc);
+      const double m = (sw ? cc : s) * r;
       SX(0, i) = r;
-      SX(1, i) = c1;
-      SX(2, i) = 0.0;
+      SX(1, i) = sw ? dn : c1;
+      SX(2, i) = sw ? en : 0.0;
       SX(3, i) = m;
-      SX(4, i) = 0.0;
-      c0 = dn - m * c1;
-      c1 = en;
-    } else {
-      const double r = 1.0 / s;
-      const double m = c0 * r;
-      SX(0, i) = r;
-      SX(1, i) = dn;
-      SX(2, i) = en;
-      SX(3, i) = m;
-      SX(4, i) = 1.0;
-      c0 = c1 - m * dn;
-      c1 = -m * en;
+      SX(4, i) = sw ? 1.0 : 0.0;
+      const double n0 = sw ? fma(-m, dn, c1) : fma(-m, c1, dn);
+      c1 = sw ? -m * en : en;
+      c0 = n0;
+      s = s1;
+      dn = dn1;
+      en = en1;
     }
   }
   if (fabs(c0) < tiny) c0 = (c0 < 0 ? -tiny : tiny);
-  SX(0, n - 1) = 1.0 / c0;
+  SX(0, n - 1) = invit_rcp(c0);
   SX(1, n - 1) = 0.0;
   SX(2, n - 1) = 0.0;
-  // the iterate lives in shared memory next to the factors; column j of Z is written at the end
+  // the iterate lives in shared memory next to the factors; column j of Z is written at the end.
+  // Its scale (1 / norm of the last iteration) is applied as it is read, and the random start is
+  // made as it is first read: two passes less over the shared memory per iteration.
 #define IZ(i) SX(5, i)
-  for (int i = 0; i < n; ++i) IZ(i) = hash_unit(((unsigned long long)(j + 1) << 32) ^ (unsigned long long)i);
+  double inv = 1.0;
   for (int it = 0; it < 2; ++it) {
-    double y = IZ(0);
-    for (int i = 0; i < n - 1; ++i) {
-      double yn = IZ(i + 1), yi = y;
-      if (SX(4, i) != 0.0) { yi = yn; yn = y; }
-      IZ(i) = yi;
-      y = yn - SX(3, i) * yi;
+    auto read = [&](int i) {
+      return it == 0 ? hash_unit(((unsigned long long)(j + 1) << 32) ^ (unsigned long long)i) : IZ(i) * inv;
+    };
+    double y = read(0);
+    {
+      double yn = read(n > 1 ? 1 : 0), m = SX(3, 0), sw = SX(4, 0);
+      for (int i = 0; i < n - 1; ++i) {
+        const int i1 = min(i + 1, n - 2), i2 = min(i + 2, n - 1);
+        const double yn1 = read(i2), m1 = SX(3, i1), sw1 = SX(4, i1);  // ahead of the store
+        const double yi = sw != 0.0 ? yn : y, yo = sw != 0.0 ? y : yn;
+        IZ(i) = yi;
+        y = fma(-m, yi, yo);
+        yn = yn1;
+        m = m1;
+        sw = sw1;
+      }
     }
     IZ(n - 1) = y;
     double x1 = 0.0, x2 = 0.0, nrm = 0.0;
-    for (int i = n - 1; i >= 0; --i) {
-      const double xi = (IZ(i) - SX(1, i) * x1 - SX(2, i) * x2) * SX(0, i);
-      IZ(i) = xi;
-      nrm += xi * xi;
-      x2 = x1;
-      x1 = xi;
+    {
+      double v = y, u1 = SX(1, n - 1), u2 = SX(2, n - 1), r = SX(0, n - 1);
+      for (int i = n - 1; i >= 0; --i) {
+        const int i1 = max(i - 1, 0);
+        const double v1 = IZ(i1), u11 = SX(1, i1), u21 = SX(2, i1), r1 = SX(0, i1);
+        const double xi = fma(-u1, x1, fma(-u2, x2, v)) * r;
+        IZ(i) = xi;
+        nrm = fma(xi, xi, nrm);
+        x2 = x1;
+        x1 = xi;
+        v = v1;
+        u1 = u11;
+        u2 = u21;
+        r = r1;
+      }
     }
     nrm = sqrt(nrm);
     if (!(nrm > 0.0) || !isfinite(nrm)) {
       for (int i = 0; i < n; ++i) IZ(i) = (i == (n - 1 - j) % n) ? 1.0 : 0.0;
+      inv = 1.0;
       break;
     }
-    const double inv = 1.0 / nrm;
-    for (int i = 0; i < n; ++i) IZ(i) *= inv;
+    inv = 1.0 / nrm;
   }
-  for (int i = 0; i < n; ++i) Z[(ll)i * K + j] = IZ(i);
+#pragma unroll 8
+  for (int i = 0; i < n; ++i) Z[(ll)i * K + j] = IZ(i) * inv;
 #undef IZ
 #undef SX
 }
@@ -1514,7 +1551,7 @@ void tridiag_eigvecs(const double* d, const double* e, int n, int K, const doubl
   int vpb = (int)std::min<size_t>(8, (220 * 1024 - sizeof(double) * 2 * (size_t)n) / per);
   if (vpb < 1) throw std::runtime_error("inverse iteration: matrix order too large");
   const size_t smem = sizeof(double) * 2 * (size_t)n + per * vpb;
-  tridiag_invit_kernel<<<(K + vpb - 1) / vpb, vpb, smem, s>>>(d, e, n, K, lam, tr, Z, gtol_rel);
+  tridiag_invit_kernel<<<(K + vpb - 1) / vpb, std::max(vpb, 32), smem, s>>>(d, e, n, K, lam, tr, Z, gtol_rel, vpb);
   DMRG2_CHECK_LAUNCH();
 }
 
