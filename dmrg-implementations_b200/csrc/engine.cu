@@ -156,8 +156,8 @@ class Engine final : public EngineBase {
       build_wmix_right(hW_[i].data(), Dl[i], Dr[i], d_, hmr[i]);
     }
     for (int i = 0; i + 1 < L_; ++i) build_wwt(hW_[i].data(), hW_[i + 1].data(), Dl[i], Dr[i], Dr[i + 1], d_, hww[i]);
-    // each bond's fused MPO also in its nonzero form; the mixing step uses it where at
-    // most half the entries are nonzero (DMRG2_MIX_DENSE=1: always the dense form)
+    // each bond's fused MPO also in its nonzero form; mixing steps of more than 32 inputs use it
+    // where at most half the entries are nonzero (DMRG2_MIX_DENSE=1: the dense product)
     static const bool mix_dense = [] {
       const char* e = std::getenv("DMRG2_MIX_DENSE");
       return e && e[0] == '1';
@@ -483,7 +483,8 @@ class Engine final : public EngineBase {
     const ll m = (ll)cL * d_, nc = (ll)d_ * cR;
     row_scale<T>(mps_[bs + 1], V, cM, nc, l.svdX, false, l.st);  // diag(V) psi_R
     theta_form(mps_[bs], l.svdX, l.theta, cL, cM, cR, d_, l.st);
-    const double e = lanczos(bs, m * nc, ss);
+    LanczosResult r = lanczos(bs, m * nc, false);
+    const double e = lanczos_stats(bs, cL, cR, r, ss);
     DMRG2_CUDA(cudaEventRecord(l.ev_c, l.st));
     DMRG2_CUDA(cudaMemcpyAsync(l.svdX, l.theta, sizeof(T) * (size_t)(m * nc), cudaMemcpyDeviceToDevice, l.st));
     set_identity(l.svdQ, (int)m, l.st);
@@ -734,8 +735,10 @@ class Engine final : public EngineBase {
     const int cL = dims_[i], cM = dims_[i + 1], cR = dims_[i + 2];
     const ll n = (ll)cL * d_ * d_ * cR;
     theta_form(mps_[i], mps_[i + 1], ln().theta, cL, cM, cR, d_, ln().st);
-    double e = lanczos(i, n, ss);
+    // the split is enqueued behind the solve; its own wait covers both
+    LanczosResult r = lanczos(i, n, true);
     svd_split(i, dir, chi, ss);
+    const double e = lanczos_stats(i, cL, cR, r, ss);
     if (dir == 'R')
       env_left(lenv_[i], mps_[i], wml_[i], lenv_[i + 1], ln().X, ln().Y, dims_[i], dims_[i + 1], d_, Dl_[i],
                Dr_[i], ln().st);
@@ -745,10 +748,10 @@ class Engine final : public EngineBase {
     return e;
   }
 
-  double lanczos(int i, ll n, SweepStats& ss) {
+  // the ground state of the bond's H_eff; defer: see lanczos_solve
+  LanczosResult lanczos(int i, ll n, bool defer) {
     const int cL = dims_[i], cR = dims_[i + 2];
     const int Dl = Db_[i], Dr = Db_[i + 2];
-    const double fl = heff_flops(cL, cR, d_, Dl, Dr, ST<T>::cplx);
     const ll kk = (ll)Dl * d_ * d_ * d_ * d_ * Dr;  // entries of the dense fused MPO
     const bool sparse = wwt_sparse_[i] != 0;
     auto mv = [&](const T* in, T* out, const int* skip) {
@@ -780,7 +783,7 @@ class Engine final : public EngineBase {
                                           graph ? &key_lp : nullptr);
       r = lanczos_solve<T>(ln().lw, ln().theta, n, std::min(cfg_.krylov_max, 16), cfg_.lanczos_tol, 1,
                            cfg_.seed + 7919u * (unsigned)i + 1u, mv_hp, ln().st, graph ? &key_hp : nullptr);
-      ss.lowprec_matvecs += lp.matvecs;
+      r.lowprec = lp.matvecs;
       r.matvecs += lp.matvecs;
       r.iters += lp.iters;
       r.matvec_s += lp.matvec_s;
@@ -795,14 +798,22 @@ class Engine final : public EngineBase {
       };
       const LzKey key{sparse ? 3 : 2, cL, cR, Dl, Dr, d_, (ll)sL, (ll)sR, (ll)sW, (ll)ln().X, (ll)ln().Y};
       r = lanczos_solve<T>(ln().lw, ln().theta, n, cfg_.krylov_max, cfg_.lanczos_tol, cfg_.max_restarts,
-                           cfg_.seed + 7919u * (unsigned)i, mvs, ln().st, &key);
+                           cfg_.seed + 7919u * (unsigned)i, mvs, ln().st, &key, defer);
     } else {
       r = lanczos_solve<T>(ln().lw, ln().theta, n, cfg_.krylov_max, cfg_.lanczos_tol, cfg_.max_restarts,
                            cfg_.seed + 7919u * (unsigned)i, mv, ln().st);
     }
+    return r;
+  }
+
+  // completes a solve (the stream has run it) and adds it to the sweep's statistics; cL, cR: the
+  // bond's outer dimensions at the solve
+  double lanczos_stats(int i, int cL, int cR, LanczosResult& r, SweepStats& ss) {
+    if (r.pending) lanczos_collect(ln().lw, r, ln().st);
     ss.heff_s += r.matvec_s;
     ss.matvecs += r.matvecs;
-    ss.heff_flops += fl * r.matvecs;
+    ss.lowprec_matvecs += r.lowprec;
+    ss.heff_flops += heff_flops(cL, cR, d_, Db_[i], Db_[i + 2], ST<T>::cplx) * r.matvecs;
     ss.lanczos_iters += r.iters;
     ss.device_loops += r.device_loops;
     if (!r.converged) ss.lanczos_unconverged += 1;

@@ -105,7 +105,30 @@ struct LanczosResult {
   int converged = 0;
   double matvec_s = 0.0;  // device time of the matvecs
   int device_loops = 0;   // restarts run as the device-looped graph
+  int lowprec = 0;        // of the matvecs, those on the split-BF16 operator (set by the engine)
+  bool pending = false;   // enqueued only: lanczos_collect completes it once the stream has run it
+  long long launches = 0, fixed = 0;  // kernels per loop body and around the loop (pending solves)
 };
+
+// Adds what the finished solve reported (W.h_st) to res; s: its stream (idle up to the solve's end).
+template <typename T>
+void lanczos_collect(LanczosWork<T>& W, LanczosResult& res, cudaStream_t s) {
+  const LanczosHost& h = *W.h_st;
+  if (!h.done || h.n_iter < 1) {
+    // (a grid barrier that gave up leaves its counters behind)
+    DMRG2_CUDA(cudaMemsetAsync(W.st, 0, sizeof(LanczosDev), s));
+    throw std::runtime_error("Lanczos did not terminate");
+  }
+  launch_counter() += h.guard * res.launches + res.fixed;
+  thread_launches() += h.guard * res.launches + res.fixed;
+  res.matvecs += h.guard;
+  res.iters += h.n_iter;
+  res.energy = h.e_cur;
+  res.matvec_s += (double)h.mv_ns * 1e-9;
+  res.converged = h.converged;
+  res.device_loops += 1;
+  res.pending = false;
+}
 
 // Captures one solve of W's buffers and this matvec into G (nothing runs): the start
 // (norm, first vector), the WHILE node over the Krylov steps, the Ritz vector with the
@@ -143,12 +166,14 @@ void lz_build_graph(LanczosWork<T>& W, GraphEntry& G, T* theta, ll n, int kmax, 
 // matvec(in, out, skip_flag) enqueues out = H in on stream s, doing nothing when
 // *skip_flag != 0 on the device. theta: start vector on entry, normalised Ritz
 // vector on exit. With a key: the device-looped form, cached in W.graphs (the key must
-// identify everything the matvec reads and writes besides in and out).
+// identify everything the matvec reads and writes besides in and out). With defer, a
+// device-looped solve without restarts is only enqueued (res.pending): the caller enqueues what
+// follows, waits for the stream and calls lanczos_collect, one host round trip less.
 template <typename T>
 LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, double tol,
                             int max_restarts, unsigned seed,
                             const std::function<void(const T*, T*, const int*)>& matvec,
-                            cudaStream_t s, const LzKey* key = nullptr) {
+                            cudaStream_t s, const LzKey* key = nullptr, bool defer = false) {
   LanczosResult res;
   const bool timed = !W.ev_mv.empty();
   const int kmax = (int)std::min<ll>(std::min(krylov_max, W.kcap), n);
@@ -172,29 +197,20 @@ LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, d
       build = true;
     }
   }
-  auto check_done = [&]() {
-    if (W.h_st->done && W.h_st->n_iter >= 1) return;
-    // (a grid barrier that gave up leaves its counters behind)
-    DMRG2_CUDA(cudaMemsetAsync(W.st, 0, sizeof(LanczosDev), s));
-    throw std::runtime_error("Lanczos did not terminate");
-  };
   for (int rs = 0; rs <= max_restarts; ++rs) {
     if (G && G->ex) {
       // the solve reads the pinned seed before the host writes it again (the wait below)
       *W.h_seed = seed + 104729u * (unsigned)rs;
       DMRG2_CUDA(cudaGraphLaunch(G->ex, s));
       W.graphs.replays += 1;
+      res.launches = G->launches;
+      res.fixed = G->fixed;
+      if (defer && max_restarts == 0) {
+        res.pending = true;
+        return res;
+      }
       DMRG2_CUDA(cudaStreamSynchronize(s));
-      check_done();
-      const int bodies = W.h_st->guard;
-      launch_counter() += bodies * G->launches + G->fixed;
-      thread_launches() += bodies * G->launches + G->fixed;
-      res.matvecs += bodies;
-      res.iters += W.h_st->n_iter;
-      res.energy = W.h_st->e_cur;
-      res.matvec_s += (double)W.h_st->mv_ns * 1e-9;
-      res.converged = W.h_st->converged;
-      res.device_loops += 1;
+      lanczos_collect(W, res, s);
       if (res.converged) break;
       continue;
     }
@@ -216,7 +232,10 @@ LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, d
     }
     lz_ritz(W.krylov, n, theta, W.st, W.red, W.h_st, s);
     DMRG2_CUDA(cudaStreamSynchronize(s));
-    check_done();
+    if (!W.h_st->done || W.h_st->n_iter < 1) {
+      DMRG2_CUDA(cudaMemsetAsync(W.st, 0, sizeof(LanczosDev), s));
+      throw std::runtime_error("Lanczos did not terminate");
+    }
     const int used = std::min(issued, W.h_st->n_iter);
     for (int j = 0; timed && j < used; ++j) {
       float ms = 0.f;
