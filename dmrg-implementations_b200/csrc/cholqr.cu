@@ -11,14 +11,15 @@
 // the peer's shared memory. A published tile is never written again, and nothing is
 // copied asynchronously, so the only exit condition is the final cluster barrier
 // (no CTA leaves while a peer may still read it). Per tile column t:
-//   P  CTA r > t: L_rt = A_rt X_tt^T with X_tt = L_tt^{-1}, whose fragments every warp reads
-//      straight from CTA t (one 16 x 8 piece per warp, FP64 tensor cores);
+//   P  CTA r > t: L_rt = A_rt X_tt^T with X_tt = L_tt^{-1}, staged from CTA t (one 16 x 8 piece per
+//      warp, FP64 tensor cores);
 //   T  CTA r > t: A_rj -= L_rt L_jt^T for the peers' tiles t < j < r (one warp per
 //      tile, the fragments of L_jt straight from CTA j) and the diagonal tile j = r (one 16 x 8
 //      piece per warp);
 //   D  CTA t, once its row is updated: in-register Cholesky of the diagonal tile
-//      (one warp, lane = row; the chain of pivots is the critical path), then X_tt by
-//      forward substitution (lane = column), then the counter says "row complete".
+//      (one warp, lane = row; the chain of pivots is the critical path) and, one block of
+//      8 columns behind in a second warp, X_tt by forward substitution (lane = column);
+//      then the counter says "row complete".
 // The critical path is one P, one diagonal update and one D per tile column; the
 // wider updates of the rows further down overlap with it. A poll that runs out marks
 // the result invalid (status) and the CTA carries on with what it has, so every CTA
@@ -27,8 +28,11 @@
 // by shuffles, behind it the finished 8 columns update the rest of the tile through shared
 // memory as one rank-8 product. Shuffling every column to all 31 others instead put ~265
 // cycles of issue between two pivots (35 us of a factor at k = 256).
-// Per factor at k = 256: 89.6 us before (fused multiply-add loops for P and T on staged
-// copies, 32-column shuffles in D), 67.6 us now.
+// Per factor at k = 256 inside a sweep: 89.6 us with multiply-add loops for P and T on staged copies
+// and 32-column shuffles in D, 67.6 us with the tensor cores and the blocked pivots. Back to back
+// (k = 256 / 512): 88.4 / 193 us with every row reading X_tt's fragments remotely as soon as it is
+// published (uncoalesced reads of one CTA by all others), 74.0 / 150 us staged in whole rows with
+// the critical row served first, 62.7 / 139 us with the inverse one block behind the factor.
 //
 // trsm_rows_kernel: Y = Z L^{-T}, 16 rows of Z per CTA, column block by column block:
 // Y_b = (Z_b - sum_{j<b} Y_j L_bj^T) X_bb^T on the FP64 tensor cores (DMMA), the tiles
@@ -69,10 +73,12 @@ __device__ inline bool wait_tiles(const int* peer_done, int need) {
 // column J of the in-register Cholesky of one diagonal tile (lane i holds row i) with a
 // reciprocal square root per pivot, then the columns after it (those of its block of 8 at
 // once, the rest at the block's end from blk, [NB][8] in shared memory); compile-time J keeps
-// every index of a[] static. Entries above the diagonal are left undefined.
+// every index of a[] static. Entries above the diagonal are left undefined. Each finished block
+// goes to L (shared memory, pitch TP) and is announced on named barrier 1 + block (the warp that
+// inverts the tile waits there).
 template <int J>
 __device__ __forceinline__ void tile_chol_col(double (&a)[NB], int lane, double piv_min, double piv_sub, bool& bad,
-                                              double* rd, double* blk) {
+                                              double* rd, double* blk, double* L) {
   constexpr int B0 = J & ~7, BE = B0 + 8;
   double piv = __shfl_sync(0xffffffffu, a[J], J);
   if (!(piv > piv_min)) {  // also catches NaN
@@ -86,6 +92,11 @@ __device__ __forceinline__ void tile_chol_col(double (&a)[NB], int lane, double 
   for (int c = J + 1; c < BE; ++c) {
     const double lc = __shfl_sync(0xffffffffu, a[J], c);
     a[c] -= a[J] * lc;
+  }
+  if constexpr (J + 1 == BE) {
+#pragma unroll
+    for (int q = B0; q < BE; ++q) L[lane * TP + q] = a[q];
+    asm volatile("bar.arrive %0, 64;" ::"r"(1 + B0 / 8) : "memory");
   }
   if constexpr (J + 1 == BE && BE < NB) {
     double2* row = reinterpret_cast<double2*>(blk + lane * 8);
@@ -104,7 +115,7 @@ __device__ __forceinline__ void tile_chol_col(double (&a)[NB], int lane, double 
     }
     __syncwarp();
   }
-  if constexpr (J + 1 < NB) tile_chol_col<J + 1>(a, lane, piv_min, piv_sub, bad, rd, blk);
+  if constexpr (J + 1 < NB) tile_chol_col<J + 1>(a, lane, piv_min, piv_sub, bad, rd, blk, L);
 }
 
 // acc += sign * A B^T for 16 rows of A and 8 rows of B, k = 0 .. NB-1; b[k step][2]: the
@@ -136,7 +147,8 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
   extern __shared__ __align__(16) double ctsm[];
   double* Lt = ctsm;                 // [C] tiles of block row r: A_rj, turned into L_rj
   double* Xr = Lt + C * TT;          // X_rr = L_rr^{-1} (zeros above the diagonal)
-  double* blk = Xr + TT;             // [NB][8] finished columns of D's current block
+  double* Xs = Xr + TT;              // X_tt of the tile column being solved
+  double* blk = Xs + TT;             // [NB][8] finished columns of D's current block
   double* Rd = blk + NB * 8;         // 1 / diag of L_rr
   __shared__ int done_s;             // tiles of this block row that are final (read by peers)
   __shared__ int fail_s;
@@ -199,13 +211,25 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
 
   if (r < nb) {
     for (int t = 0; t < r; ++t) {
-      // ---- P: L_rt = A_rt X_tt^T once CTA t has published X_tt (its row complete)
-      if (lane == 0 && !wait_tiles(cluster.map_shared_rank(&done_s, t), t + 1)) fail_s = 1;
-      __syncwarp();  // lane 0 acquired the tile for the warp
+      // ---- P: L_rt = A_rt X_tt^T once CTA t has published X_tt (its row complete). The next row
+      // (r = t + 1) is the critical one: the others wait for its L first, so that their reads of
+      // X_tt do not compete with its own
+      {
+        const int from = r == t + 1 ? t : t + 1;
+        if (lane == 0 && !wait_tiles(cluster.map_shared_rank(&done_s, from), t + 1)) fail_s = 1;
+        __syncwarp();  // lane 0 acquired the tile for the warp
+        const double* Xp = cluster.map_shared_rank(Xr, t);
+        double v[NB / CT_WARPS];
+#pragma unroll
+        for (int u = 0; u < NB / CT_WARPS; ++u) v[u] = Xp[(warp * (NB / CT_WARPS) + u) * TP + lane];
+#pragma unroll
+        for (int u = 0; u < NB / CT_WARPS; ++u) Xs[(warp * (NB / CT_WARPS) + u) * TP + lane] = v[u];
+      }
+      __syncthreads();
       double* Art = T_(Lt, t);
       {
         double b[NB / 8][2], o[4] = {0.0, 0.0, 0.0, 0.0};
-        load_frag(b, cluster.map_shared_rank(Xr, t) + pc * TP, gq, tq);
+        load_frag(b, Xs + pc * TP, gq, tq);
         piece_mma(o, Art + pr * TP, 1.0, b, gq, tq);
         __syncthreads();  // the tile is read before it is overwritten
 #pragma unroll
@@ -248,19 +272,19 @@ __global__ void __launch_bounds__(CT_THREADS, 1)
       }
       __syncthreads();  // tile (r, t+1) and the diagonal tile are final for this column
     }
-    // ---- D: L_rr (registers, lane = row), then X_rr = L_rr^{-1} (lane = column)
+    // ---- D: warp 0 factors L_rr (registers, lane = row); warp 1 inverts it (lane = column), one
+    // block of 8 rows behind: row i of X_rr needs L_rr's columns up to i only
+    double* Lrr = T_(Lt, r);
     if (warp == 0) {
-      double* Lrr = T_(Lt, r);
       double a[NB];
 #pragma unroll
       for (int j = 0; j < NB; ++j) a[j] = (j <= lane) ? Lrr[lane * TP + j] : 0.0;
-      tile_chol_col<0>(a, lane, piv_min, piv_sub, bad, Rd, blk);
-#pragma unroll
-      for (int j = 0; j < NB; ++j) Lrr[lane * TP + j] = (j <= lane) ? a[j] : 0.0;
-      __syncwarp();
+      tile_chol_col<0>(a, lane, piv_min, piv_sub, bad, Rd, blk, Lrr);
+    } else if (warp == 1) {
       double x[NB];
 #pragma unroll
       for (int i = 0; i < NB; ++i) {
+        if (i % 8 == 0) asm volatile("bar.sync %0, 64;" ::"r"(1 + i / 8) : "memory");
         // four partial sums break the dependent chain of the row's dot product
         double s0 = (i == lane) ? 1.0 : 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
 #pragma unroll
@@ -449,7 +473,7 @@ __global__ void __launch_bounds__(256) col_scale_kernel(double* __restrict__ Y, 
 template <int C>
 void chol_tiles_launch(const double* G, int k, int nb, ll ldg, double* LX, ll ldx, int* status, double rel_tol,
                        double shift_rel, double* dscale, cudaStream_t s) {
-  constexpr size_t smem = sizeof(double) * ((size_t)(C + 1) * TT + NB * 8 + NB);
+  constexpr size_t smem = sizeof(double) * ((size_t)(C + 2) * TT + NB * 8 + NB);
   static std::atomic<unsigned long long> attr{0};
   set_smem_attr_once(attr, (const void*)chol_tiles_kernel<C>, (int)smem);
   if constexpr (C > 8) {
