@@ -37,6 +37,8 @@ template <> struct ST<double> {
   __host__ __device__ static double re(double a) { return a; }
   __host__ __device__ static double im(double) { return 0.0; }
   __host__ __device__ static double abs2(double a) { return a * a; }
+  __host__ __device__ static bool finite(double a) { return a - a == 0.0; }
+  __host__ __device__ static bool nonzero(double a) { return a != 0.0; }
   __host__ __device__ static double make(double r, double) { return r; }
   __host__ __device__ static double mul(double a, double b) { return a * b; }
   __host__ __device__ static double add(double a, double b) { return a + b; }
@@ -52,6 +54,8 @@ template <> struct ST<zc> {
   __host__ __device__ static double re(zc a) { return a.re; }
   __host__ __device__ static double im(zc a) { return a.im; }
   __host__ __device__ static double abs2(zc a) { return a.re * a.re + a.im * a.im; }
+  __host__ __device__ static bool finite(zc a) { return a.re - a.re == 0.0 && a.im - a.im == 0.0; }
+  __host__ __device__ static bool nonzero(zc a) { return a.re != 0.0 || a.im != 0.0; }
   __host__ __device__ static zc make(double r, double i) { return mkz(r, i); }
   __host__ __device__ static zc mul(zc a, zc b) { return a * b; }
   __host__ __device__ static zc add(zc a, zc b) { return a + b; }

@@ -107,8 +107,13 @@ __global__ void __launch_bounds__(MIX_WIDE_NT)
   const T* xa = X + blockIdx.y * sX + e;
   T* ya = Y + blockIdx.y * sY + e;
   const int* col = rowp + Kout + 1;
+  bool bad = false;
 #pragma unroll 8
-  for (int k = warp; k < Kin; k += W) xs[k * 32 + lane] = in ? xa[(ll)k * cR] : ST<T>::zero();
+  for (int k = warp; k < Kin; k += W) {
+    const T x = in ? xa[(ll)k * cR] : ST<T>::zero();
+    bad |= !ST<T>::finite(x);
+    xs[k * 32 + lane] = x;
+  }
   for (int i = threadIdx.x; i <= Kout; i += MIX_WIDE_NT) rp[i] = rowp[i];
   // (the slots behind the last nonzero exist: the block holds Kin Kout of them)
   const int st = min(MIX_WIDE_NNZ, Kin * Kout);
@@ -116,7 +121,20 @@ __global__ void __launch_bounds__(MIX_WIDE_NT)
     cs[i] = col[i] * 32;
     vs[i] = val[i];
   }
-  __syncthreads();
+  // An infinity or a NaN among the inputs: zero entries count too, as in the dense product.
+  if (__syncthreads_or(bad)) {
+    for (int o = warp; o < Kout; o += W) {
+      const int j1 = rp[o + 1];
+      T acc = ST<T>::zero();
+      for (int k = 0, j = rp[o]; k < Kin; ++k) {
+        const bool nz = j < j1 && col[j] == k;
+        acc = acc + ST<T>::mul(nz ? val[j] : ST<T>::zero(), xs[k * 32 + lane]);
+        j += nz;
+      }
+      if (in) ya[(ll)o * cR] = acc;
+    }
+    return;
+  }
   const bool staged = rp[Kout] <= MIX_WIDE_NNZ;
   for (int o = warp; o < Kout; o += W) {
     const int j0 = rp[o], j1 = rp[o + 1];
@@ -142,7 +160,7 @@ int wwt_sparse_block(std::vector<T>& w, int Kin, int Kout) {
     ints[(size_t)o] = nnz;
     for (int k = 0; k < Kin; ++k) {
       const T v = w[(size_t)o * Kin + k];
-      if (ST<T>::abs2(v) != 0.0) {
+      if (ST<T>::nonzero(v)) {
         val[(size_t)nnz] = v;
         ints[(size_t)(Kout + 1 + nnz)] = k;
         ++nnz;

@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(HS_THREADS) heff_small_kernel(HsArgs g) {
 #pragma unroll
     for (int h = 0; h < HS_KMAX / HS_WARPS; ++h) {
       const int o = warp + h * HS_WARPS;
-      const bool nz = ST<T>::abs2(wv[h]) != 0.0;
+      const bool nz = ST<T>::nonzero(wv[h]);
       const unsigned m = __ballot_sync(0xffffffffu, nz);
       if (nz) {
         const int at = o * Kin + __popc(m & ((1u << lane) - 1u));
@@ -174,6 +174,7 @@ __global__ void __launch_bounds__(HS_THREADS) heff_small_kernel(HsArgs g) {
   __syncthreads();
 
   // ---- step 1
+  bool bad = false;  // an infinity or a NaN in X
   {
     const int nt = cols / 8, et = El / 8;
     const int kc = ((kp1 / 8 + g.ks1 - 1) / g.ks1) * 8;
@@ -190,12 +191,16 @@ __global__ void __launch_bounds__(HS_THREADS) heff_small_kernel(HsArgs g) {
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int row = gq + ((r & 2) ? 8 : 0);
-        if (row < rows1) xo[row * g.pX + (r & 1)] = acc[0].get(r);
+        if (row < rows1) {
+          xo[row * g.pX + (r & 1)] = acc[0].get(r);
+          bad |= !ST<T>::finite(acc[0].get(r));
+        }
       }
     }
   }
-  __syncthreads();
-  // ---- step 2 (columns beyond cR get zeros: step 3 sums over them)
+  bad = __syncthreads_or(bad);
+  // ---- step 2 (columns beyond cR get zeros: step 3 sums over them; with an infinity or a NaN in X
+  // the zeros of WW count too, as in a dense product)
   {
     const ll xsl = (ll)g.Ta * Dl * g.pX;
     for (int u = tid; u < na * Kout * El; u += HS_THREADS) {
@@ -205,13 +210,13 @@ __global__ void __launch_bounds__(HS_THREADS) heff_small_kernel(HsArgs g) {
         const T* x = Xs + (ll)al * Dl * g.pX + e;
         const unsigned char* wc = wcol + o * Kin;
         const T* wl = wval + o * Kin;
-        const int cnt = wcnt[o];
+        const int cnt = bad ? Kin : wcnt[o];
         for (int j = 0; j < cnt; ++j) {
-          const int k = wc[j];
+          const int k = bad ? j : wc[j];
           const T* xk = x + koff[k];
           T v = xk[0];
           for (int sl = 1; sl < g.ks1; ++sl) v = v + xk[sl * xsl];
-          sum = sum + ST<T>::mul(wl[j], v);
+          sum = sum + ST<T>::mul(bad ? Wg[o * Kin + j] : wl[j], v);
         }
       }
       Ys[(al * dd + o / Dr) * g.pY + (o % Dr) * El + e] = sum;

@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(1024) wwt_nonzeros_kernel(const T* __restrict_
     int n = 0;
 #pragma unroll
     for (int g = 0; g < R; ++g) {
-      mask[h][g] = __ballot_sync(0xffffffffu, ST<T>::abs2(v[g]) != 0.0);
+      mask[h][g] = __ballot_sync(0xffffffffu, ST<T>::nonzero(v[g]));
       n += __popc(mask[h][g]);
     }
     if (lane == 0) cnt[o] = n;

@@ -5,6 +5,8 @@ beyond it, dense and sparse MPOs, against numpy.
 Each output is a sum of cL Dl d^2 Dr cR products in three stages; with inputs of unit size the
 rounding error stays below eps (cL + Dl d^2 + Dr cR) of the result's scale.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -47,3 +49,33 @@ def test_heff_matches_numpy(shape, sparse, cplx):
     out = dmrg2.apply_heff(L, R, WL, WR, th)
     scale = max(np.abs(ref).max(), 1e-300)
     assert np.abs(out - ref).max() <= 2.3e-16 * (cL + Dl * d * d + Dr * cR) * scale
+
+
+@pytest.mark.parametrize("shape,cplx", [((16, 9, 2, 5, 5, 5), False), ((17, 33, 2, 8, 8, 8), True),
+                                        ((128, 128, 5, 4, 4, 4), True), ((160, 150, 3, 8, 8, 8), False)])
+def test_zeros_of_a_sparse_mpo(shape, cplx):
+    """The forms that go over the MPO's nonzeros treat its zeros as the dense product does: an entry
+    whose square underflows counts, and an infinity times a zero is NaN in every output it meets."""
+    import torch
+    cL, cR, d, Dl, Dm, Dr = shape
+    rng = np.random.default_rng(12)
+    dt = np.complex128 if cplx else np.float64
+    L, R, WL, WR, th = (rng.standard_normal(s).astype(dt) for s in (
+        (cL, Dl, cL), (cR, Dr, cR), (Dl, Dm, d, d), (Dm, Dr, d, d), (cL, d, d, cR)))
+    WL *= (rng.random(WL.shape) < 0.15) * 1e-100
+    WR *= (rng.random(WR.shape) < 0.15) * 1e-100
+
+    def run(th):
+        t = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (L, R, WL, WR, th)]
+        out = torch.empty_like(t[4])
+        rc = dmrg2.load_library().dmrg2_op_heff_noalloc(
+            dmrg2.C128 if cplx else dmrg2.F64, *shape, *[ctypes.c_void_p(x.data_ptr()) for x in (*t, out)],
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == 0
+        return out.cpu().numpy()
+
+    ref = _ref(L, R, WL * 1e100, WR * 1e100, th)
+    out = run(th) * 1e100 * 1e100
+    assert np.abs(out - ref).max() <= 2.3e-16 * (cL + Dl * d * d + Dr * cR + 4) * np.abs(ref).max()
+    th[cL // 2, 0, d - 1, cR - 1] = np.inf
+    assert not np.isfinite(run(th)).any()
