@@ -1,6 +1,4 @@
 // extern "C" boundary of the engine (declared in include/dmrg2_b200.h).
-#include <sys/mman.h>
-
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
@@ -12,8 +10,6 @@
 #include <memory>
 #include <random>
 #include <string>
-#include <system_error>
-#include <utility>
 #include <vector>
 
 #include "../../include/dmrg2_b200.h"
@@ -84,40 +80,6 @@ struct DBuf {
   DBuf& operator=(const DBuf&) = delete;
   template <typename T>
   T* as() const { return (T*)p; }
-};
-
-// Makes the pages of the caller's result arrays resident while the device works. Result arrays are
-// usually fresh memory, whose first write per page is a fault, which the copy back then waits
-// for. MADV_POPULATE_WRITE does not change the contents; where the kernel refuses it, the copy
-// back faults as before. For the splits, whose host otherwise waits for milliseconds of device
-// work (512 x 512, 256 kept: 3430 -> 2840 us per call); an environment update or a matvec has
-// too little of it to hide a thread (490 -> 500-550 us).
-class Prefault {
- public:
-  void add(void* p, size_t bytes) {
-    if (p && bytes >= MIN_BYTES) ranges_.push_back({p, bytes});
-  }
-  void start() {
-    if (ranges_.empty()) return;
-    try {
-      t_ = std::thread([r = ranges_] {
-        for (const auto& x : r) {
-          const uintptr_t page = 4095, b = (uintptr_t)x.first & ~page, e = ((uintptr_t)x.first + x.second + page) & ~page;
-          (void)madvise((void*)b, e - b, 23 /* MADV_POPULATE_WRITE */);
-        }
-      });
-    } catch (const std::system_error&) {  // no thread: the copy back takes the faults
-    }
-  }
-  void join() {
-    if (t_.joinable()) t_.join();
-  }
-  ~Prefault() { join(); }
-
- private:
-  static constexpr size_t MIN_BYTES = 256 << 10;  // below, a thread costs more than the faults
-  std::vector<std::pair<void*, size_t>> ranges_;
-  std::thread t_;
 };
 
 // reference column-major MPS  ->  row-major (a, s, b)
@@ -201,18 +163,12 @@ void do_op_svd_eig(int m, int n, const void* M, int max_bond, double cutoff, cha
   const int nn = R ? m : n;
   const int kmin = std::min(m, n);
   DBuf dM(M, sb * (size_t)m * n), dl(sb * (size_t)m * kmin), dr(sb * (size_t)kmin * n);
-  const size_t kc = (size_t)std::min(max_bond, kmin);
-  Prefault pf;
-  pf.add(left, sb * m * kc);
-  pf.add(right, sb * kc * n);
-  pf.start();
   EigWork<T> W;
   std::vector<double> lam(nn);
   try {
     W.init(nn, nn);
     SvdOut o = eig_split<T>(W, dM.as<T>(), m, n, R ? 'R' : 'L', std::min(max_bond, kmin), cutoff,
                             false, dl.as<T>(), dr.as<T>(), 0, nn, lam.data());
-    pf.join();
     const int k = o.k;
     if (S)
       for (int r = 0; r < kmin; ++r) S[r] = std::sqrt(std::max(lam[r], 0.0));
@@ -241,17 +197,12 @@ bool do_op_warm_split(int m, int n, const void* M, const void* warm, int k, char
   red.counter = cnt.as<unsigned>();
   red.nblk = 1184;
   DMRG2_CUDA(cudaMemset(cnt.p, 0, sizeof(unsigned) * 4));
-  Prefault pf;
-  pf.add(left, sb * (size_t)m * k);
-  pf.add(right, sb * (size_t)k * n);
-  pf.start();
   WstWork W;
   bool ok = false;
   double te = 0.0;
   try {
     W.init(std::max(m, n), k);
     ok = wst_split(W, red, dM.as<double>(), m, n, dir, k, dw.as<double>(), dl.as<double>(), dr.as<double>(), te, 0);
-    pf.join();
     if (ok) {
       if (left) DMRG2_CUDA(cudaMemcpy(left, dl.p, sb * (size_t)m * k, cudaMemcpyDeviceToHost));
       if (right) DMRG2_CUDA(cudaMemcpy(right, dr.p, sb * (size_t)k * n, cudaMemcpyDeviceToHost));
