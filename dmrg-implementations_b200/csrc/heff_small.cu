@@ -295,6 +295,11 @@ HsPlan hs_plan(int cL, int cR, int dd, int Dl, int Dr) {
   return p;
 }
 
+template <typename T>
+bool overlaps(const T* a, ll na, const T* b, ll nb) {
+  return (uintptr_t)a < (uintptr_t)(b + nb) && (uintptr_t)b < (uintptr_t)(a + na);
+}
+
 template <typename T, int MT3>
 void hs_launch(const HsPlan& p, const HsArgs& a, cudaStream_t s) {
   static std::atomic<unsigned long long> attr{0};
@@ -321,6 +326,11 @@ void hs_launch(const HsPlan& p, const HsArgs& a, cudaStream_t s) {
 template <typename T>
 bool heff_small(const T* Lenv, const T* Renv, const T* WWt, const T* in, T* out, int cL, int cR, int dd, int Dl, int Dr,
                 const int* skip, cudaStream_t s) {
+  // Clusters write their rows of out while others still read the operands: an out that shares memory
+  // with the input or the left environment (which the tiled contractions are done with before
+  // they write out) is theirs to serve.
+  const ll n = (ll)cL * dd * cR;
+  if (overlaps(out, n, in, n) || overlaps(out, n, Lenv, (ll)cL * Dl * cL)) return false;
   const HsPlan p = hs_plan<T>(cL, cR, dd, Dl, Dr);
   if (!p.C) return false;
   HsArgs a;

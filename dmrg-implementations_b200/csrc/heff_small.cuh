@@ -22,7 +22,7 @@ inline bool heff_small_fits(int cL, int cR, int dd, int Dl, int Dr) {
 
 // out = H_eff in, with dd the physical dimension of the block (d^2 of a two-site bond, d of one
 // site) and WWt the (dd Dr) x (Dl dd) mixing matrix; false, with nothing launched, where the
-// shape is not one for this kernel
+// shape is not one for this kernel, or out overlaps in or Lenv
 template <typename T>
 bool heff_small(const T* Lenv, const T* Renv, const T* WWt, const T* in, T* out, int cL, int cR, int dd, int Dl, int Dr,
                 const int* skip, cudaStream_t s);

@@ -282,7 +282,9 @@ int dmrg2_op_gemm_bf16x3(int dtype, int transA, int transB, int M, int N, int K,
  * without synchronising. The first call on each device resolves the scratch
  * address and loads its module; make it before any stream capture. All calls
  * on a device share the one scratch array: calls on the same stream are safe,
- * calls that overlap in time on other streams or threads race. */
+ * calls that overlap in time on other streams or threads race. out may be theta
+ * itself, or overlap theta, L, WL or WR (their contents are then lost); it must not
+ * overlap R. */
 #define DMRG2_NOALLOC_SCRATCH_BYTES (64ull << 20)
 int dmrg2_op_heff_noalloc(int dtype, int cL, int cR, int d, int Dl, int Dm, int Dr, const void* L,
                           const void* R, const void* WL, const void* WR, const void* theta, void* out,

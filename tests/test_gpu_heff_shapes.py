@@ -79,3 +79,37 @@ def test_zeros_of_a_sparse_mpo(shape, cplx):
     assert np.abs(out - ref).max() <= 2.3e-16 * (cL + Dl * d * d + Dr * cR + 4) * np.abs(ref).max()
     th[cL // 2, 0, d - 1, cR - 1] = np.inf
     assert not np.isfinite(run(th)).any()
+
+
+@pytest.mark.parametrize("shape,cplx", [((16, 24, 2, 5, 5, 5), False), ((64, 64, 2, 5, 5, 5), False),
+                                        ((30, 25, 3, 4, 4, 4), True), ((96, 90, 2, 5, 5, 5), False),
+                                        ((64, 64, 5, 4, 4, 4), True)])
+@pytest.mark.parametrize("where", ["theta", "shifted", "L"])
+def test_out_may_overlap_theta_or_the_left_environment(shape, cplx, where):
+    """The one-launch form writes rows of the result while other clusters still read the operands, so
+    calls whose result overlaps them take the tiled contractions, at every size."""
+    import torch
+    cL, cR, d, Dl, Dm, Dr = shape
+    rng = np.random.default_rng(13)
+    dt = np.complex128 if cplx else np.float64
+
+    def rnd(*s):
+        x = rng.standard_normal(s)
+        return x + 1j * rng.standard_normal(s) if cplx else x
+
+    L, R, WL, WR, th = rnd(cL, Dl, cL), rnd(cR, Dr, cR), rnd(Dl, Dm, d, d), rnd(Dm, Dr, d, d), rnd(cL, d, d, cR)
+    ref = _ref(L, R, WL, WR, th)
+    n = th.size
+    # one buffer: [left environment | theta | room for a shifted result]
+    buf = torch.from_numpy(np.concatenate([L.ravel(), th.ravel(), np.zeros(n, dt)])).cuda()
+    Rd, WLd, WRd = (torch.from_numpy(x).cuda() for x in (R, WL, WR))
+    at_th = L.size
+    # (two elements further keeps 16-byte alignment)
+    at_out = {"theta": at_th, "shifted": at_th + 2, "L": 0}[where]
+    ptr = [ctypes.c_void_p(x) for x in (buf.data_ptr(), Rd.data_ptr(), WLd.data_ptr(), WRd.data_ptr(),
+                                        buf[at_th:].data_ptr(), buf[at_out:].data_ptr())]
+    rc = dmrg2.load_library().dmrg2_op_heff_noalloc(dmrg2.C128 if cplx else dmrg2.F64, *shape, *ptr,
+                                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    out = buf[at_out:at_out + n].cpu().numpy().reshape(ref.shape)
+    assert np.abs(out - ref).max() <= 2.3e-16 * (cL + Dl * d * d + Dr * cR) * np.abs(ref).max()
