@@ -1131,7 +1131,8 @@ class Engine final : public EngineBase {
     l.svdX = (T*)al(sizeof(T) * (size_t)nmax_);
     l.svdQ = (T*)al(sizeof(T) * (size_t)(qmax_ * qmax_));
     l.tmp = (T*)al(sizeof(T) * (size_t)cfg_.chi_max * cfg_.chi_max);
-    l.lw.init(cfg_.krylov_max, nmax_);
+    // lanes of a parallel sweep run beside other lanes' Jacobi merges
+    l.lw.init(cfg_.krylov_max, nmax_, true, !primary || cfg_.svd_method == 1);
     l.ew.init((int)qmax_, cfg_.chi_max);
     if (primary) bytes_ += l.lw.bytes(nmax_) + l.ew.bytes;
     if (warm_capable(cfg_)) {

@@ -42,9 +42,10 @@ struct RedScratch {
   double* part = nullptr;   // [nblk][ncoef*2]
   unsigned* counter = nullptr;
   int nblk = 0;
+  int step_blocks = 0;      // blocks a cooperative Lanczos kernel may have (0: none is launched)
 };
 
-constexpr int STEP_BLOCKS = 148;  // blocks of a cooperative Lanczos step (one per SM)
+constexpr int STEP_BLOCKS = 148;  // blocks of a cooperative Lanczos step at most (one per SM)
 int vec_blocks(ll n);
 // blocks' worth of partial sums (2 (KRYLOV_CAP + 2) each) RedScratch::part holds for vectors
 // of up to n elements: the streaming passes', or the fused step's two sets

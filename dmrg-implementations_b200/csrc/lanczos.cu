@@ -266,7 +266,8 @@ __device__ bool lz_finish_step(LanczosDev* st, StepState& sh, int k, int kmax, d
 // solves the tridiagonal problem while the others finish their slices. Every block sums the
 // partial products itself, in the same fixed order.
 // The barrier: up to LS_CLUSTER blocks are one thread-block cluster (hardware barrier);
-// beyond, a cooperative launch of one block per SM with a counter barrier (bounded).
+// beyond, a cooperative launch of one block per SM with a counter barrier (bounded), except
+// where Jacobi kernels of other streams would keep it waiting (cooperative_step_blocks).
 // The staged basis is read four times a step, so a slice costs one pass over the L2.
 // Per step at chi = 256 (n = 262,144, 3 Krylov vectors) 31 us in five launches before and
 // 15 us now; in a 12-site chain at chi = 64 (n <= 16,384) 33 us before, 16 us now.
@@ -287,14 +288,15 @@ struct StepGrid {
 };
 
 template <typename T>
-static StepGrid step_grid(ll n) {
+static StepGrid step_grid(ll n, int coop) {
   // slices of 512 elements (one per thread) until 16 blocks are reached, which a cluster holds up
-  // to 2048 elements each; then one block per SM
+  // to 2048 elements each; then one block per SM (`coop` of them at most)
   StepGrid g;
   const ll cl_max = 2048 / (ll)(sizeof(T) / sizeof(double));
   ll nb = (n + LS_THREADS - 1) / LS_THREADS;
   g.cluster = n <= LS_CLUSTER * cl_max;
-  const ll cap = g.cluster ? LS_CLUSTER : STEP_BLOCKS;
+  const ll cap = g.cluster ? LS_CLUSTER : std::min(coop, STEP_BLOCKS);
+  if (cap < 1) return g;
   if (nb > cap) nb = cap;
   const ll ch = ((n + nb - 1) / nb + 1) & ~1ll;  // even: 16-byte slices
   if (ch * (ll)sizeof(T) > (ll)LS_SMEM_W) return g;
@@ -1001,7 +1003,7 @@ void norm2(const T* x, ll n, double* out_dev, RedScratch& r, cudaStream_t s) {
 template <typename T>
 void lz_start(T* theta, T* v0, ll n, LanczosDev* st, RedScratch& r, unsigned seed, double tol,
               int kmax, cudaStream_t s, T* cur, const unsigned* seed_host) {
-  const StepGrid g = step_grid<T>(n);
+  const StepGrid g = step_grid<T>(n, r.step_blocks);
   if (g.blocks && g.cluster) return start_launch<T, true>(g, theta, v0, cur, n, st, r, seed, seed_host, tol, kmax, s);
   if (g.blocks) return start_launch<T, false>(g, theta, v0, cur, n, st, r, seed, seed_host, tol, kmax, s);
   norm2<T>(theta, n, &st->nrm2, r, s);
@@ -1027,7 +1029,7 @@ void step_passes(T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, int km
 
 template <typename T>
 void lz_step(T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, int kmax, int* host_done, cudaStream_t s) {
-  const StepGrid g = step_grid<T>(n);
+  const StepGrid g = step_grid<T>(n, r.step_blocks);
   if (g.blocks && g.cluster)
     return step_launch<T, true>(g, V, nv, n, w, nullptr, st, r, kmax, 0, cudaGraphConditionalHandle{}, host_done, s);
   if (g.blocks)
@@ -1043,7 +1045,7 @@ void lz_step(T* V, int nv, ll n, T* w, LanczosDev* st, RedScratch& r, int kmax, 
 template <typename T>
 void lz_step_dev(T* V, ll n, T* w, T* cur, LanczosDev* st, RedScratch& r, int kmax, cudaGraphConditionalHandle h,
                  cudaStream_t s) {
-  const StepGrid g = step_grid<T>(n);
+  const StepGrid g = step_grid<T>(n, r.step_blocks);
   if (g.blocks && g.cluster) return step_launch<T, true>(g, V, 0, n, w, cur, st, r, kmax, 1, h, nullptr, s);
   if (g.blocks) return step_launch<T, false>(g, V, 0, n, w, cur, st, r, kmax, 1, h, nullptr, s);
   step_passes<T>(V, -1, n, w, st, r, kmax, s);
@@ -1055,7 +1057,7 @@ void lz_step_dev(T* V, ll n, T* w, T* cur, LanczosDev* st, RedScratch& r, int km
 
 template <typename T>
 void lz_ritz(const T* V, ll n, T* out, LanczosDev* st, RedScratch& r, LanczosHost* host, cudaStream_t s) {
-  const StepGrid g = step_grid<T>(n);
+  const StepGrid g = step_grid<T>(n, r.step_blocks);
   if (g.blocks && g.cluster) return ritz_launch<T, true>(g, V, n, out, st, r, host, s);
   if (g.blocks) return ritz_launch<T, false>(g, V, n, out, st, r, host, s);
   lz_ritz_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(V, n, out, st);

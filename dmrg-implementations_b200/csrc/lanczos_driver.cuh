@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <array>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <stdexcept>
@@ -36,6 +37,26 @@ using LzKey = std::array<long long, 11>;
 // below the cap keep what the cutoff leaves); a graph is a few kilobytes
 constexpr int LZ_GRAPH_CAP = 1024;
 
+// Blocks a solve's cooperative kernels may have (vectors beyond the cluster form): one per SM this
+// context has (fewer than 148 in a partition of the GPU). None where other streams run Jacobi
+// kernels beside the solve (`shared`): a cooperative kernel starts only once every SM can take
+// one of its blocks, a Jacobi split holds some SMs for tens of milliseconds, and all solves wait for
+// it at every Krylov step, where the streaming passes fit in between. Segments of a parallel sweep
+// (L = 100, chi = 256, ms per iteration of 2 / 4 / 8 segments): 281 / 431 / 1235 cooperative,
+// 239 / 400 / 509 with 74 blocks, 243 / 360 / 494 streaming. Engines with Jacobi splits (L = 30,
+// chi = 128, s for 1 / 4 / 6 at once): 2.31 / 2.60 / 2.98 cooperative, 2.31 / 2.39 / 2.51 streaming.
+// Engines with the other splits gain from the cooperative form also together (8 requests at
+// L = 40, chi = 256: 1.36 s streaming, 0.77 s with all of the cooperative form's changes).
+// DMRG2_TEST_STEP_BLOCKS caps the count (tests).
+inline int cooperative_step_blocks(bool shared) {
+  if (shared) return 0;
+  int dev = 0, sms = 0;
+  DMRG2_CUDA(cudaGetDevice(&dev));
+  DMRG2_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (const char* e = std::getenv("DMRG2_TEST_STEP_BLOCKS")) sms = std::min(sms, std::atoi(e));
+  return std::min(sms, STEP_BLOCKS);
+}
+
 template <typename T>
 struct LanczosWork {
   static constexpr int POLL_RING = 8;
@@ -54,7 +75,9 @@ struct LanczosWork {
   std::vector<void*> owned;
 
   // timing: the host-driven form measures its matvecs (an event pair per Krylov step)
-  void init(int kcap_, ll nmax, bool timing = true) {
+  // shared: see cooperative_step_blocks
+  void init(int kcap_, ll nmax, bool timing = true, bool shared = false) {
+    red.step_blocks = cooperative_step_blocks(shared);
     graphs.cap = LZ_GRAPH_CAP;
     graphs.name = "lanczos";
     kcap = std::min(kcap_, KRYLOV_CAP);

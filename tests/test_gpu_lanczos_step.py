@@ -6,6 +6,10 @@ The lengths n = 4 cL cR cover one block, one full cluster and the first length b
 grid of one block per SM, ragged slices, and (680 x 680) the streaming passes that serve
 vectors beyond the step kernel's shared memory.
 """
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -80,3 +84,22 @@ def test_zero_start_is_replaced_by_a_random_vector():
                for c in (ev[2][0], ev[2][-1]) for d in (ev[3][0], ev[3][-1]))
     assert abs(e - best) < 1e-9 * abs(best)
     assert abs(np.linalg.norm(v) - 1.0) < 1e-13
+
+
+CHILD = """
+import test_gpu_lanczos_step as t
+for case in [(64, 129, False), (100, 101, False), (150, 151, True)]:
+    t.test_fixed_number_of_steps_matches_numpy(*case)
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("blocks", [0, 17, 60])
+def test_fewer_blocks_than_sms(blocks):
+    """A context with fewer SMs (a partition of the GPU) runs the cooperative kernels on as many blocks, and
+    the streaming passes where there are none."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, DMRG2_TEST_STEP_BLOCKS=str(blocks), PYTHONPATH=os.pathsep.join([here] + sys.path))
+    r = subprocess.run([sys.executable, "-c", CHILD], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.split() == ["ok"], r.stderr
+
