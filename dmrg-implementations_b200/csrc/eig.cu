@@ -1328,38 +1328,61 @@ __global__ void __launch_bounds__(AQ_THREADS, 1)
   }
 }
 
-// max |S - I| over the leading k x k block; sets out->ns_done once below tol.
+// The leading k x k block of S = Z^T Z against 1, E = S - 1: ns_done once every entry of E is below
+// tol; else ns_near says whether one Newton-Schulz step Z (3 - S) / 2 brings it there. That step
+// leaves -3/4 E^2 + 1/4 E^3 (the step's Gram matrix is (1 - E/2)^2 (1 + E)); with q the largest
+// squared norm of a row of E, no entry of E^2 is above q (Cauchy-Schwarz; its diagonal reaches q),
+// and none of E^3 above q |E|_2 <= q sqrt(k q). Rounding of S and of the step adds at most
+// (2 rows + 8) 2^-53 per entry, 0.56 tol for the callers' tol = 4e-16 rows; the bound may take the rest.
 // Partial maxima per CTA, the last CTA to arrive decides.
-__global__ void ns_check_kernel(const double* __restrict__ S, int K, SvdOut* out, double tol,
-                                double* part, unsigned* counter) {
-  __shared__ double mx[256];
+constexpr int NSC_BLOCKS = 32;
+constexpr double NSC_STEP_SHARE = 0.4;
+__global__ void __launch_bounds__(256) ns_check_kernel(const double* __restrict__ S, int K, SvdOut* out, double tol,
+                                                       double* part, unsigned* counter) {
+  __shared__ double mx[8], rows[8];
   __shared__ int last;
-  const int k = min(out->k, K);
-  double m = 0.0;
+  const int k = min(out->k, K), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // (a maximum that keeps a NaN)
+  auto worse = [](double a, double b) { return (b > a || b != b) ? b : a; };
+  double m = 0.0, q = 0.0;
   if (!out->ns_done)
-    for (ll e = (ll)blockIdx.x * blockDim.x + threadIdx.x; e < (ll)k * k; e += (ll)gridDim.x * blockDim.x) {
-      const int a = (int)(e / k), b = (int)(e % k);
-      m = fmax(m, fabs(S[(ll)a * K + b] - (a == b ? 1.0 : 0.0)));
+    for (int a = blockIdx.x * 8 + warp; a < k; a += NSC_BLOCKS * 8) {
+      const double* row = S + (ll)a * K;
+      double ss = 0.0;
+      for (int b = lane; b < k; b += 32) {
+        const double e = row[b] - (a == b ? 1.0 : 0.0);
+        m = fmax(m, fabs(e));
+        ss = fma(e, e, ss);
+      }
+      q = worse(q, warp_sum_d(ss));
     }
-  mx[threadIdx.x] = m;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) mx[threadIdx.x] = fmax(mx[threadIdx.x], mx[threadIdx.x + o]);
-    __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) {
+    mx[warp] = m;
+    rows[warp] = q;
   }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    part[blockIdx.x] = mx[0];
+    for (int w = 1; w < 8; ++w) {
+      m = fmax(m, mx[w]);
+      q = worse(q, rows[w]);
+    }
+    part[blockIdx.x] = m;
+    part[NSC_BLOCKS + blockIdx.x] = q;
     __threadfence();
     last = (atomicAdd(counter, 1u) == gridDim.x - 1);
   }
   __syncthreads();
   if (last && threadIdx.x == 0) {
     __threadfence();
-    double t = 0.0;
-    for (int b = 0; b < (int)gridDim.x; ++b) t = fmax(t, part[b]);
+    m = q = 0.0;
+    for (int b = 0; b < NSC_BLOCKS; ++b) {
+      m = fmax(m, part[b]);
+      q = worse(q, part[NSC_BLOCKS + b]);
+    }
     if (!out->ns_done) {
-      if (t < tol) out->ns_done = 1;
-      out->ns_near = t * t < tol ? 1 : 0;
+      if (m < tol) out->ns_done = 1;
+      out->ns_near = q * (0.75 + 0.25 * sqrt(k * q)) < NSC_STEP_SHARE * tol ? 1 : 0;
     }
     *counter = 0u;
   }
@@ -1620,7 +1643,7 @@ void apply_q(const T* R, ll ld, const T* tau, int n, const double* Z, int K, con
 
 void ns_check(const double* S, int K, SvdOut* out, double tol, double* part, unsigned* counter,
               cudaStream_t s) {
-  ns_check_kernel<<<32, 256, 0, s>>>(S, K, out, tol, part, counter);
+  ns_check_kernel<<<NSC_BLOCKS, 256, 0, s>>>(S, K, out, tol, part, counter);
   DMRG2_CHECK_LAUNCH();
 }
 

@@ -94,7 +94,7 @@ struct SvdOut {
   int jacobi_sweeps;
   int jacobi_err;
   int ns_done;      // eigenvector block already orthonormal (Newton-Schulz steps skipped)
-  int ns_near;      // one Newton-Schulz step makes it so (its deviation squared is below the tolerance)
+  int ns_near;      // one Newton-Schulz step makes it so (a bound on every entry it leaves is below the tolerance)
 };
 
 template <typename T>
@@ -134,6 +134,7 @@ void wy_build(const T* R, ll ld, const T* tau, int n, int K, T* Tb, cudaStream_t
 template <typename T>
 void apply_q(const T* R, ll ld, const T* tau, int n, const double* Z, int K, const SvdOut* tr, T* Zg,
              T* Tb, cudaStream_t s, bool wy_ready = false);
+// sets out->ns_done and out->ns_near from S = Z^T Z (K x K); part: 64 doubles
 void ns_check(const double* S, int K, SvdOut* out, double tol, double* part, unsigned* counter,
               cudaStream_t s);
 // Up to `iters` Newton-Schulz steps of Z (n x K) in one launch, with ns_check's flag; false, with

@@ -374,8 +374,8 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
   };
   const int* done = &W.out->ns_done;
   // Newton-Schulz polish of the nearly orthonormal Z (rows x k) into dst: S = Z^T Z; within tol of
-  // the identity Z is copied, else dst = 1.5 Z - 0.5 Z S, whose deviation is the square of Z's
-  // (a deviation too large for one step makes the split report a failure)
+  // the identity Z is copied, else dst = 1.5 Z - 0.5 Z S. The result is not measured again: a split
+  // whose bound on it (ns_check) is above tol reports a failure
   auto orth = [&](double* Z, ll rows, double tol, double* dst) {
     mul(true, Z, k, k, k, (int)rows, Z, k, false, W.S, k, 1.0, 0.0, nullptr);
     ns_check(W.S, k, W.out, tol, W.part, W.counter, s);

@@ -130,7 +130,7 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
     extract_pairs(W.Z2, rows, k, dst, s);
   };
   // one Newton-Schulz step on the embedding of Z (rows x k) unless it is orthonormal already, result
-  // into dst; a deviation too large for one step makes the split report a failure
+  // into dst; a split whose bound on the step's result (ns_check) is above the tolerance reports a failure
   auto polish = [&](const zc* Z, ll rows, zc* dst) {
     const ll r2 = 2 * rows;
     embed_pairs(Z, rows, k, W.Z1, s);
