@@ -132,10 +132,12 @@ inline int ceil_div(ll a, ll b) { return (int)((a + b - 1) / b); }
 
 // Test hook for the bounded device waits: with DMRG2_TEST_UNSIGNALLED_WAITS=1 in the
 // environment, the kernels that wait on a completion (the tensor-core commit of the
-// split GEMM, the grid barrier of the cooperative Jacobi SVD) wait on one that nothing
-// signals, with a short poll limit, so a test can see the timeout reported as
-// DMRG2_ERR_NUMERIC while the device stays usable.
+// split GEMM, the grid barriers of the cooperative Jacobi SVD and of the cooperative Lanczos
+// kernels) wait on one that nothing signals, with a short poll limit, so a test can see the
+// timeout reported as DMRG2_ERR_NUMERIC while the device stays usable. The value start, step
+// or ritz picks that Lanczos kernel alone. In the Lanczos kernels it is the last block's wait.
 bool test_unsignalled_waits();
+bool test_unsignalled_wait(const char* kernel);
 
 // Device memory of the library, from the device's stream-ordered pool (cudaMallocAsync
 // on a private stream of the calling thread, which the call then waits for). Unlike

@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -114,6 +115,11 @@ bool test_unsignalled_waits() {
     return e && e[0] == '1';
   }();
   return on;
+}
+
+bool test_unsignalled_wait(const char* kernel) {
+  static const char* e = std::getenv("DMRG2_TEST_UNSIGNALLED_WAITS");
+  return e && (e[0] == '1' || std::strcmp(e, kernel) == 0);
 }
 
 template <typename T, typename G, bool TA, bool TB, bool CA, bool VA, bool VB>

@@ -18,6 +18,7 @@ struct LanczosDev {
   double e_prev, e_cur;
   double tol;
   int done;                            // 1 once converged / broken down / Krylov space full
+  int gave_up;                         // a block's bounded wait at a grid barrier ran out: no result
   int converged;
   int n_iter;                          // size of the tridiagonal matrix
   int randomized;
@@ -35,6 +36,7 @@ struct LanczosHost {
   double e_cur;
   unsigned long long mv_ns;
   int done, converged, n_iter, guard;
+  int gave_up;  // cleared by the host before a solve, only ever set by its kernels
 };
 
 // Reduction scratch shared by the vector kernels.

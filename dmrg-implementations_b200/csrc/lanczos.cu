@@ -280,6 +280,7 @@ constexpr size_t LS_SMEM_W = 96 * 1024;        // slice of w per block at most
 // for a second block, since the clusters of concurrent solves share the SMs
 constexpr size_t LS_SMEM_GRID = 176 * 1024, LS_SMEM_CLUSTER = 72 * 1024;
 constexpr long long LS_SPIN = 1ll << 22;       // barrier polls before a block gives up (seconds)
+constexpr long long LS_SPIN_TEST = 1ll << 14;  // the same under the unsignalled-wait test hook
 
 struct StepGrid {
   int blocks = 0;  // 0: the vector does not fit, the streaming passes run
@@ -311,9 +312,11 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
   return v;
 }
 
-// all blocks of the grid meet; false when the bounded wait ran out
+// all blocks of the grid meet; false when this block's bounded wait ran out (unsignalled: the test
+// hook, the last block waits for one more than there are). The caller records it in st->gave_up: a
+// single block that went on without the others has wrong sums, whoever it is.
 template <bool CL>
-__device__ __forceinline__ bool step_barrier(unsigned* bar) {
+__device__ __forceinline__ bool step_barrier(unsigned* bar, int unsignalled) {
   if constexpr (CL) {
     cooperative_groups::this_cluster().sync();
     return true;
@@ -321,11 +324,14 @@ __device__ __forceinline__ bool step_barrier(unsigned* bar) {
     __syncthreads();
     bool ok = true;
     if (threadIdx.x == 0) {
+      const bool hook = unsignalled && blockIdx.x == gridDim.x - 1;
+      const unsigned need = gridDim.x + (hook ? 1u : 0u);
+      const long long spin = hook ? LS_SPIN_TEST : LS_SPIN;
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
       long long it = 0;
-      while (ld_acquire_gpu(bar) < gridDim.x && ++it < LS_SPIN) {
+      while (ld_acquire_gpu(bar) < need && ++it < spin) {
       }
-      ok = it < LS_SPIN;
+      ok = it < spin;
     }
     return __syncthreads_and(ok ? 1 : 0) != 0;
   }
@@ -434,7 +440,7 @@ __device__ __forceinline__ double slice_update(const BasisSlice<T>& V, int nv, T
 // go through part[c][block] and the grid barrier. Returns false when a bounded wait ran out.
 template <bool CL>
 __device__ __forceinline__ bool exchange_sums(const double* wsum, int wpitch, int ncoef, double* part, unsigned* bar,
-                                              double* xch, double* dst) {
+                                              double* xch, double* dst, int unsignalled) {
   const int tid = threadIdx.x, lane = tid & 31, nblk = gridDim.x;
   const bool push = CL && ncoef <= LS_PUSH;
   __syncthreads();
@@ -449,7 +455,7 @@ __device__ __forceinline__ bool exchange_sums(const double* wsum, int wpitch, in
       part[(ll)c * nblk + blockIdx.x] = s;
     }
   }
-  const bool ok = step_barrier<CL>(bar);
+  const bool ok = step_barrier<CL>(bar, unsignalled);
   if (push) {
     for (int c = tid; c < ncoef; c += LS_THREADS) {
       double s = 0.0;
@@ -490,7 +496,7 @@ __device__ __forceinline__ void copy_async(T* dst, const T* src, int count, bool
 template <typename T, bool CL>
 __global__ void __launch_bounds__(LS_THREADS, 1)
     lz_step_kernel(T* V, int nv, ll n, const T* w, T* cur, LanczosDev* st, double* part, int kmax, int chunk,
-                   int ncache, int loop, cudaGraphConditionalHandle h, volatile int* host_done) {
+                   int ncache, int loop, cudaGraphConditionalHandle h, volatile int* host_done, int unsignalled) {
   extern __shared__ __align__(16) unsigned char ls_smem[];
   __shared__ StepState sh;
   __shared__ double csum[2 * KRYLOV_CAP + 1];
@@ -504,7 +510,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
   __shared__ int s_j, s_guard, s_done;
   __shared__ double s_eprev, s_tol;
   if (tid == 0) {
-    s_done = *((volatile int*)&st->done);
+    s_done = *((volatile int*)&st->done) | *((volatile int*)&st->gave_up);
     s_j = *((volatile int*)&st->j);
     s_guard = *((volatile int*)&st->guard);
     s_eprev = *((volatile double*)&st->e_prev);
@@ -512,7 +518,9 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
   }
   __syncthreads();
   const int j = s_j, guard = s_guard;
-  if (s_done) {  // set by an earlier launch only: the same for every block
+  // set by an earlier launch, so the same for every block (or by a block of this one that gave up
+  // waiting for this block: the solve is lost either way)
+  if (s_done) {
     if (lead && tid == 0) {
       if (host_done) *host_done = 1;
       if (loop) cudaGraphSetConditional(h, 0u);
@@ -549,7 +557,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
   cp_async_wait<0>();
   __syncthreads();
   slice_dots<T>(B, nv, ws, len, wsum, wpitch);
-  bool ok = exchange_sums<CL>(wsum, wpitch, nc, part, &st->bar[0], xch, csum);
+  bool ok = exchange_sums<CL>(wsum, wpitch, nc, part, &st->bar[0], xch, csum, unsignalled);
   const double a0 = csum[CV * (nv - 1)];
   {
     const double ww = warp_sum(slice_update<T>(B, nv, ws, len, csum));
@@ -557,7 +565,8 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
     if ((tid & 31) == 0) wsum[(tid >> 5) * wpitch + nc] = ww;
   }
   ok = exchange_sums<CL>(wsum, wpitch, nc + 1, part + (ll)nc * gridDim.x, &st->bar[1],
-                         xch + (CL ? LS_CLUSTER * LS_PUSH : 0), csum) && ok;
+                         xch + (CL ? LS_CLUSTER * LS_PUSH : 0), csum, unsignalled) && ok;
+  if (!ok && tid == 0) *((volatile int*)&st->gave_up) = 1;
   double c2 = 0.0;
   for (int c = 0; c < nc; ++c) c2 += csum[c] * csum[c];
   const double nrm2 = fmax(csum[nc] - c2, 0.0);
@@ -609,7 +618,7 @@ __device__ inline double hash_uniform(unsigned long long x) {
 template <typename T, bool CL>
 __global__ void __launch_bounds__(LS_THREADS, 1)
     lz_start_kernel(T* theta, T* v0, T* cur, ll n, LanczosDev* st, double* part, unsigned seed,
-                    const unsigned* seed_host, double tol, int kmax, int chunk) {
+                    const unsigned* seed_host, double tol, int kmax, int chunk, int unsignalled) {
   __shared__ double wsum[LS_WARPS], xch_s[2][LS_CLUSTER], tot;
   const int tid = threadIdx.x;
   const bool lead = blockIdx.x == 0;
@@ -622,7 +631,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
     for (int x = tid; x < len; x += LS_THREADS) ww += ST<T>::abs2(theta[x0 + x]);
     ww = warp_sum(ww);
     if ((tid & 31) == 0) wsum[tid >> 5] = ww;
-    return exchange_sums<CL>(wsum, 1, 1, p, bar, xch, &tot);
+    return exchange_sums<CL>(wsum, 1, 1, p, bar, xch, &tot, unsignalled);
   };
   if (lead && tid == 0 && !CL) *((volatile unsigned*)&st->bar[4]) = 0u;  // the last solve's
   bool ok = norm(part, &st->bar[2], xch_s[0]);
@@ -644,6 +653,7 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
     v0[x0 + x] = v;
     if (cur) cur[x0 + x] = v;
   }
+  if (!ok && tid == 0) *((volatile int*)&st->gave_up) = 1;
   if (lead && tid == 0) {
     st->nrm2 = tot;
     st->randomized = tiny ? 1 : 0;
@@ -669,13 +679,15 @@ __device__ __forceinline__ void lz_report(const LanczosDev* st, LanczosHost* hos
   h->converged = st->converged;
   h->n_iter = st->n_iter;
   h->guard = st->guard;
+  if (st->gave_up) h->gave_up = 1;
 }
 __global__ void lz_report_kernel(const LanczosDev* st, LanczosHost* host) { lz_report(st, host); }
 
 // end of a solve: out = sum_i ritz_i v_i, normalised, and the report to the host
 template <typename T, bool CL>
 __global__ void __launch_bounds__(LS_THREADS, 1)
-    lz_ritz_norm_kernel(const T* V, ll n, T* out, LanczosDev* st, double* part, LanczosHost* host, int chunk) {
+    lz_ritz_norm_kernel(const T* V, ll n, T* out, LanczosDev* st, double* part, LanczosHost* host, int chunk,
+                        int unsignalled) {
   extern __shared__ __align__(16) unsigned char ls_smem[];
   __shared__ double r[KRYLOV_CAP], wsum[LS_WARPS], xch[LS_CLUSTER], tot;
   const int tid = threadIdx.x;
@@ -698,7 +710,8 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
   }
   ww = warp_sum(ww);
   if ((tid & 31) == 0) wsum[tid >> 5] = ww;
-  exchange_sums<CL>(wsum, 1, 1, part, &st->bar[4], xch, &tot);
+  if (!exchange_sums<CL>(wsum, 1, 1, part, &st->bar[4], xch, &tot, unsignalled) && tid == 0)
+    *((volatile int*)&host->gave_up) = 1;
   const double inv = tot > 0.0 ? 1.0 / sqrt(tot) : 0.0;
   for (int x = tid; x < len; x += LS_THREADS) out[x0 + x] = ST<T>::scale(inv, ws[x]);
   if (blockIdx.x == 0 && tid == 0) st->nrm2 = tot;
@@ -974,21 +987,21 @@ void step_launch(const StepGrid& g, T* V, int nv, ll n, const T* w, T* cur, Lanc
   const int ncache = cap > row ? (int)std::min<size_t>((cap - row) / row, (size_t)nvm) : 0;
   const size_t smem = row * (size_t)(1 + ncache) + sizeof(double) * (size_t)LS_WARPS * (nc + 1);
   launch_step(lz_step_kernel<T, CL>, attr, attr_c, g, smem, s, V, nv, n, w, cur, st, r.part, kmax, g.chunk,
-              ncache, loop, h, (volatile int*)host_done);
+              ncache, loop, h, (volatile int*)host_done, test_unsignalled_wait("step") ? 1 : 0);
 }
 template <typename T, bool CL>
 void start_launch(const StepGrid& g, T* theta, T* v0, T* cur, ll n, LanczosDev* st, RedScratch& r, unsigned seed,
                   const unsigned* seed_host, double tol, int kmax, cudaStream_t s) {
   static std::atomic<unsigned long long> attr{0}, attr_c{0};
   launch_step(lz_start_kernel<T, CL>, attr, attr_c, g, 0, s, theta, v0, cur, n, st, r.part, seed, seed_host, tol, kmax,
-              g.chunk);
+              g.chunk, test_unsignalled_wait("start") ? 1 : 0);
 }
 template <typename T, bool CL>
 void ritz_launch(const StepGrid& g, const T* V, ll n, T* out, LanczosDev* st, RedScratch& r, LanczosHost* host,
                  cudaStream_t s) {
   static std::atomic<unsigned long long> attr{0}, attr_c{0};
   launch_step(lz_ritz_norm_kernel<T, CL>, attr, attr_c, g, sizeof(T) * (size_t)g.chunk, s, V, n, out, st, r.part,
-              host, g.chunk);
+              host, g.chunk, test_unsignalled_wait("ritz") ? 1 : 0);
 }
 }  // namespace
 

@@ -133,15 +133,21 @@ struct LanczosResult {
   long long launches = 0, fixed = 0;  // kernels per loop body and around the loop (pending solves)
 };
 
+// throws where the finished solve (W.h_st) left no result
+template <typename T>
+void lanczos_check(LanczosWork<T>& W, cudaStream_t s) {
+  const LanczosHost& h = *W.h_st;
+  if (h.done && h.n_iter >= 1 && !h.gave_up) return;
+  // (a grid barrier that gave up leaves its counters behind)
+  DMRG2_CUDA(cudaMemsetAsync(W.st, 0, sizeof(LanczosDev), s));
+  throw std::runtime_error("Lanczos did not terminate");
+}
+
 // Adds what the finished solve reported (W.h_st) to res; s: its stream (idle up to the solve's end).
 template <typename T>
 void lanczos_collect(LanczosWork<T>& W, LanczosResult& res, cudaStream_t s) {
   const LanczosHost& h = *W.h_st;
-  if (!h.done || h.n_iter < 1) {
-    // (a grid barrier that gave up leaves its counters behind)
-    DMRG2_CUDA(cudaMemsetAsync(W.st, 0, sizeof(LanczosDev), s));
-    throw std::runtime_error("Lanczos did not terminate");
-  }
+  lanczos_check(W, s);
   launch_counter() += h.guard * res.launches + res.fixed;
   thread_launches() += h.guard * res.launches + res.fixed;
   res.matvecs += h.guard;
@@ -221,6 +227,7 @@ LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, d
     }
   }
   for (int rs = 0; rs <= max_restarts; ++rs) {
+    W.h_st->gave_up = 0;  // (the last solve on W has been waited for)
     if (G && G->ex) {
       // the solve reads the pinned seed before the host writes it again (the wait below)
       *W.h_seed = seed + 104729u * (unsigned)rs;
@@ -255,10 +262,7 @@ LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, d
     }
     lz_ritz(W.krylov, n, theta, W.st, W.red, W.h_st, s);
     DMRG2_CUDA(cudaStreamSynchronize(s));
-    if (!W.h_st->done || W.h_st->n_iter < 1) {
-      DMRG2_CUDA(cudaMemsetAsync(W.st, 0, sizeof(LanczosDev), s));
-      throw std::runtime_error("Lanczos did not terminate");
-    }
+    lanczos_check(W, s);
     const int used = std::min(issued, W.h_st->n_iter);
     for (int j = 0; timed && j < used; ++j) {
       float ms = 0.f;

@@ -53,3 +53,34 @@ def test_unsignalled_waits_time_out_with_numeric_status():
     assert np.abs(C - A @ B).max() <= 1e-5 * np.abs(A).max() * np.abs(B).max() * 300 ** 0.5
     U, S, Vh, _ = dmrg2.truncated_svd(A, 64, direction="R", method="jacobi")
     np.testing.assert_allclose(S[:64], np.linalg.svd(A, compute_uv=False)[:64], rtol=1e-12, atol=1e-12)
+
+
+LANCZOS_CHILD = r"""
+import numpy as np, dmrg2
+rng = np.random.default_rng(0)
+cL, cR = 64, 130
+def herm(n):
+    x = rng.standard_normal((n, n))
+    return ((x + x.T) / np.sqrt(n))[:, None, :]
+L, R, W, th = herm(cL), herm(cR), np.eye(2)[None, None], rng.standard_normal((cL, 2, 2, cR))
+for n in (2, 1):
+    try:
+        dmrg2.optimize_two_site(L, R, W, W, th, max_iter=6, tol=0.0, max_restarts=0)
+        print("returned")
+    except dmrg2.Dmrg2Error as e:
+        print("status", str(e).split("(status ")[1].split(")")[0], "terminate" in str(e))
+A = rng.standard_normal((30, 20))
+print("gemm", np.allclose(dmrg2.gemm(A, A, "N", "T"), A @ A.T))
+"""
+
+
+@pytest.mark.parametrize("kernel", ["start", "step", "ritz"])
+def test_a_lanczos_block_that_gives_up_ends_the_solve(kernel):
+    """Each cooperative Lanczos kernel in turn, with the last block's wait unsignalled: one block goes on
+    with sums that lack the others', the rest of the grid meets as usual, and the solve must not
+    return a vector that is scaled differently in that block's slice."""
+    env = dict(os.environ, DMRG2_TEST_UNSIGNALLED_WAITS=kernel,
+               PYTHONPATH=os.pathsep.join([str(REPO / "dmrg-implementations_b200"), str(REPO)]))
+    r = subprocess.run([sys.executable, "-c", LANCZOS_CHILD], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.strip().splitlines() == [f"status {dmrg2.ERR_NUMERIC} True"] * 2 + ["gemm True"], r.stdout
