@@ -735,9 +735,12 @@ class Engine final : public EngineBase {
     const int cL = dims_[i], cM = dims_[i + 1], cR = dims_[i + 2];
     const ll n = (ll)cL * d_ * d_ * cR;
     theta_form(mps_[i], mps_[i + 1], ln().theta, cL, cM, cR, d_, ln().st);
-    // the split is enqueued behind the solve; its own wait covers both
+    // the split is enqueued behind the solve; its own wait covers both, and the sites are written only
+    // where the solve left a result
     LanczosResult r = lanczos(i, n, true);
-    svd_split(i, dir, chi, ss);
+    svd_split(i, dir, chi, ss, [&] {
+      if (r.pending) lanczos_collect(ln().lw, r, ln().st);
+    });
     const double e = lanczos_stats(i, cL, cR, r, ss);
     if (dir == 'R')
       env_left(lenv_[i], mps_[i], wml_[i], lenv_[i + 1], ln().X, ln().Y, dims_[i], dims_[i + 1], d_, Dl_[i],
@@ -949,7 +952,8 @@ class Engine final : public EngineBase {
     return te <= te_ref_[i] * (1.0 + WARM_SHORT_SLACK) + 64.0 * 2.220446049250313e-16 * fro2;
   }
 
-  void svd_split(int i, char dir, int chi, SweepStats& ss) {
+  // solved: throws, once the stream has run the solve, where it left no result
+  void svd_split(int i, char dir, int chi, SweepStats& ss, const std::function<void()>& solved) {
     const int cL = dims_[i], cR = dims_[i + 2];
     const ll m = (ll)cL * d_, nc = (ll)d_ * cR;
     DMRG2_CUDA(cudaEventRecord(ln().ev_c, ln().st));
@@ -962,10 +966,10 @@ class Engine final : public EngineBase {
           bool done;
           if constexpr (ST<T>::cplx)
             done = wst_split_c(ln().wstc, ln().red, ln().theta, (int)m, (int)nc, dir, k, warm, mps_[i], mps_[i + 1], te,
-                               ln().st, mode, ln().ev_d);
+                               ln().st, mode, ln().ev_d, ln().lw.st, solved);
           else
             done = wst_split(ln().wst, ln().red, ln().theta, (int)m, (int)nc, dir, k, warm, mps_[i], mps_[i + 1], te,
-                             ln().st, mode, cfg_.graphs, ln().ev_d);
+                             ln().st, mode, cfg_.graphs, ln().ev_d, ln().lw.st, solved);
           return done && warm_split_keeps_rank(k, chi, m, nc, te, warm_fro2());
         };
         bool ok = false, short_kept = false;
@@ -1012,7 +1016,7 @@ class Engine final : public EngineBase {
       bool ok = false;
       try {
         ok = rsvd_split(ln().rsvd, ln().ew, ln().red, ln().theta, (int)m, (int)nc, dir, chi, cfg_.cutoff, seed, mps_[i],
-                        mps_[i + 1], o, ln().st);
+                        mps_[i + 1], o, ln().st, solved);
       } catch (const NumericError&) {
         ok = false;  // the small split's eigenvectors: the exact split below decides
       }
@@ -1034,9 +1038,13 @@ class Engine final : public EngineBase {
     }
     SvdOut o;
     bool jacobi = (cfg_.svd_method == 1);
-    if (!jacobi) {
+    if (jacobi) {
+      DMRG2_CUDA(cudaStreamSynchronize(ln().st));
+      solved();
+    } else {
       try {
-        o = eig_split(ln().ew, ln().theta, (int)m, (int)nc, dir, chi, cfg_.cutoff, false, mps_[i], mps_[i + 1], ln().st);
+        o = eig_split(ln().ew, ln().theta, (int)m, (int)nc, dir, chi, cfg_.cutoff, false, mps_[i], mps_[i + 1], ln().st,
+                      0, nullptr, solved);
         DMRG2_CUDA(cudaEventRecord(ln().ev_d, ln().st));
         DMRG2_CUDA(cudaEventSynchronize(ln().ev_d));
       } catch (const NumericError&) {

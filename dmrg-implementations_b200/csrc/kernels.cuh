@@ -77,6 +77,10 @@ void lz_step_dev(T* V, ll n, T* w, T* cur, LanczosDev* st, RedScratch& r, int km
 template <typename T>
 void lz_ritz(const T* V, ll n, T* out, LanczosDev* st, RedScratch& r, LanczosHost* host, cudaStream_t s);
 
+// Test hook: this many deferred solves from now (0: none) one is made to fail, as by a barrier that gave up.
+std::atomic<int>& lz_fail_countdown();
+void lz_fail(LanczosDev* st, LanczosHost* host, cudaStream_t s);
+
 // ---------------------------------------------------------------- SVD
 struct JacobiCtl {
   unsigned bar_count;
@@ -165,6 +169,11 @@ void split_begin(int* status, SvdOut* out, int k, cudaStream_t s);
 template <typename T>
 void split_finish(const T* theta, ll nt, const T* kept, ll nk, const int* status, const SvdOut* out, SplitHost* host,
                   RedScratch& r, cudaStream_t s);
+
+// left <- l (nl elements) and right <- r (nr), unless the solve whose vector was split (solve, when given)
+// left no result: the sites then stay as they are
+template <typename T>
+void split_commit(const T* l, T* left, ll nl, const T* r, T* right, ll nr, const LanczosDev* solve, cudaStream_t s);
 
 // ---------------------------------------------------------------- misc
 template <typename T>

@@ -710,8 +710,10 @@ __global__ void __launch_bounds__(LS_THREADS, 1)
   }
   ww = warp_sum(ww);
   if ((tid & 31) == 0) wsum[tid >> 5] = ww;
-  if (!exchange_sums<CL>(wsum, 1, 1, part, &st->bar[4], xch, &tot, unsignalled) && tid == 0)
+  if (!exchange_sums<CL>(wsum, 1, 1, part, &st->bar[4], xch, &tot, unsignalled) && tid == 0) {
+    *((volatile int*)&st->gave_up) = 1;
     *((volatile int*)&host->gave_up) = 1;
+  }
   const double inv = tot > 0.0 ? 1.0 / sqrt(tot) : 0.0;
   for (int x = tid; x < len; x += LS_THREADS) out[x0 + x] = ST<T>::scale(inv, ws[x]);
   if (blockIdx.x == 0 && tid == 0) st->nrm2 = tot;
@@ -1144,6 +1146,38 @@ void split_finish(const T* theta, ll nt, const T* kept, ll nk, const int* status
 }
 
 template <typename T>
+__global__ void __launch_bounds__(256)
+    split_commit_kernel(const T* __restrict__ l, T* __restrict__ left, ll nl, const T* __restrict__ r,
+                        T* __restrict__ right, ll nr, const LanczosDev* solve) {
+  if (solve && (solve->gave_up || !solve->done || solve->n_iter < 1)) return;
+  const ll step = (ll)gridDim.x * blockDim.x, t0 = (ll)blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll 4
+  for (ll i = t0; i < nl; i += step) left[i] = l[i];
+#pragma unroll 4
+  for (ll i = t0; i < nr; i += step) right[i] = r[i];
+}
+
+template <typename T>
+void split_commit(const T* l, T* left, ll nl, const T* r, T* right, ll nr, const LanczosDev* solve, cudaStream_t s) {
+  const int g = (int)std::min<ll>(4 * STEP_BLOCKS, std::max<ll>(1, (std::max(nl, nr) + 511) / 512));
+  split_commit_kernel<T><<<g, 256, 0, s>>>(l, left, nl, r, right, nr, solve);
+  DMRG2_CHECK_LAUNCH();
+}
+
+std::atomic<int>& lz_fail_countdown() {
+  static std::atomic<int> n{0};
+  return n;
+}
+__global__ void lz_fail_kernel(LanczosDev* st, LanczosHost* host) {
+  st->gave_up = 1;
+  *((volatile int*)&host->gave_up) = 1;
+}
+void lz_fail(LanczosDev* st, LanczosHost* host, cudaStream_t s) {
+  lz_fail_kernel<<<1, 1, 0, s>>>(st, host);
+  DMRG2_CHECK_LAUNCH();
+}
+
+template <typename T>
 void scale_inplace(T* x, ll n, const double* nrm2_dev, cudaStream_t s) {
   scale_by_inv_sqrt_kernel<T><<<grid_for(n), VEC_THREADS, 0, s>>>(x, n, nrm2_dev);
   DMRG2_CHECK_LAUNCH();
@@ -1158,6 +1192,7 @@ void scale_inplace(T* x, ll n, const double* nrm2_dev, cudaStream_t s) {
   template void lz_ritz<T>(const T*, ll, T*, LanczosDev*, RedScratch&, LanczosHost*, cudaStream_t); \
   template void split_finish<T>(const T*, ll, const T*, ll, const int*, const SvdOut*, SplitHost*, \
                                 RedScratch&, cudaStream_t);                                       \
+  template void split_commit<T>(const T*, T*, ll, const T*, T*, ll, const LanczosDev*, cudaStream_t); \
   template void norm2<T>(const T*, ll, double*, RedScratch&, cudaStream_t);                       \
   template void scale_inplace<T>(T*, ll, const double*, cudaStream_t);
 INST(double)

@@ -70,6 +70,7 @@ struct LanczosWork {
   RedScratch red;
   int* h_flags = nullptr;
   LanczosHost* h_st = nullptr;  // the solve's report (pinned, written by its last kernel)
+  bool pending = false;         // a deferred solve has not been collected
   unsigned* h_seed = nullptr;   // the device-looped solve's seed (pinned, read by its first kernel)
   std::vector<cudaEvent_t> ev_poll, ev_mv;
   std::vector<void*> owned;
@@ -147,6 +148,7 @@ void lanczos_check(LanczosWork<T>& W, cudaStream_t s) {
 template <typename T>
 void lanczos_collect(LanczosWork<T>& W, LanczosResult& res, cudaStream_t s) {
   const LanczosHost& h = *W.h_st;
+  W.pending = false;
   lanczos_check(W, s);
   launch_counter() += h.guard * res.launches + res.fixed;
   thread_launches() += h.guard * res.launches + res.fixed;
@@ -197,13 +199,19 @@ void lz_build_graph(LanczosWork<T>& W, GraphEntry& G, T* theta, ll n, int kmax, 
 // vector on exit. With a key: the device-looped form, cached in W.graphs (the key must
 // identify everything the matvec reads and writes besides in and out). With defer, a
 // device-looped solve without restarts is only enqueued (res.pending): the caller enqueues what
-// follows, waits for the stream and calls lanczos_collect, one host round trip less.
+// follows, waits for the stream and calls lanczos_collect, one host round trip less. What follows must
+// leave nothing behind that a failed solve may not: see split_commit.
 template <typename T>
 LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, double tol,
                             int max_restarts, unsigned seed,
                             const std::function<void(const T*, T*, const int*)>& matvec,
                             cudaStream_t s, const LzKey* key = nullptr, bool defer = false) {
   LanczosResult res;
+  if (W.pending) {  // an error kept the caller from collecting the last solve: leave nothing of it
+    W.pending = false;
+    DMRG2_CUDA(cudaStreamSynchronize(s));
+    DMRG2_CUDA(cudaMemsetAsync(W.st, 0, sizeof(LanczosDev), s));
+  }
   const bool timed = !W.ev_mv.empty();
   const int kmax = (int)std::min<ll>(std::min(krylov_max, W.kcap), n);
   if (kmax < 1) throw std::runtime_error("lanczos: empty problem");
@@ -236,7 +244,9 @@ LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, d
       res.launches = G->launches;
       res.fixed = G->fixed;
       if (defer && max_restarts == 0) {
-        res.pending = true;
+        int left = lz_fail_countdown().load();
+        if (left > 0 && --lz_fail_countdown() == 0) lz_fail(W.st, W.h_st, s);
+        W.pending = res.pending = true;
         return res;
       }
       DMRG2_CUDA(cudaStreamSynchronize(s));

@@ -116,11 +116,11 @@ inline bool rsvd_applies(const RsvdWork<T>& W, int m, int nt, char dir, int chi)
 // cutoff: writes left (m x k) and right (k x nt) as eig_split does and returns its
 // summary with trunc_err covering the whole discarded weight; returns false (nothing
 // written) when the CholeskyQR passes could not orthonormalise the sketch, and the
-// caller then runs the exact split. The host waits twice.
+// caller then runs the exact split. The host waits twice. solved: see eig_split.
 template <typename T>
 inline bool rsvd_split(RsvdWork<T>& W, EigWork<T>& ew, RedScratch& red, const T* theta, int m, int nt, char dir,
                        int chi, double cutoff, unsigned long long seed, T* left, T* right, SvdOut& o,
-                       cudaStream_t s) {
+                       cudaStream_t s, const std::function<void()>& solved = nullptr) {
   constexpr int C = RsvdWork<T>::C;
   const bool R = (dir == 'R');
   const int full_k = std::min(m, nt), k = std::min(chi, full_k);
@@ -175,6 +175,7 @@ inline bool rsvd_split(RsvdWork<T>& W, EigWork<T>& ew, RedScratch& red, const T*
   }
   DMRG2_CUDA(cudaMemcpyAsync(W.h_status, W.status, sizeof(int), cudaMemcpyDeviceToHost, s));
   DMRG2_CUDA(cudaStreamSynchronize(s));
+  if (solved) solved();
   if (*W.h_status) return false;
   // B = Q^H theta ('R', r x nt) or theta Q ('L', m x r)
   {

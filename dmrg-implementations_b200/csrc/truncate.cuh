@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <stdexcept>
 #include <vector>
 
@@ -92,11 +93,13 @@ struct EigWork {
 // k = min(chi, rank, #{sigma > cutoff}) (relative: sigma > cutoff * sigma_max),
 // singular values below the density-matrix noise floor count as zero.
 // The host waits once (to learn k). Returns the device-side summary.
-// K_compute (>= chi) eigenpairs are computed; lam_out (optional, host) receives them.
+// K_compute (>= chi) eigenpairs are computed; lam_out (optional, host) receives them. solved (optional)
+// is called after that wait, before left and right are written: it throws where theta is not
+// the vector of a finished solve.
 template <typename T>
 SvdOut eig_split(EigWork<T>& W, const T* theta, int m, int nt, char dir, int chi, double cutoff,
                  bool relative, T* left, T* right, cudaStream_t s, int K_compute = 0,
-                 double* lam_out = nullptr) {
+                 double* lam_out = nullptr, const std::function<void()>& solved = nullptr) {
   const bool R = (dir == 'R');
   const int n = R ? m : nt;
   if (n > W.nmax) throw std::runtime_error("eig_split: workspace too small");
@@ -159,6 +162,7 @@ SvdOut eig_split(EigWork<T>& W, const T* theta, int m, int nt, char dir, int chi
   apply_q<T>(W.G, n, W.tau, n, W.Z, K, W.out, W.Zg, W.Tb, s, true);
   DMRG2_CUDA(cudaMemcpyAsync(W.h_out, W.out, sizeof(SvdOut), cudaMemcpyDeviceToHost, s));
   DMRG2_CUDA(cudaStreamSynchronize(s));
+  if (solved) solved();
   SvdOut o = *W.h_out;
   if (!std::isfinite(o.fro2))
     throw std::runtime_error("eigensolver: non-finite density matrix or tridiagonal reduction");
@@ -263,7 +267,7 @@ struct WstWork {
   unsigned* counter = nullptr;
   int* status = nullptr;
   SvdOut* out = nullptr;    // k and the Newton-Schulz convergence flag
-  // with graphs: the warm factor in, and both factors out, pass through these fixed slots
+  // both factors out and, with graphs, the warm factor in pass through these fixed slots
   // (qmax x kmax each), so one graph serves every bond of a shape
   double *Win = nullptr, *Lout = nullptr, *Rout = nullptr;
   SplitHost* h_rep = nullptr;  // pinned: the split's report
@@ -340,21 +344,23 @@ inline bool wst_debug() {
 //   WST_SHORT  one, from the warm factor: left = tri(theta B^T) ('R'), right^T =
 //              tri(theta^T A) ('L'), each polished and the other factor projected;
 //   WST_RESUME the two after a WST_SHORT call on the same theta, starting from the
-//              basis that call left (in `left` for 'R', in W.Ya for 'L'); together they
-//              are WST_FULL.
+//              basis that call left in the workspace; together they are WST_FULL.
 enum WstMode { WST_FULL = 0, WST_SHORT = 1, WST_RESUME = 2 };
 
 // Warm-started split of theta (m x nt) at kept rank k; `warm` is B (k x nt) for 'R',
 // A (m x k) for 'L'. Writes left (m x k) and right (k x nt) and returns true, or returns
 // false (left / right undefined) when the warm start was not good enough. The host
-// waits once; ev_end, when given, is recorded after the split's kernels. With graphs on (and a stream other than the legacy default one), the work
-// between the status reset and that wait is one cached graph per (direction, mode,
-// shapes): the warm factor is copied into W.Win and the factors come out of W.Lout and
-// W.Rout, so the graph's buffers do not depend on the bond; a key's second call launches
-// the kernels and then captures them, later calls replay the capture.
+// waits once; ev_end, when given, is recorded after the split's kernels. The factors come out of
+// W.Lout and W.Rout and are copied from there (split_commit: not when `solve` left no result;
+// solved, when given, is called after the wait). With graphs on (and a stream other than the legacy
+// default one), the work between the status reset and those copies is one cached graph per
+// (direction, mode, shapes): the warm factor is copied into W.Win, so the graph's buffers do not
+// depend on the bond; a key's second call launches the kernels and then captures them, later calls
+// replay the capture.
 inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, int nt, char dir, int k,
                       const double* warm, double* left, double* right, double& trunc_err, cudaStream_t s,
-                      WstMode mode = WST_FULL, bool allow_graph = true, cudaEvent_t ev_end = nullptr) {
+                      WstMode mode = WST_FULL, bool allow_graph = true, cudaEvent_t ev_end = nullptr,
+                      const LanczosDev* solve = nullptr, const std::function<void()>& solved = nullptr) {
   if (k > W.kmax || m > W.qmax || nt > W.qmax) throw std::runtime_error("wst_split: workspace too small");
   if (std::max(m, nt) > 32 * COLNORM_MAX_CHUNKS) return false;  // longer columns take the exact split
   split_begin(W.status, W.out, k, s);
@@ -409,9 +415,9 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
                                  cudaMemcpyDeviceToDevice, s));
       warm = W.Win;
     }
-    left = W.Lout;
-    right = W.Rout;
   }
+  left = W.Lout;
+  right = W.Rout;
   auto body = [&]() {
   const double* kept = nullptr;
   ll nkept = 0;
@@ -475,13 +481,13 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
         graphs_disable(e.what());
       }
     }
-    DMRG2_CUDA(cudaMemcpyAsync(left_out, W.Lout, sizeof(double) * (size_t)m * k, cudaMemcpyDeviceToDevice, s));
-    DMRG2_CUDA(cudaMemcpyAsync(right_out, W.Rout, sizeof(double) * (size_t)k * nt, cudaMemcpyDeviceToDevice, s));
   } else {
     body();
   }
+  split_commit(W.Lout, left_out, (ll)m * k, W.Rout, right_out, (ll)k * nt, solve, s);
   if (ev_end) DMRG2_CUDA(cudaEventRecord(ev_end, s));  // the split's device work ends here
   DMRG2_CUDA(cudaStreamSynchronize(s));
+  if (solved) solved();
   const SplitHost& rep = *W.h_rep;
   if (rep.failed || !std::isfinite(rep.theta2) || !std::isfinite(rep.kept2)) return false;
   trunc_err = std::max(rep.theta2 - rep.kept2, 0.0);

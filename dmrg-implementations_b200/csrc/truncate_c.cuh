@@ -86,10 +86,12 @@ inline size_t wstc_bytes(ll qmax, ll kmax) {
 // Warm-started split of complex theta (m x nt) at kept rank k; `warm` is B (k x nt) for
 // 'R', A (m x k) for 'L'. Writes left (m x k) and right (k x nt) and returns true, or
 // returns false (left / right undefined) when the warm start was not good enough. The
-// host waits once; ev_end, when given, is recorded after the split's kernels.
+// host waits once; ev_end, when given, is recorded after the split's kernels. The factors are formed in
+// the workspace and copied from there; solve and solved: see wst_split.
 inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, int nt, char dir, int k,
                         const zc* warm, zc* left, zc* right, double& trunc_err, cudaStream_t s,
-                        WstMode mode = WST_FULL, cudaEvent_t ev_end = nullptr) {
+                        WstMode mode = WST_FULL, cudaEvent_t ev_end = nullptr, const LanczosDev* solve = nullptr,
+                        const std::function<void()>& solved = nullptr) {
   if (k > W.kmax || m > W.qmax || nt > W.qmax) throw std::runtime_error("wst_split_c: workspace too small");
   if (2 * std::max(m, nt) > 32 * COLNORM_MAX_CHUNKS) return false;  // longer columns take the exact split
   split_begin(W.status, W.out, k, s);
@@ -139,7 +141,7 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
     mulr(false, W.Z1, k2, (int)r2, k2, k2, W.S, k2, W.Z2, k2, -0.5, 1.5, &W.out->ns_done, W.Z1);
     extract_pairs(W.Z2, rows, k, dst, s);
   };
-  const zc* kept = nullptr;
+  const zc *kept = nullptr, *l = nullptr, *r = nullptr;  // the projected factor; both factors
   ll nkept = 0;
   if (dir == 'R') {
     if (mode != WST_RESUME) {
@@ -147,7 +149,7 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
       transpose<zc>(W.Yb, W.Ya, (ll)k, (ll)m, s);                          // theta B^H (m x k)
       tri(W.Ya, m, W.Yb);                                                  // U1
     } else {
-      DMRG2_CUDA(cudaMemcpyAsync(W.Yb, left, sizeof(zc) * (size_t)m * k, cudaMemcpyDeviceToDevice, s));
+      DMRG2_CUDA(cudaMemcpyAsync(W.Yb, W.Ya, sizeof(zc) * (size_t)m * k, cudaMemcpyDeviceToDevice, s));  // U1
     }
     if (mode != WST_SHORT) {
       mulz(true, true, theta, nt, nt, k, m, W.Yb, k, false, W.Ya, k);  // theta^H U1
@@ -155,9 +157,10 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
       mulz(false, false, theta, nt, m, k, nt, W.Yb, k, false, W.Ya, k);  // theta V1
       tri(W.Ya, m, W.Yb);                                                // U2
     }
-    polish(W.Yb, m, left);
-    mulz(true, true, left, k, k, nt, m, theta, nt, false, right, nt);  // right = U^H theta
-    kept = right;
+    polish(W.Yb, m, W.Ya);                                             // U in Ya
+    mulz(true, true, W.Ya, k, k, nt, m, theta, nt, false, W.Yb, nt);   // right = U^H theta
+    l = W.Ya;
+    r = kept = W.Yb;
     nkept = (ll)k * nt;
   } else {
     if (mode != WST_RESUME) {
@@ -173,14 +176,17 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
       tri(W.Ya, nt, W.Yb);                                               // V2
     }
     polish(W.Yb, nt, W.Ya);                                              // V in Ya
-    transpose_conj<zc>(W.Ya, k, nt, k, right, s);                        // right = V^H
-    mulz(false, false, theta, nt, m, k, nt, W.Ya, k, false, left, k);    // left = theta V
-    kept = left;
+    transpose_conj<zc>(W.Ya, k, nt, k, (zc*)W.Z1, s);                    // right = V^H
+    mulz(false, false, theta, nt, m, k, nt, W.Ya, k, false, W.Yb, k);    // left = theta V
+    r = (const zc*)W.Z1;
+    l = kept = W.Yb;
     nkept = (ll)m * k;
   }
   split_finish(theta, (ll)m * nt, kept, nkept, W.status, W.out, W.h_rep, red, s);
+  split_commit(l, left, (ll)m * k, r, right, (ll)k * nt, solve, s);
   if (ev_end) DMRG2_CUDA(cudaEventRecord(ev_end, s));
   DMRG2_CUDA(cudaStreamSynchronize(s));
+  if (solved) solved();
   const SplitHost& rep = *W.h_rep;
   if (rep.failed || !std::isfinite(rep.theta2) || !std::isfinite(rep.kept2)) return false;
   trunc_err = std::max(rep.theta2 - rep.kept2, 0.0);

@@ -43,4 +43,7 @@ int probe_ns_check(const double* S, int K, int k, double tol, int* flags) {
   });
 }
 
+// the n-th deferred Lanczos solve from now fails
+void probe_fail_solve(int n) { lz_fail_countdown() = n; }
+
 }  // extern "C"
