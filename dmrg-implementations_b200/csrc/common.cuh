@@ -39,6 +39,10 @@ template <> struct ST<double> {
   __host__ __device__ static double abs2(double a) { return a * a; }
   __host__ __device__ static bool finite(double a) { return a - a == 0.0; }
   __host__ __device__ static bool nonzero(double a) { return a != 0.0; }
+#ifdef __CUDACC__
+  // the top half without its sign: at least 0x7ff00000 for an infinity or a NaN only
+  __device__ static unsigned exponent_bits(double a) { return (unsigned)__double2hiint(a) & 0x7fffffffu; }
+#endif
   __host__ __device__ static double make(double r, double) { return r; }
   __host__ __device__ static double mul(double a, double b) { return a * b; }
   __host__ __device__ static double add(double a, double b) { return a + b; }
@@ -56,6 +60,12 @@ template <> struct ST<zc> {
   __host__ __device__ static double abs2(zc a) { return a.re * a.re + a.im * a.im; }
   __host__ __device__ static bool finite(zc a) { return a.re - a.re == 0.0 && a.im - a.im == 0.0; }
   __host__ __device__ static bool nonzero(zc a) { return a.re != 0.0 || a.im != 0.0; }
+#ifdef __CUDACC__
+  __device__ static unsigned exponent_bits(zc a) {
+    const unsigned r = ST<double>::exponent_bits(a.re), i = ST<double>::exponent_bits(a.im);
+    return r > i ? r : i;
+  }
+#endif
   __host__ __device__ static zc make(double r, double i) { return mkz(r, i); }
   __host__ __device__ static zc mul(zc a, zc b) { return a * b; }
   __host__ __device__ static zc add(zc a, zc b) { return a + b; }

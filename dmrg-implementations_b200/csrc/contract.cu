@@ -39,60 +39,21 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// The same mixing with W in its nonzero form (row starts, ascending columns, values; Kin,
-// Kout <= 32 and at most MIX_SPARSE_NNZ nonzeros): each output sums only its row's
-// nonzeros, in the order of the dense loop above (whose other terms are exact zeros). A
-// thread first loads its Kin inputs together (a static loop, as the dense kernel does)
-// into its own column of shared memory, so the sums read shared memory, not L2.
-constexpr int MIX_SPARSE_NNZ = 512;
-constexpr int MIX_SPARSE_NT = 64;
-template <typename T>
-__global__ void __launch_bounds__(MIX_SPARSE_NT)
-    mpo_mix_sparse_kernel(const T* __restrict__ X, const T* __restrict__ val, const int* __restrict__ rowp,
-                          T* __restrict__ Y, int Kin, int Kout, int cR, ll sX, ll sY, const int* skip) {
-  pdl_wait();
-  if (skip && *((volatile const int*)skip)) return;
-  constexpr int KM = 32, NT = MIX_SPARSE_NT;
-  __shared__ int rp[KM + 1];
-  __shared__ int cs[MIX_SPARSE_NNZ];
-  __shared__ T vs[MIX_SPARSE_NNZ];
-  __shared__ T xs[KM * NT];  // xs[k][thread]
-  const int tid = threadIdx.x;
-  for (int i = tid; i <= Kout; i += NT) rp[i] = rowp[i];
-  __syncthreads();
-  const int nnz = min(rp[Kout], MIX_SPARSE_NNZ);
-  const int* col = rowp + Kout + 1;
-  for (int i = tid; i < nnz; i += NT) {
-    cs[i] = col[i];
-    vs[i] = val[i];
-  }
-  __syncthreads();
-  const int e = blockIdx.x * NT + tid;
-  if (e >= cR) return;
-  const ll a = blockIdx.y;
-  const T* xa = X + a * sX + e;
-  T* ya = Y + a * sY + e;
-#pragma unroll
-  for (int k = 0; k < KM; ++k)
-    if (k < Kin) xs[k * NT + tid] = xa[(ll)k * cR];
-  for (int o = 0; o < Kout; ++o) {
-    T acc = ST<T>::zero();
-    const int j1 = min(rp[o + 1], nnz);
-    for (int j = rp[o]; j < j1; ++j) acc = acc + ST<T>::mul(vs[j], xs[cs[j] * NT + tid]);
-    ya[(ll)o * cR] = acc;
-  }
-}
-
-// The same mixing for up to MIX_WIDE_K inputs (complex chains with d^2 D = 100, say): a CTA takes
-// one a and 32 columns e, stages all Kin inputs of them in shared memory, and its warps walk the
-// rows of W (nonzeros read through L1, the same for every lane). Bandwidth-bound on L2: X read
-// once, Y written once, and no work for W's zeros, which as a dense product on the tensor
-// cores cost 28% of a Josephson matvec's flops (187 of 10,000 entries are nonzero there).
+// The same mixing with W in its nonzero form (row starts, ascending columns, values), for up to
+// MIX_WIDE_K inputs: a CTA takes one a and 32 columns e, stages all Kin inputs of them in shared
+// memory, and its warps walk the rows of W; each output sums only its row's nonzeros, in the order
+// of the dense loop above. Bandwidth-bound on L2: X read once, Y written once, and no work for
+// W's zeros, which as a dense product on the tensor cores cost 28% of a Josephson matvec's flops
+// (187 of 10,000 entries are nonzero there). Real data, us at cL = cR = 96 / 180 / 256, dense above
+// / here: 20 x 20, 30 nonzeros (XXZ, D = 5) 5.3 / 6.9 / 8.7 and 3.4 / 4.9 / 7.3; 32 x 32, 48 nonzeros
+// (J1-J2, D = 8) 7.2 / 9.7 / 12.2 and 4.2 / 6.6 / 10.0; with 409 of 1024 entries nonzero (128 x 128)
+// they meet at 7.3, where the engine's rule (at most half) stops using it. A form with one thread
+// per column and its inputs in shared memory took 5.8 / 6.2 / 7.0 and 8.1 / 8.5 / 9.6.
 constexpr int MIX_WIDE_NT = 256;
 constexpr int MIX_WIDE_NNZ = 768;  // nonzeros staged in shared memory (more are read through L1)
 template <typename T>
 __global__ void __launch_bounds__(MIX_WIDE_NT)
-    mpo_mix_wide_kernel(const T* __restrict__ X, const T* __restrict__ val, const int* __restrict__ rowp,
+    mpo_mix_nonzero_kernel(const T* __restrict__ X, const T* __restrict__ val, const int* __restrict__ rowp,
                         T* __restrict__ Y, int Kin, int Kout, int cR, ll sX, ll sY, const int* skip) {
   pdl_wait();
   if (skip && *((volatile const int*)skip)) return;
@@ -107,11 +68,11 @@ __global__ void __launch_bounds__(MIX_WIDE_NT)
   const T* xa = X + blockIdx.y * sX + e;
   T* ya = Y + blockIdx.y * sY + e;
   const int* col = rowp + Kout + 1;
-  bool bad = false;
+  unsigned top = 0;  // largest exponent field among this thread's inputs
 #pragma unroll 8
   for (int k = warp; k < Kin; k += W) {
     const T x = in ? xa[(ll)k * cR] : ST<T>::zero();
-    bad |= !ST<T>::finite(x);
+    top = max(top, ST<T>::exponent_bits(x));
     xs[k * 32 + lane] = x;
   }
   for (int i = threadIdx.x; i <= Kout; i += MIX_WIDE_NT) rp[i] = rowp[i];
@@ -122,7 +83,7 @@ __global__ void __launch_bounds__(MIX_WIDE_NT)
     vs[i] = val[i];
   }
   // An infinity or a NaN among the inputs: zero entries count too, as in the dense product.
-  if (__syncthreads_or(bad)) {
+  if (__syncthreads_or(top >= 0x7ff00000u)) {
     for (int o = warp; o < Kout; o += W) {
       const int j1 = rp[o + 1];
       T acc = ST<T>::zero();
@@ -180,18 +141,12 @@ int wwt_sparse_block(std::vector<T>& w, int Kin, int Kout) {
 template <typename T>
 static void mix_rows(const T* X, const T* W, T* Y, int cL, int cR, int Kin, int Kout, const int* skip,
                      cudaStream_t s, const T* wsp = nullptr) {
-  if (wsp && Kin <= 32 && Kout <= 32 && 2 * Kin * Kout <= 2 * MIX_SPARSE_NNZ && cL <= 65535) {
-    // (the engine uses the nonzero form only where nnz <= Kin Kout / 2 <= MIX_SPARSE_NNZ)
-    const ll kk = (ll)Kin * Kout;
-    dim3 grid(ceil_div(cR, MIX_SPARSE_NT), cL);
-    launch_pdl(mpo_mix_sparse_kernel<T>, grid, MIX_SPARSE_NT, 0, s, X, wsp, (const int*)(wsp + kk), Y, Kin, Kout, cR,
-               (ll)Kin * cR, (ll)Kout * cR, skip);
-  } else if (wsp && Kin <= MIX_WIDE_K && Kout <= MIX_WIDE_K && cL <= 65535) {
+  if (wsp && Kin <= MIX_WIDE_K && Kout <= MIX_WIDE_K && cL <= 65535) {
     const ll kk = (ll)Kin * Kout;
     static std::atomic<unsigned long long> attr{0};
-    set_smem_attr_once(attr, (const void*)mpo_mix_wide_kernel<T>, (int)(sizeof(T) * MIX_WIDE_K * 32));
+    set_smem_attr_once(attr, (const void*)mpo_mix_nonzero_kernel<T>, (int)(sizeof(T) * MIX_WIDE_K * 32));
     dim3 grid(ceil_div(cR, 32), cL);
-    launch_pdl(mpo_mix_wide_kernel<T>, grid, MIX_WIDE_NT, sizeof(T) * (size_t)Kin * 32, s, X, wsp,
+    launch_pdl(mpo_mix_nonzero_kernel<T>, grid, MIX_WIDE_NT, sizeof(T) * (size_t)Kin * 32, s, X, wsp,
                (const int*)(wsp + kk), Y, Kin, Kout, cR, (ll)Kin * cR, (ll)Kout * cR, skip);
   } else if (Kin <= 32 && Kout <= 32 && cL <= 65535) {
     dim3 grid(ceil_div(cR, 128), cL);

@@ -156,8 +156,8 @@ class Engine final : public EngineBase {
       build_wmix_right(hW_[i].data(), Dl[i], Dr[i], d_, hmr[i]);
     }
     for (int i = 0; i + 1 < L_; ++i) build_wwt(hW_[i].data(), hW_[i + 1].data(), Dl[i], Dr[i], Dr[i + 1], d_, hww[i]);
-    // each bond's fused MPO also in its nonzero form; mixing steps of more than 32 inputs use it
-    // where at most half the entries are nonzero (DMRG2_MIX_DENSE=1: the dense product)
+    // each bond's fused MPO also in its nonzero form; the mixing step uses it up to MIX_WIDE_K inputs
+    // where at most half the entries are nonzero (DMRG2_MIX_DENSE=1: always the dense form)
     static const bool mix_dense = [] {
       const char* e = std::getenv("DMRG2_MIX_DENSE");
       return e && e[0] == '1';

@@ -224,7 +224,7 @@ void heff_noalloc(int cL, int cR, int d, int Dl, int Dm, int Dr, const T* L, con
   // returns at once cost about 6 us, the mixing then its traffic; the batched GEMM on the dense
   // W runs at about 25 TFLOP/s of its padded size. Josephson, d = 5 (us per matvec, nonzeros /
   // dense): 64 x 64 49 / 46, 96 x 96 91 / 107, 128 x 128 155 / 181. At most 32 inputs the
-  // dense kernel is as fast.
+  // list costs more than it saves (32 x 32 at 171 x 187: mixing 9.7 us dense, 6.3 over the nonzeros).
   const int Kin = (int)(Dl * dd), Kout = (int)(dd * Dr);
   const size_t sp_b = round256((size_t)wwt_block_elems(Kin, Kout, sizeof(T)) * sizeof(T)) + 256;
   const double dense_us = 2e6 * (ST<T>::cplx ? 4.0 : 1.0) * cL * (double)cR * (ceil_div(Kout, 32) * 32.0) * Kin / 25e12;

@@ -1,5 +1,6 @@
 // Entry points on host arrays for internal pieces that no call of the public interface reaches at
 // the values a test needs. Compiled by internal.py and linked against the engine's library.
+#include "contract.cuh"
 #include "kernels.cuh"
 
 using namespace dmrg2;
@@ -16,6 +17,20 @@ struct Dev {  // a device copy of host data
   T* as() const { return (T*)p; }
   void to(void* h, size_t b) const { DMRG2_CUDA(cudaMemcpy(h, p, b, cudaMemcpyDeviceToHost)); }
 };
+template <typename T>
+void heff_nonzeros(int cL, int cR, int d, int Dl, int Dm, int Dr, const void* L, const void* R, const void* WL,
+                   const void* WR, const void* theta, void* out, int* nnz) {
+  const size_t b = sizeof(T), dd = (size_t)d * d, n = cL * dd * cR, Kin = Dl * dd, Kout = dd * Dr;
+  std::vector<T> w;
+  build_wwt((const T*)WL, (const T*)WR, Dl, Dm, Dr, d, w);
+  *nnz = wwt_sparse_block(w, (int)Kin, (int)Kout);
+  const size_t xs = (size_t)cL * cR * (Kin > Kout ? Kin : Kout);
+  Dev dL(L, b * cL * Dl * cL), dR(R, b * cR * Dr * cR), dW(w.data(), b * w.size()), in(theta, b * n), o(nullptr, b * n),
+      X(nullptr, b * xs), Y(nullptr, b * xs);
+  heff_apply(dL.as<T>(), dR.as<T>(), dW.as<T>(), in.as<T>(), o.as<T>(), X.as<T>(), Y.as<T>(), cL, cR, d, Dl, Dr, nullptr,
+             0, dW.as<T>() + Kin * Kout);
+  o.to(out, b * n);
+}
 template <typename F>
 int guarded(F f) {
   try {
@@ -45,5 +60,14 @@ int probe_ns_check(const double* S, int K, int k, double tol, int* flags) {
 
 // the n-th deferred Lanczos solve from now fails
 void probe_fail_solve(int n) { lz_fail_countdown() = n; }
+
+// H_eff with the MPO's nonzero form beside the dense one, as the engine calls it
+int probe_heff_nonzeros(int cplx, int cL, int cR, int d, int Dl, int Dm, int Dr, const void* L, const void* R,
+                        const void* WL, const void* WR, const void* theta, void* out, int* nnz) {
+  return guarded([&] {
+    if (cplx) heff_nonzeros<zc>(cL, cR, d, Dl, Dm, Dr, L, R, WL, WR, theta, out, nnz);
+    else heff_nonzeros<double>(cL, cR, d, Dl, Dm, Dr, L, R, WL, WR, theta, out, nnz);
+  });
+}
 
 }  // extern "C"

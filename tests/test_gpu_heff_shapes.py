@@ -12,6 +12,8 @@ import pytest
 
 import dmrg2
 
+from internal import load, ptr
+
 pytestmark = pytest.mark.gpu
 
 
@@ -113,3 +115,50 @@ def test_out_may_overlap_theta_or_the_left_environment(shape, cplx, where):
     assert rc == 0
     out = buf[at_out:at_out + n].cpu().numpy().reshape(ref.shape)
     assert np.abs(out - ref).max() <= 2.3e-16 * (cL + Dl * d * d + Dr * cR) * np.abs(ref).max()
+
+
+# (shape, complex, share of each W's entries kept): from 16 to 100 inputs, with the nonzeros staged in shared
+# memory and with more than fit there
+NONZERO = [((96, 90, 2, 5, 5, 5), False, 0.3), ((61, 67, 2, 5, 5, 5), True, 0.3), ((128, 130, 2, 4, 3, 5), False, 0.4),
+           ((70, 66, 5, 1, 4, 1), True, 0.5), ((100, 96, 2, 8, 8, 8), False, 0.2), ((64, 60, 2, 8, 6, 8), True, 0.2),
+           ((90, 70, 3, 4, 4, 4), False, 0.3), ((30, 40, 5, 4, 4, 4), True, 0.1), ((30, 40, 5, 4, 4, 4), False, 0.5)]
+
+
+def _nonzeros(shape, cplx, keep):
+    cL, cR, d, Dl, Dm, Dr = shape
+    rng = np.random.default_rng(14)
+
+    def rnd(*s):
+        x = rng.standard_normal(s)
+        return x + 1j * rng.standard_normal(s) if cplx else x
+
+    L, R, WL, WR, th = rnd(cL, Dl, cL), rnd(cR, Dr, cR), rnd(Dl, Dm, d, d), rnd(Dm, Dr, d, d), rnd(cL, d, d, cR)
+    WL *= rng.random(WL.shape) < keep
+    WR *= rng.random(WR.shape) < keep
+
+    def run(th):
+        out, nnz = np.empty_like(th), ctypes.c_int()
+        assert load().probe_heff_nonzeros(int(cplx), *shape, *[ptr(x) for x in (L, R, WL, WR, th, out)],
+                                          ctypes.byref(nnz)) == 0
+        return out, nnz.value
+
+    return run, th, _ref(L, R, WL, WR, th)
+
+
+@pytest.mark.parametrize("shape,cplx,keep", NONZERO)
+def test_nonzero_forms_of_the_tiled_path(shape, cplx, keep):
+    cL, cR, d, Dl, Dm, Dr = shape
+    run, th, ref = _nonzeros(shape, cplx, keep)
+    out, nnz = run(th)
+    entries = Dl * d ** 4 * Dr
+    assert 0 < nnz < entries and (nnz > 768 or keep < 0.5 or entries < 1000)
+    assert np.abs(out - ref).max() <= 2.3e-16 * (cL + Dl * d * d + Dr * cR) * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("shape,cplx,keep", NONZERO)
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_nonzero_forms_spread_what_is_not_finite(shape, cplx, keep, bad):
+    """An infinity times a zero of the MPO is NaN in every output that entry meets, as in the dense product."""
+    run, th, _ = _nonzeros(shape, cplx, keep)
+    th[shape[0] // 2, 0, shape[2] - 1, shape[1] - 1] = bad
+    assert not np.isfinite(run(th)[0]).any()
