@@ -847,16 +847,6 @@ __device__ inline double hash_unit(unsigned long long x) {
   x ^= x >> 31;
   return (double)(x >> 11) * (1.0 / 9007199254740992.0) * 2.0 - 1.0;
 }
-// 1/a from the hardware estimate and two Newton-Raphson steps y <- y + y (1 - a y); 0 and values
-// outside the estimate's range take the division
-__device__ __forceinline__ double invit_rcp(double a) {
-  const double m = fabs(a);
-  if (!(m > 1e-290 && m < 1e290)) return 1.0 / a;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  y = fma(y, fma(-a, y, 1.0), y);
-  return fma(y, fma(-a, y, 1.0), y);
-}
 
 __global__ void tridiag_invit_kernel(const double* __restrict__ dg, const double* __restrict__ eg,
                                      int n, int K, const double* __restrict__ lam,
@@ -910,11 +900,11 @@ __global__ void tridiag_invit_kernel(const double* __restrict__ dg, const double
       if (fmin(gap_up, gap_dn) >= 1e4 * shift) sft = (gap_up >= gap_dn) ? lam[first] + shift : lam[last] - shift;
     }
   }
-  // Bound by the dependent chain of one row (reciprocal, product, update): the row exchange is
-  // selects on one path (lanes that differ would run both branches, each with its division),
-  // the reciprocal the hardware's estimate and two Newton steps, and the next row's entries are
-  // loaded ahead of this row's stores. At n = K = 512: 216 us with branches, a division per row
-  // and loads behind the stores, 137 us now.
+  // Bound by the dependent chain of one row (division, product, update): the row exchange is
+  // selects on one path with one division (lanes that differ would run both branches, each with its
+  // own), and the next row's entries are loaded ahead of this row's stores. At n = K = 512: 216 us
+  // with branches and loads behind the stores, 127 us now (137 us with a hardware estimate and
+  // two Newton steps in place of the division).
   double c0 = d[0] - sft, c1 = e[0];
   {
     double s = e[0], dn = d[1 < n ? 1 : 0] - sft, en = e[1 < n ? 1 : 0];
@@ -923,7 +913,7 @@ __global__ void tridiag_invit_kernel(const double* __restrict__ dg, const double
       const double s1 = e[i1], dn1 = d[i2] - sft, en1 = e[i2];
       const bool sw = fabs(c0) < fabs(s);
       const double cc = (!sw && fabs(c0) < tiny) ? (c0 < 0 ? -tiny : tiny) : c0;
-      const double r = invit_rcp(sw ? s : cc);
+      const double r = 1.0 / (sw ? s : cc);
       const double m = (sw ? cc : s) * r;
       SX(0, i) = r;
       SX(1, i) = sw ? dn : c1;
@@ -939,7 +929,7 @@ __global__ void tridiag_invit_kernel(const double* __restrict__ dg, const double
     }
   }
   if (fabs(c0) < tiny) c0 = (c0 < 0 ? -tiny : tiny);
-  SX(0, n - 1) = invit_rcp(c0);
+  SX(0, n - 1) = 1.0 / c0;
   SX(1, n - 1) = 0.0;
   SX(2, n - 1) = 0.0;
   // the iterate lives in shared memory next to the factors; column j of Z is written at the end.
