@@ -267,8 +267,8 @@ struct WstWork {
   unsigned* counter = nullptr;
   int* status = nullptr;
   SvdOut* out = nullptr;    // k and the Newton-Schulz convergence flag
-  // both factors out and, with graphs, the warm factor in pass through these fixed slots
-  // (qmax x kmax each), so one graph serves every bond of a shape
+  // with graphs: the warm factor in, and both factors out, pass through these fixed slots
+  // (qmax x kmax each), so one graph serves every bond of a shape; behind a deferred solve the factors do
   double *Win = nullptr, *Lout = nullptr, *Rout = nullptr;
   SplitHost* h_rep = nullptr;  // pinned: the split's report
   SvdOut* h_out = nullptr;  // pinned (diagnostics)
@@ -344,19 +344,21 @@ inline bool wst_debug() {
 //   WST_SHORT  one, from the warm factor: left = tri(theta B^T) ('R'), right^T =
 //              tri(theta^T A) ('L'), each polished and the other factor projected;
 //   WST_RESUME the two after a WST_SHORT call on the same theta, starting from the
-//              basis that call left in the workspace; together they are WST_FULL.
+//              basis that call left (`left`, or its slot, for 'R', W.Ya for 'L'); together they
+//              are WST_FULL.
 enum WstMode { WST_FULL = 0, WST_SHORT = 1, WST_RESUME = 2 };
 
 // Warm-started split of theta (m x nt) at kept rank k; `warm` is B (k x nt) for 'R',
 // A (m x k) for 'L'. Writes left (m x k) and right (k x nt) and returns true, or returns
 // false (left / right undefined) when the warm start was not good enough. The host
-// waits once; ev_end, when given, is recorded after the split's kernels. The factors come out of
-// W.Lout and W.Rout and are copied from there (split_commit: not when `solve` left no result;
-// solved, when given, is called after the wait). With graphs on (and a stream other than the legacy
-// default one), the work between the status reset and those copies is one cached graph per
-// (direction, mode, shapes): the warm factor is copied into W.Win, so the graph's buffers do not
-// depend on the bond; a key's second call launches the kernels and then captures them, later calls
-// replay the capture.
+// waits once; ev_end, when given, is recorded after the split's kernels. Behind a deferred solve
+// (solve, its state) the factors come out of W.Lout and W.Rout and are copied from there
+// (split_commit: not where the solve left no result); solved, when given, is called after the
+// wait. With graphs on (and a stream other than the legacy default one), the work between the
+// status reset and those copies is one cached graph per (direction, mode, shapes): the warm factor
+// is copied into W.Win and the factors again come out of W.Lout and W.Rout, so the graph's
+// buffers do not depend on the bond; a key's second call launches the kernels and then captures
+// them, later calls replay the capture.
 inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, int nt, char dir, int k,
                       const double* warm, double* left, double* right, double& trunc_err, cudaStream_t s,
                       WstMode mode = WST_FULL, bool allow_graph = true, cudaEvent_t ev_end = nullptr,
@@ -416,8 +418,11 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
       warm = W.Win;
     }
   }
-  left = W.Lout;
-  right = W.Rout;
+  const bool slots = graph || solve;
+  if (slots) {
+    left = W.Lout;
+    right = W.Rout;
+  }
   auto body = [&]() {
   const double* kept = nullptr;
   ll nkept = 0;
@@ -484,7 +489,7 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
   } else {
     body();
   }
-  split_commit(W.Lout, left_out, (ll)m * k, W.Rout, right_out, (ll)k * nt, solve, s);
+  if (slots) split_commit(W.Lout, left_out, (ll)m * k, W.Rout, right_out, (ll)k * nt, solve, s);
   if (ev_end) DMRG2_CUDA(cudaEventRecord(ev_end, s));  // the split's device work ends here
   DMRG2_CUDA(cudaStreamSynchronize(s));
   if (solved) solved();

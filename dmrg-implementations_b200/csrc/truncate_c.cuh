@@ -86,8 +86,8 @@ inline size_t wstc_bytes(ll qmax, ll kmax) {
 // Warm-started split of complex theta (m x nt) at kept rank k; `warm` is B (k x nt) for
 // 'R', A (m x k) for 'L'. Writes left (m x k) and right (k x nt) and returns true, or
 // returns false (left / right undefined) when the warm start was not good enough. The
-// host waits once; ev_end, when given, is recorded after the split's kernels. The factors are formed in
-// the workspace and copied from there; solve and solved: see wst_split.
+// host waits once; ev_end, when given, is recorded after the split's kernels; solve and solved: see
+// wst_split (the slots are parts of the workspace that are free by then).
 inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, int nt, char dir, int k,
                         const zc* warm, zc* left, zc* right, double& trunc_err, cudaStream_t s,
                         WstMode mode = WST_FULL, cudaEvent_t ev_end = nullptr, const LanczosDev* solve = nullptr,
@@ -141,7 +141,12 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
     mulr(false, W.Z1, k2, (int)r2, k2, k2, W.S, k2, W.Z2, k2, -0.5, 1.5, &W.out->ns_done, W.Z1);
     extract_pairs(W.Z2, rows, k, dst, s);
   };
-  const zc *kept = nullptr, *l = nullptr, *r = nullptr;  // the projected factor; both factors
+  zc *const left_out = left, *const right_out = right;
+  if (solve) {
+    left = dir == 'R' ? W.Ya : W.Yb;
+    right = dir == 'R' ? W.Yb : (zc*)W.Z1;
+  }
+  const zc* kept = nullptr;
   ll nkept = 0;
   if (dir == 'R') {
     if (mode != WST_RESUME) {
@@ -149,7 +154,7 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
       transpose<zc>(W.Yb, W.Ya, (ll)k, (ll)m, s);                          // theta B^H (m x k)
       tri(W.Ya, m, W.Yb);                                                  // U1
     } else {
-      DMRG2_CUDA(cudaMemcpyAsync(W.Yb, W.Ya, sizeof(zc) * (size_t)m * k, cudaMemcpyDeviceToDevice, s));  // U1
+      DMRG2_CUDA(cudaMemcpyAsync(W.Yb, left, sizeof(zc) * (size_t)m * k, cudaMemcpyDeviceToDevice, s));  // U1
     }
     if (mode != WST_SHORT) {
       mulz(true, true, theta, nt, nt, k, m, W.Yb, k, false, W.Ya, k);  // theta^H U1
@@ -157,10 +162,9 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
       mulz(false, false, theta, nt, m, k, nt, W.Yb, k, false, W.Ya, k);  // theta V1
       tri(W.Ya, m, W.Yb);                                                // U2
     }
-    polish(W.Yb, m, W.Ya);                                             // U in Ya
-    mulz(true, true, W.Ya, k, k, nt, m, theta, nt, false, W.Yb, nt);   // right = U^H theta
-    l = W.Ya;
-    r = kept = W.Yb;
+    polish(W.Yb, m, left);
+    mulz(true, true, left, k, k, nt, m, theta, nt, false, right, nt);  // right = U^H theta
+    kept = right;
     nkept = (ll)k * nt;
   } else {
     if (mode != WST_RESUME) {
@@ -176,14 +180,13 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
       tri(W.Ya, nt, W.Yb);                                               // V2
     }
     polish(W.Yb, nt, W.Ya);                                              // V in Ya
-    transpose_conj<zc>(W.Ya, k, nt, k, (zc*)W.Z1, s);                    // right = V^H
-    mulz(false, false, theta, nt, m, k, nt, W.Ya, k, false, W.Yb, k);    // left = theta V
-    r = (const zc*)W.Z1;
-    l = kept = W.Yb;
+    transpose_conj<zc>(W.Ya, k, nt, k, right, s);                        // right = V^H
+    mulz(false, false, theta, nt, m, k, nt, W.Ya, k, false, left, k);    // left = theta V
+    kept = left;
     nkept = (ll)m * k;
   }
   split_finish(theta, (ll)m * nt, kept, nkept, W.status, W.out, W.h_rep, red, s);
-  split_commit(l, left, (ll)m * k, r, right, (ll)k * nt, solve, s);
+  if (solve) split_commit<zc>(left, left_out, (ll)m * k, right, right_out, (ll)k * nt, solve, s);
   if (ev_end) DMRG2_CUDA(cudaEventRecord(ev_end, s));
   DMRG2_CUDA(cudaStreamSynchronize(s));
   if (solved) solved();
