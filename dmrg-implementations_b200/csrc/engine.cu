@@ -1166,6 +1166,8 @@ class Engine final : public EngineBase {
     l.red.part = (double*)al(sizeof(double) * (size_t)l.red.nblk * 2 * (KRYLOV_CAP + 2));
     l.red.counter = (unsigned*)al(sizeof(unsigned) * 4);
     DMRG2_CUDA(cudaMemset(l.red.counter, 0, sizeof(unsigned) * 4));
+    // every counter is zero before the lane's stream, which does not wait for the legacy one
+    DMRG2_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     l.h_svd = (SvdOut*)host_pinned(sizeof(SvdOut));
     DMRG2_CUDA(cudaEventCreate(&l.ev_c));
     DMRG2_CUDA(cudaEventCreate(&l.ev_d));

@@ -262,7 +262,10 @@ __device__ bool lz_finish_step(LanczosDev* st, StepState& sh, int k, int kmax, d
 //   coef0 = V^H w | w -= V coef0, coef1 = V^H w, |w|^2 | w -= V coef1, v_(j+1) = w / |w|
 // (the same classical Gram-Schmidt, applied twice). The norm after the second projection
 // follows from the one before it, |w'|^2 - |coef1|^2 (V is orthonormal to rounding, coef1 is
-// the rounding left by the first projection), so no third barrier is needed, and block 0
+// the rounding left by the first projection, a few eps |H|; the difference is relatively good to
+// eps (1 + |coef1|^2 / beta^2), and beta is above 1e-14 or the solve ends, so |H| would have to
+// reach 1e5 before a beta of pure rounding noise lost half its digits), so no third barrier is
+// needed, and block 0
 // solves the tridiagonal problem while the others finish their slices. Every block sums the
 // partial products itself, in the same fixed order.
 // The barrier: up to LS_CLUSTER blocks are one thread-block cluster (hardware barrier);

@@ -93,6 +93,9 @@ struct LanczosWork {
     owned.push_back(slab.commit());
     DMRG2_CUDA(cudaMemset(red.counter, 0, sizeof(unsigned) * 4));
     DMRG2_CUDA(cudaMemset(st, 0, sizeof(LanczosDev)));
+    // the barrier counters are zero before the solve's own stream, which does not wait for the
+    // legacy one, may count on them
+    DMRG2_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     h_flags = (int*)host_pinned(sizeof(int) * POLL_RING);
     h_st = (LanczosHost*)host_pinned(sizeof(LanczosHost));
     h_seed = (unsigned*)host_pinned(sizeof(unsigned));
