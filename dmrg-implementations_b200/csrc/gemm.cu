@@ -234,6 +234,13 @@ GemmChoice choose(const Gemm<T>& d) {
   const int nt = ST<T>::cplx ? 2 : 3;
   const double rate = ST<T>::cplx ? 16.0 : 64.0;
   const int bk = ST<T>::cplx ? 8 : 16;
+  // Real sums over more k than this go in slices: a rounding error is made against the running value at
+  // each addition, and H_eff's last step at chi = 256 (K = 1280) in one chain left a matvec 7.6e-16 from
+  // the exact result, four slices leave 5.4e-16 at 70.8 us for 69.5 (J1-J2, 171 x 187, K = 1496: 8.7e-16
+  // and 55.0 us in two slices, 7.3e-16 and 53.6 us in eight). A complex product keeps one chain: two
+  // slices would take the Josephson matvec at chi = 128 (K = 512) from 7.0e-16 to 6.1e-16, and from
+  // 151 to 161 us.
+  const int chain_max = ST<T>::cplx ? 1 << 30 : 384;
   const int nb = d.nb1 * d.nb2;
   const double narrow_a = rows16(d.A, d.lda, d.sA1, d.sA2) ? 0.0 : 8.0 / 32;
   const double narrow_b = rows16(d.B, d.ldb, d.sB1, d.sB2) ? 0.0 : 8.0 / 32;
@@ -245,6 +252,7 @@ GemmChoice choose(const Gemm<T>& d) {
       if (sk > 1 && ceil_div(d.K, sk) < 2 * bk) break;  // at least two k tiles per slice
       const int kc = ceil_div(ceil_div(d.K, sk), bk) * bk, ns = ceil_div(d.K, kc);
       if (ns < sk) continue;
+      if (nb == 1 && kc > chain_max && sk < 8) continue;
       const double q = std::ceil(out * ns / 148.0);
       const double f = share[std::min((int)std::min(q, 6.0), tiles[t].occ) - 1];
       const double time = q * (tiles[t].bm * tiles[t].bn * (double)kc / rate / f + (ns > 1 ? 1600.0 : 0.0) +

@@ -40,6 +40,24 @@ def test_gemm_tiles(shape, ta, tb, cplx):
     assert np.all(np.abs(out - (al * (opA @ opB) + be * C0)) <= (2 * K + 8) * EPS * bound)
 
 
+@pytest.mark.parametrize("shape", [(1024, 256, 1280), (684, 187, 1496), (1000, 240, 1200), (700, 250, 1500)])
+def test_long_sums_are_split(shape):
+    """H_eff's last step sums over D chi values. Against one chain of fused multiply-adds over them (formed
+    here, rounded at each addition), slices of at most 384 leave at most sqrt(384 / K) of its error."""
+    M, N, K = shape
+    rng = np.random.default_rng(9)
+    A, B = rng.standard_normal((M, K)), rng.standard_normal((N, K))
+    rows = np.arange(0, M, 37)
+    a, b = A[rows].astype(np.longdouble), B.T.astype(np.longdouble)
+    exact = a @ b
+    chain = np.zeros(exact.shape)
+    for k in range(K):
+        chain = (chain + a[:, k:k + 1] * b[k]).astype(np.float64)
+    err = np.linalg.norm((dmrg2.gemm(A, B, "N", "T")[rows] - exact).astype(np.float64))
+    one = np.linalg.norm((chain - exact).astype(np.float64))
+    assert err <= 1.15 * np.sqrt(384.0 / K) * one  # (15%: the sum over the slices, and the sample)
+
+
 @pytest.mark.parametrize("cplx", [False, True])
 @pytest.mark.parametrize("n", [1, 2, 3, 16, 31, 63, 64, 65, 128, 129])
 def test_exact_split_orders(n, cplx):
