@@ -1665,7 +1665,9 @@ __global__ void copy_cols_conj_kernel(const T* __restrict__ in, ll ldi, int rows
 }
 // out[j][r] = conj(in[r][j]) (j < k)
 template <typename T>
-__global__ void transpose_conj_kernel(const T* __restrict__ in, ll ldi, int rows, int k, T* __restrict__ out) {
+__global__ void transpose_conj_kernel(const T* __restrict__ in, ll ldi, int rows, int k, T* __restrict__ out,
+                                      const int* skip) {
+  if (skip && *((volatile const int*)skip)) return;
   const ll tot = (ll)rows * k;
   for (ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (ll)gridDim.x * blockDim.x) {
     int j = (int)(t / rows);
@@ -1684,14 +1686,14 @@ void copy_cols_conj(const T* in, ll ldi, int rows, int k, T* out, cudaStream_t s
   DMRG2_CHECK_LAUNCH();
 }
 template <typename T>
-void transpose_conj(const T* in, ll ldi, int rows, int k, T* out, cudaStream_t s) {
-  transpose_conj_kernel<T><<<eg_grid((ll)rows * k), 256, 0, s>>>(in, ldi, rows, k, out);
+void transpose_conj(const T* in, ll ldi, int rows, int k, T* out, cudaStream_t s, const int* skip) {
+  transpose_conj_kernel<T><<<eg_grid((ll)rows * k), 256, 0, s>>>(in, ldi, rows, k, out, skip);
   DMRG2_CHECK_LAUNCH();
 }
 template void copy_cols_conj<double>(const double*, ll, int, int, double*, cudaStream_t);
 template void copy_cols_conj<zc>(const zc*, ll, int, int, zc*, cudaStream_t);
-template void transpose_conj<double>(const double*, ll, int, int, double*, cudaStream_t);
-template void transpose_conj<zc>(const zc*, ll, int, int, zc*, cudaStream_t);
+template void transpose_conj<double>(const double*, ll, int, int, double*, cudaStream_t, const int*);
+template void transpose_conj<zc>(const zc*, ll, int, int, zc*, cudaStream_t, const int*);
 
 template void hetrd_cluster<double>(double*, int, ll, double*, double*, double*, cudaStream_t);
 template void hetrd_cluster<zc>(zc*, int, ll, double*, double*, zc*, cudaStream_t);

@@ -738,7 +738,7 @@ class Engine final : public EngineBase {
     // the split is enqueued behind the solve; its own wait covers both, and the sites are written only
     // where the solve left a result
     LanczosResult r = lanczos(i, n, true);
-    svd_split(i, dir, chi, ss, r.pending ? ln().lw.st : nullptr, [&] {
+    svd_split(i, dir, chi, ss, r.pending ? &ln().lw.st->gave_up : nullptr, [&] {
       if (r.pending) lanczos_collect(ln().lw, r, ln().st);
     });
     const double e = lanczos_stats(i, cL, cR, r, ss);
@@ -952,8 +952,9 @@ class Engine final : public EngineBase {
     return te <= te_ref_[i] * (1.0 + WARM_SHORT_SLACK) + 64.0 * 2.220446049250313e-16 * fro2;
   }
 
-  // solve: the state of a deferred solve; solved: throws, once the stream has run it, where it left no result
-  void svd_split(int i, char dir, int chi, SweepStats& ss, const LanczosDev* solve,
+  // skip: the gave_up flag of a deferred solve; solved: throws, once the stream has run it, where it
+  // left no result
+  void svd_split(int i, char dir, int chi, SweepStats& ss, const int* skip,
                  const std::function<void()>& solved) {
     const int cL = dims_[i], cR = dims_[i + 2];
     const ll m = (ll)cL * d_, nc = (ll)d_ * cR;
@@ -967,10 +968,10 @@ class Engine final : public EngineBase {
           bool done;
           if constexpr (ST<T>::cplx)
             done = wst_split_c(ln().wstc, ln().red, ln().theta, (int)m, (int)nc, dir, k, warm, mps_[i], mps_[i + 1], te,
-                               ln().st, mode, ln().ev_d, solve, solved);
+                               ln().st, mode, ln().ev_d, skip, solved);
           else
             done = wst_split(ln().wst, ln().red, ln().theta, (int)m, (int)nc, dir, k, warm, mps_[i], mps_[i + 1], te,
-                             ln().st, mode, cfg_.graphs, ln().ev_d, solve, solved);
+                             ln().st, mode, cfg_.graphs, ln().ev_d, skip, solved);
           return done && warm_split_keeps_rank(k, chi, m, nc, te, warm_fro2());
         };
         bool ok = false, short_kept = false;

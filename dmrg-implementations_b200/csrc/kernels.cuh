@@ -154,7 +154,7 @@ void eig_truncate(const double* d, const double* lam, int n, int K, int chi_max,
 template <typename T>
 void copy_cols_conj(const T* in, ll ldi, int rows, int k, T* out, cudaStream_t s);
 template <typename T>
-void transpose_conj(const T* in, ll ldi, int rows, int k, T* out, cudaStream_t s);
+void transpose_conj(const T* in, ll ldi, int rows, int k, T* out, cudaStream_t s, const int* skip = nullptr);
 
 // ---------------------------------------------------------------- warm-started split
 // What the host needs of a split, in page-locked host memory.
@@ -170,10 +170,9 @@ template <typename T>
 void split_finish(const T* theta, ll nt, const T* kept, ll nk, const int* status, const SvdOut* out, SplitHost* host,
                   RedScratch& r, cudaStream_t s);
 
-// left <- l (nl elements) and right <- r (nr), unless the solve whose vector was split (solve, when given)
-// left no result: the sites then stay as they are
+// left <- l (nl elements) and right <- r (nr), unless *skip
 template <typename T>
-void split_commit(const T* l, T* left, ll nl, const T* r, T* right, ll nr, const LanczosDev* solve, cudaStream_t s);
+void split_commit(const T* l, T* left, ll nl, const T* r, T* right, ll nr, const int* skip, cudaStream_t s);
 
 // ---------------------------------------------------------------- misc
 template <typename T>

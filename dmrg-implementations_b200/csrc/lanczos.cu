@@ -1151,8 +1151,8 @@ void split_finish(const T* theta, ll nt, const T* kept, ll nk, const int* status
 template <typename T>
 __global__ void __launch_bounds__(256)
     split_commit_kernel(const T* __restrict__ l, T* __restrict__ left, ll nl, const T* __restrict__ r,
-                        T* __restrict__ right, ll nr, const LanczosDev* solve) {
-  if (solve && (solve->gave_up || !solve->done || solve->n_iter < 1)) return;
+                        T* __restrict__ right, ll nr, const int* skip) {
+  if (skip && *((volatile const int*)skip)) return;
   const ll step = (ll)gridDim.x * blockDim.x, t0 = (ll)blockIdx.x * blockDim.x + threadIdx.x;
 #pragma unroll 4
   for (ll i = t0; i < nl; i += step) left[i] = l[i];
@@ -1161,9 +1161,9 @@ __global__ void __launch_bounds__(256)
 }
 
 template <typename T>
-void split_commit(const T* l, T* left, ll nl, const T* r, T* right, ll nr, const LanczosDev* solve, cudaStream_t s) {
+void split_commit(const T* l, T* left, ll nl, const T* r, T* right, ll nr, const int* skip, cudaStream_t s) {
   const int g = (int)std::min<ll>(4 * STEP_BLOCKS, std::max<ll>(1, (std::max(nl, nr) + 511) / 512));
-  split_commit_kernel<T><<<g, 256, 0, s>>>(l, left, nl, r, right, nr, solve);
+  split_commit_kernel<T><<<g, 256, 0, s>>>(l, left, nl, r, right, nr, skip);
   DMRG2_CHECK_LAUNCH();
 }
 
@@ -1195,7 +1195,7 @@ void scale_inplace(T* x, ll n, const double* nrm2_dev, cudaStream_t s) {
   template void lz_ritz<T>(const T*, ll, T*, LanczosDev*, RedScratch&, LanczosHost*, cudaStream_t); \
   template void split_finish<T>(const T*, ll, const T*, ll, const int*, const SvdOut*, SplitHost*, \
                                 RedScratch&, cudaStream_t);                                       \
-  template void split_commit<T>(const T*, T*, ll, const T*, T*, ll, const LanczosDev*, cudaStream_t); \
+  template void split_commit<T>(const T*, T*, ll, const T*, T*, ll, const int*, cudaStream_t);        \
   template void norm2<T>(const T*, ll, double*, RedScratch&, cudaStream_t);                       \
   template void scale_inplace<T>(T*, ll, const double*, cudaStream_t);
 INST(double)

@@ -202,8 +202,8 @@ void lz_build_graph(LanczosWork<T>& W, GraphEntry& G, T* theta, ll n, int kmax, 
 // vector on exit. With a key: the device-looped form, cached in W.graphs (the key must
 // identify everything the matvec reads and writes besides in and out). With defer, a
 // device-looped solve without restarts is only enqueued (res.pending): the caller enqueues what
-// follows, waits for the stream and calls lanczos_collect, one host round trip less. What follows must
-// leave nothing behind that a failed solve may not: see split_commit.
+// follows, waits for the stream and calls lanczos_collect, one host round trip less. Until then
+// what follows may write what must outlast a failed solve only where W.st->gave_up is not set.
 template <typename T>
 LanczosResult lanczos_solve(LanczosWork<T>& W, T* theta, ll n, int krylov_max, double tol,
                             int max_restarts, unsigned seed,

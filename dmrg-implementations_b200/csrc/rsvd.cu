@@ -47,7 +47,8 @@ __global__ void embed_pairs_kernel(const zc* __restrict__ Y, ll len, int r, doub
 }
 
 // Q (len x r complex) from the even columns of QR (2 len x 2 r real)
-__global__ void extract_pairs_kernel(const double* __restrict__ QR, ll len, int r, zc* __restrict__ Q) {
+__global__ void extract_pairs_kernel(const double* __restrict__ QR, ll len, int r, zc* __restrict__ Q, const int* skip) {
+  if (skip && *((volatile const int*)skip)) return;
   const ll tot = len * r;
   for (ll t = (ll)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (ll)gridDim.x * blockDim.x) {
     const ll i = t / r;
@@ -79,9 +80,9 @@ void embed_pairs(const zc* Y, ll len, int r, double* YR, cudaStream_t s) {
   DMRG2_CHECK_LAUNCH();
 }
 
-void extract_pairs(const double* QR, ll len, int r, zc* Q, cudaStream_t s) {
+void extract_pairs(const double* QR, ll len, int r, zc* Q, cudaStream_t s, const int* skip) {
   if (len < 1 || r < 1) return;
-  extract_pairs_kernel<<<grid_for(len * r), 256, 0, s>>>(QR, len, r, Q);
+  extract_pairs_kernel<<<grid_for(len * r), 256, 0, s>>>(QR, len, r, Q, skip);
   DMRG2_CHECK_LAUNCH();
 }
 

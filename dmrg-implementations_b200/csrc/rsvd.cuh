@@ -36,7 +36,7 @@ template <typename T>
 void rsvd_omega(T* om, ll n, unsigned long long seed, cudaStream_t s);
 // real embedding of a complex column block and back (see above)
 void embed_pairs(const zc* Y, ll len, int r, double* YR, cudaStream_t s);
-void extract_pairs(const double* QR, ll len, int r, zc* Q, cudaStream_t s);
+void extract_pairs(const double* QR, ll len, int r, zc* Q, cudaStream_t s, const int* skip = nullptr);
 
 template <typename T>
 struct RsvdWork {

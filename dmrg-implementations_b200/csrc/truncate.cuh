@@ -352,9 +352,8 @@ enum WstMode { WST_FULL = 0, WST_SHORT = 1, WST_RESUME = 2 };
 // A (m x k) for 'L'. Writes left (m x k) and right (k x nt) and returns true, or returns
 // false (left / right undefined) when the warm start was not good enough. The host
 // waits once; ev_end, when given, is recorded after the split's kernels. Behind a deferred solve
-// (solve, its state) the factors come out of W.Lout and W.Rout and are copied from there
-// (split_commit: not where the solve left no result); solved, when given, is called after the
-// wait. With graphs on (and a stream other than the legacy default one), the work between the
+// skip is its gave_up flag: the factors come out of W.Lout and W.Rout and are copied from there
+// unless it is set; solved, when given, is called after the wait. With graphs on (and a stream other than the legacy default one), the work between the
 // status reset and those copies is one cached graph per (direction, mode, shapes): the warm factor
 // is copied into W.Win and the factors again come out of W.Lout and W.Rout, so the graph's
 // buffers do not depend on the bond; a key's second call launches the kernels and then captures
@@ -362,7 +361,7 @@ enum WstMode { WST_FULL = 0, WST_SHORT = 1, WST_RESUME = 2 };
 inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, int nt, char dir, int k,
                       const double* warm, double* left, double* right, double& trunc_err, cudaStream_t s,
                       WstMode mode = WST_FULL, bool allow_graph = true, cudaEvent_t ev_end = nullptr,
-                      const LanczosDev* solve = nullptr, const std::function<void()>& solved = nullptr) {
+                      const int* skip = nullptr, const std::function<void()>& solved = nullptr) {
   if (k > W.kmax || m > W.qmax || nt > W.qmax) throw std::runtime_error("wst_split: workspace too small");
   if (std::max(m, nt) > 32 * COLNORM_MAX_CHUNKS) return false;  // longer columns take the exact split
   split_begin(W.status, W.out, k, s);
@@ -418,7 +417,7 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
       warm = W.Win;
     }
   }
-  const bool slots = graph || solve;
+  const bool slots = graph || skip;
   if (slots) {
     left = W.Lout;
     right = W.Rout;
@@ -489,7 +488,7 @@ inline bool wst_split(WstWork& W, RedScratch& red, const double* theta, int m, i
   } else {
     body();
   }
-  if (slots) split_commit(W.Lout, left_out, (ll)m * k, W.Rout, right_out, (ll)k * nt, solve, s);
+  if (slots) split_commit(W.Lout, left_out, (ll)m * k, W.Rout, right_out, (ll)k * nt, skip, s);
   if (ev_end) DMRG2_CUDA(cudaEventRecord(ev_end, s));  // the split's device work ends here
   DMRG2_CUDA(cudaStreamSynchronize(s));
   if (solved) solved();

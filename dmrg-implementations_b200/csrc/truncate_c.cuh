@@ -86,24 +86,25 @@ inline size_t wstc_bytes(ll qmax, ll kmax) {
 // Warm-started split of complex theta (m x nt) at kept rank k; `warm` is B (k x nt) for
 // 'R', A (m x k) for 'L'. Writes left (m x k) and right (k x nt) and returns true, or
 // returns false (left / right undefined) when the warm start was not good enough. The
-// host waits once; ev_end, when given, is recorded after the split's kernels; solve and solved: see
-// wst_split (the slots are parts of the workspace that are free by then).
+// host waits once; ev_end, when given, is recorded after the split's kernels. skip and solved: see wst_split
+// (left and right are written directly, by kernels that return where skip is set).
 inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, int nt, char dir, int k,
                         const zc* warm, zc* left, zc* right, double& trunc_err, cudaStream_t s,
-                        WstMode mode = WST_FULL, cudaEvent_t ev_end = nullptr, const LanczosDev* solve = nullptr,
+                        WstMode mode = WST_FULL, cudaEvent_t ev_end = nullptr, const int* skip = nullptr,
                         const std::function<void()>& solved = nullptr) {
   if (k > W.kmax || m > W.qmax || nt > W.qmax) throw std::runtime_error("wst_split_c: workspace too small");
   if (2 * std::max(m, nt) > 32 * COLNORM_MAX_CHUNKS) return false;  // longer columns take the exact split
   split_begin(W.status, W.out, k, s);
   // complex C (M x N) = op(A) op(B): ta / ca transpose / conjugate A, tb transposes B
   auto mulz = [&](bool ta, bool ca, const zc* A, ll lda, int M, int N, int Kd, const zc* B, ll ldb, bool tb,
-                  zc* C, ll ldc) {
+                  zc* C, ll ldc, const int* no_write = nullptr) {
     Gemm<zc> g;
     g.ta = ta; g.ca = ca; g.tb = tb;
     g.M = M; g.N = N; g.K = Kd;
     g.A = A; g.lda = lda;
     g.B = B; g.ldb = ldb;
     g.C = C; g.ldc = ldc;
+    g.skip = no_write;
     launch_gemm(g, s);
   };
   // real C = alpha op(A) op(B) + beta C on the embeddings
@@ -133,19 +134,14 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
   };
   // one Newton-Schulz step on the embedding of Z (rows x k) unless it is orthonormal already, result
   // into dst; a split whose bound on the step's result (ns_check) is above the tolerance reports a failure
-  auto polish = [&](const zc* Z, ll rows, zc* dst) {
+  auto polish = [&](const zc* Z, ll rows, zc* dst, const int* skip_dst) {
     const ll r2 = 2 * rows;
     embed_pairs(Z, rows, k, W.Z1, s);
     mulr(true, W.Z1, k2, k2, k2, (int)r2, W.Z1, k2, W.S, k2, 1.0, 0.0, nullptr);
     ns_check(W.S, k2, W.out, 4e-16 * (double)r2, W.part, W.counter, s);
     mulr(false, W.Z1, k2, (int)r2, k2, k2, W.S, k2, W.Z2, k2, -0.5, 1.5, &W.out->ns_done, W.Z1);
-    extract_pairs(W.Z2, rows, k, dst, s);
+    extract_pairs(W.Z2, rows, k, dst, s, skip_dst);
   };
-  zc *const left_out = left, *const right_out = right;
-  if (solve) {
-    left = dir == 'R' ? W.Ya : W.Yb;
-    right = dir == 'R' ? W.Yb : (zc*)W.Z1;
-  }
   const zc* kept = nullptr;
   ll nkept = 0;
   if (dir == 'R') {
@@ -162,8 +158,8 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
       mulz(false, false, theta, nt, m, k, nt, W.Yb, k, false, W.Ya, k);  // theta V1
       tri(W.Ya, m, W.Yb);                                                // U2
     }
-    polish(W.Yb, m, left);
-    mulz(true, true, left, k, k, nt, m, theta, nt, false, right, nt);  // right = U^H theta
+    polish(W.Yb, m, left, skip);
+    mulz(true, true, left, k, k, nt, m, theta, nt, false, right, nt, skip);  // right = U^H theta
     kept = right;
     nkept = (ll)k * nt;
   } else {
@@ -179,14 +175,13 @@ inline bool wst_split_c(WstWorkC& W, RedScratch& red, const zc* theta, int m, in
       mulz(true, true, theta, nt, nt, k, m, W.Yb, k, false, W.Ya, k);    // theta^H U1
       tri(W.Ya, nt, W.Yb);                                               // V2
     }
-    polish(W.Yb, nt, W.Ya);                                              // V in Ya
-    transpose_conj<zc>(W.Ya, k, nt, k, right, s);                        // right = V^H
-    mulz(false, false, theta, nt, m, k, nt, W.Ya, k, false, left, k);    // left = theta V
+    polish(W.Yb, nt, W.Ya, nullptr);                                     // V in Ya
+    transpose_conj<zc>(W.Ya, k, nt, k, right, s, skip);                  // right = V^H
+    mulz(false, false, theta, nt, m, k, nt, W.Ya, k, false, left, k, skip);  // left = theta V
     kept = left;
     nkept = (ll)m * k;
   }
   split_finish(theta, (ll)m * nt, kept, nkept, W.status, W.out, W.h_rep, red, s);
-  if (solve) split_commit<zc>(left, left_out, (ll)m * k, right, right_out, (ll)k * nt, solve, s);
   if (ev_end) DMRG2_CUDA(cudaEventRecord(ev_end, s));
   DMRG2_CUDA(cudaStreamSynchronize(s));
   if (solved) solved();
