@@ -19,9 +19,8 @@ configuration's shapes (no dataset is involved).
   solve    = time to solution through the C ABI: the seeded chi=16 state, the ramp
              32/64/128/256 (three sweeps each), then chi=256 until |dE| < 1e-10
 
---impl reference runs the oracle (the reference's numpy two-site sweep loop,
-restated) on the host cores from the same warm chi=256 state, a few bonds per
-step, and reports sweeps/s from the measured per-bond times.
+--impl reference prints that the reference cannot be installed here, and why. Its numpy sweep loop, restated
+(the oracle), is timed on the host cores in the other arm's cpu_baseline.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 """
@@ -48,13 +47,12 @@ CHI = 256
 CUTOFF = 1e-12
 KRYLOV = 30
 RESTARTS = 2
-CPU_BONDS = 14        # bonds of the oracle's sweep in the GPU line's CPU baseline (edge shapes + full width)
-BONDS_PER_STEP = 2    # bonds of the oracle's sweep per step of the reference arm
+CPU_BONDS = 14        # bonds of the oracle's sweep in the CPU baseline (edge shapes + full width)
 METRIC = "sweeps/s (two-site DMRG, Heisenberg L=100, chi=256, FP64 plain form)"
-# DRAM bytes of one H_eff application at chi = 256 (dram__bytes_read.sum + dram__bytes_write.sum
-# over its four kernels: step-1 GEMM, MPO mixing, split-K step-3 GEMM, split-K reduce), from one
-# ncu capture of `python -m dmrg2.microbench heff --chi 256`; the algorithmic bytes are 9.4 MB
-HEFF_TRAFFIC_BYTES_CHI256 = 28.4e6  # ncu DRAM read bytes of the three H_eff kernels at chi=256 (no DRAM writes)
+# DRAM bytes of one H_eff application at chi = 256 (dram__bytes_read.sum + dram__bytes_write.sum over step 1's
+# GEMM 4.75, the MPO mixing 10.50 and step 3's GEMM 13.14 MB, nothing written), from an ncu capture of case
+# matvec_xxz256 of perf/cases.py with its caches flushed; the algorithmic bytes are 9.4 MB
+HEFF_TRAFFIC_BYTES_CHI256 = 28.4e6
 
 
 def workload_config(n_gpus, extra=None):
@@ -388,8 +386,9 @@ def run_ours(args):
         "roofline": {"kernel": "H_eff contraction (FP64 DMMA GEMMs)", "bound": "tensor",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak if peak else None, "traffic": HEFF_TRAFFIC_BYTES_CHI256,
-                     "traffic_note": "DRAM bytes per H_eff application at chi=256 from an ncu capture of the "
-                                     "same kernels; algorithmic bytes 9.4e6 (L, R, theta in and out)",
+                     "traffic_note": "DRAM bytes per H_eff application at chi=256 from an ncu capture (cold "
+                                     "caches) of the same kernels; algorithmic bytes 9.4e6 (L, R, theta in "
+                                     "and out)",
                      "peak_source": "cuBLAS DGEMM 8192^3 (torch.matmul float64) measured in this run; "
                                     "MEASURED_PEAKS.json has no FP64 figure"},
         "time_share": {"heff": heff_s / dev, "svd": svd_s / dev, "other": max(0.0, 1 - (heff_s + svd_s) / dev)},
@@ -397,14 +396,13 @@ def run_ours(args):
                        "eig_fallbacks": eig_fallbacks,
                        "exact_splits": n_sw * 2 * (L_SITES - 1) - warm_splits,
                        "ms_per_bond": 1e3 * svd_s / max(1, n_sw * 2 * (L_SITES - 1))},
-        "dominant_kernel": {"name": "truncation (warm-started subspace split: power half-steps, each with unit "
-                                    "columns and one triangular CholeskyQR pass; the exact density-matrix split "
-                                    "where no warm start applies)",
+        "dominant_kernel": {"name": "truncation (warm-started subspace split: power half-steps, each with one "
+                                    "triangular CholeskyQR pass on the Gram matrix of unit columns; the exact "
+                                    "density-matrix split where no warm start applies)",
                             "share": svd_s / dev, "bound": "latency",
                             "ms_per_bond": 1e3 * svd_s / max(1, n_sw * 2 * (L_SITES - 1)),
-                            "note": "the inverse Cholesky factor of each k x k Gram matrix is a chain of k "
-                                    "dependent pivots in one 8-CTA cluster; no bandwidth or tensor roofline "
-                                    "applies"},
+                            "note": "the tiled Cholesky factor of each k x k Gram matrix is a chain of k dependent "
+                                    "pivots in one 8- or 16-CTA cluster; no bandwidth or tensor roofline applies"},
         "matvecs_per_bond": mv_per_bond,
         "lanczos_graphs": {"device_loops": device_loops, "solves": n_sw * 2 * (L_SITES - 1),
                            "what": "Lanczos solves of the timed sweeps (restarts counted) that ran as one "
@@ -424,53 +422,11 @@ def run_ours(args):
 
 
 def run_reference(args):
-    """The reference's CPU path (the oracle port) on this host's cores, same workload and
-    metric: the warm chi=256 state of the L=100 chain (the GPU warm-up ramp, run before any
-    timing and read back to the host; the oracle's own ramp to chi=256 takes tens of
-    minutes), then the oracle's sweep loop, BONDS_PER_STEP bonds per step. W steps warm
-    up, K steps are timed; value = sweeps/s from the per-bond times over the chain's
-    bond-shape profile (every shape of the chain is run: the left end up to the
-    full-width middle, the right end mirrors the left)."""
-    rank, world, local = dist_env()
-    if rank != 0:
-        return
-    import dmrg2
-    from dmrg2 import models as P
-    mpo = P.xxz(L_SITES)
-    mps = P.random_mps(L_SITES, 2, 16, seed=0)
-    ramp, _ = schedule(args.warmup, 0)
-    eng = dmrg2.DMRG2GPU(L_SITES, 2, CHI, device=local, krylov_max=KRYLOV, max_restarts=RESTARTS,
-                         cutoff=CUTOFF, tol=1e-300, min_sweeps=10 ** 6)
-    eng.set_mpo(mpo)
-    eng.set_mps(mps)
-    eng.run(schedule=ramp)
-    warm = eng.get_mps()
-    eng.close()
-    set_cpu_threads()
-    sw = OracleSweep(mpo, warm, CHI, CUTOFF)
-    for _ in range(args.warmup):
-        sw.run(BONDS_PER_STEP)
-    t0 = time.perf_counter()
-    for _ in range(args.steps):
-        sw.run(BONDS_PER_STEP)
-    t_timed = time.perf_counter() - t0
-    dims = [1] + [a.shape[2] for a in warm]
-    value = 1.0 / sw.sweep_seconds(dims)
-    n_bonds = (args.warmup + args.steps) * BONDS_PER_STEP
-    line = {
-        "metric": METRIC, "value": value, "unit": "sweeps/s", "n_gpus": world, "steps": args.steps,
-        "warmup": args.warmup, "ms_per_step": t_timed / args.steps * 1e3, "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
-        "config": workload_config(world, {"bonds_per_step": BONDS_PER_STEP}), "impl": "reference",
-        "cpu_baseline": {"value": value, "unit": "sweeps/s", "cores": cpu_threads(), "kind": "port",
-                         "sample": f"the oracle's sweep loop (the reference's numpy primitives: eigsh, SVD, "
-                                   f"environment update) over bonds 0..{n_bonds - 1} of a chi={CHI} sweep of the "
-                                   f"L={L_SITES} chain from the warm state, {BONDS_PER_STEP} bonds per step, "
-                                   f"{t_timed:.1f} s timed; sweeps/s from the per-bond times over the chain's "
-                                   f"bond-shape profile"},
-        "e2e": {"value": value, "unit": "sweeps/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-    }
-    print(json.dumps(line))
+    """The reference's own code cannot be installed offline on this image."""
+    if dist_env()[0] == 0:
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "its two-site GPU driver is HIP on rocBLAS/rocSOLVER, its CUDA port needs a system LAPACK, "
+                          "and its Python package imports quimb; none of these is on this image"}))
 
 
 def c2_solve(mpo, mps, device):

@@ -218,7 +218,7 @@ struct GemmChoice {
 // do not start on 16 bytes about 8 cycles per 32 values (twice the copies, half the bytes). Measured against
 // the model's choice, M x N x K: 1280 x 1024 x 256 (64 x 64 tiles: 2.16 CTAs an SM run as
 // three, 35.2 us; 64 x 32 28.9; 32 x 32 26.9), 1024 x 256 x 1280 (64 x 64 tiles in 5 slices
-// 37.1; 4 slices 30.0; 32 x 32 unsplit 28.9), 512 x 128 x 640 (64 x 64 in 8 slices 12.4;
+// 37.1; 4 slices 30.0; 32 x 32 unsplit 28.9, in 3 or 4 slices 32), 512 x 128 x 640 (64 x 64 in 8 slices 12.4;
 // 32 x 32 unsplit 14.5, in 4 slices 8.4), 320 x 256 x 64 (64 x 64 6.4; 32 x 32 4.3).
 struct TileModel {
   int bm, bn;
@@ -280,16 +280,16 @@ void launch_choice(const Gemm<T>& d, const GemmChoice& c, cudaStream_t st) {
 }  // namespace
 
 // ---------------------------------------------------------------- autotuner
-// A single real GEMM of at least TUNE_MIN_FLOP is run in each configuration (every tile
-// with 1, 2, 4 or 8 K slices)
-// the first time its shape (transposes, M, N, K) occurs in the process, on the caller's
-// stream and operands, writing into a scratch output (never the caller's C, no skip
+// A single real GEMM of at least TUNE_MIN_FLOP is run in each configuration (every tile with 1, 2, 4
+// or 8 K slices) the first time its shape (transposes, M, N, K) occurs in the process, on the
+// caller's stream and operands, writing into a scratch output (never the caller's C, no skip
 // flag); the fastest by CUDA events serves every later GEMM of that shape. Smaller GEMMs
-// are latency-bound and keep the model's choice: their many distinct shapes (chain ends, bond-dimension ramps) would cost more to time than
-// a configuration can save. The tuning is off unless DMRG2_GEMM_TUNE=1: measured on the
-// L=100, chi=256 sweep it gains 2% on steady sweeps but loses 10% on a run that starts
-// from a fresh engine (the choices timed in isolation, on L2-resident operands, do not
-// carry over to the sweep's own cache state), and off, results do not depend on timing.
+// are latency-bound and keep the model's choice: their many distinct shapes (chain ends,
+// bond-dimension ramps) would cost more to time than a configuration can save. The tuning is off
+// unless DMRG2_GEMM_TUNE=1: measured on the L=100, chi=256 sweep it gains 2% on steady sweeps but
+// loses 10% on a run that starts from a fresh engine (the choices timed in isolation, on
+// L2-resident operands, do not carry over to the sweep's own cache state), and off, results do not
+// depend on timing.
 namespace {
 struct TuneKey {
   int ta, tb, M, N, K, dev;

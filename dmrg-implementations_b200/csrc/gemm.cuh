@@ -32,8 +32,8 @@ struct GemmArgs {
   const int* skip;  // optional device flag: when non-zero the launch does nothing (with Cin: copies it to C)
   const void* Cin;  // the matrix beta multiplies (ld ldc); C itself when null
   int kchunk;       // split-K: blockIdx.z selects the K slice [z*kchunk, (z+1)*kchunk) (0 = off)
-  int kcluster;     // > 1: the K slices of a tile form one thread-block cluster and are summed
-                    // in it, C = alpha sum + beta C written by the cluster (0: partials to C)
+  int kcluster;     // slices of a split K (0 = off): those of a tile form one thread-block cluster
+                    // and are summed in it, C = alpha sum + beta C written by the cluster
 };
 
 __device__ __forceinline__ void cp_async_8(void* smem, const void* gmem, bool pred) {
