@@ -184,10 +184,10 @@ __global__ void __launch_bounds__(G::THREADS) gemm_kernel(GemmArgs g) {
   static_assert(CPLX || NI % 2 == 0, "column pairs");
   pdl_wait();
   if (g.skip && *((volatile const int*)g.skip)) {
-    if (g.Cin && (g.kchunk == 0 || blockIdx.z == 0)) {
+    if (g.Cin) {  // (a single GEMM: the slices of a split K share the tile's copy)
       const T* src = reinterpret_cast<const T*>(g.Cin);
       T* dst = reinterpret_cast<T*>(g.C);
-      for (int e = threadIdx.x; e < BM * BN; e += G::THREADS) {
+      for (int e = blockIdx.z * G::THREADS + threadIdx.x; e < BM * BN; e += gridDim.z * G::THREADS) {
         const int row = blockIdx.y * BM + e / BN, col = blockIdx.x * BN + e % BN;
         if (row < g.M && col < g.N) dst[(ll)row * g.ldc + col] = src[(ll)row * g.ldc + col];
       }
