@@ -212,14 +212,25 @@ struct GemmChoice {
 // Tile and K split by a model of the busiest SM. It runs q = ceil(CTAs / 148) tiles of
 // BM BN K / splitk multiply-adds; the tensor pipe takes 64 (16 complex) a cycle, but only with
 // enough warps resident to cover the latency of a warp's dependent multiply-adds: the
-// measured share of the rate is 0.62 with 4 warps on the SM, 0.82 with 8, 0.86 with 12, 0.90
-// with 16 and 0.92 beyond (L2-resident operands, K from 64 to 1280). A split costs about 1600
-// cycles per CTA of the SM (cluster barrier, exchange of partial tiles); an operand whose rows
-// do not start on 16 bytes about 8 cycles per 32 values (twice the copies, half the bytes). Measured against
-// the model's choice, M x N x K: 1280 x 1024 x 256 (64 x 64 tiles: 2.16 CTAs an SM run as
-// three, 35.2 us; 64 x 32 28.9; 32 x 32 26.9), 1024 x 256 x 1280 (64 x 64 tiles in 5 slices
-// 37.1; 4 slices 30.0; 32 x 32 unsplit 28.9, in 3 or 4 slices 32), 512 x 128 x 640 (64 x 64 in 8 slices 12.4;
-// 32 x 32 unsplit 14.5, in 4 slices 8.4), 320 x 256 x 64 (64 x 64 6.4; 32 x 32 4.3).
+// share of the rate is 0.60 with 4 warps on the SM, 0.82 with 8, 0.86 with 12, 0.90 with 16 and
+// 0.92 beyond (L2-resident operands, K from 64 to 1280). Moving the operands adds 0.05 cycles per row
+// and column and value of k (smaller tiles read them more often), 0.25 where its rows do not start on
+// 16 bytes (twice the copies, half the bytes), and a split 1200 cycles per CTA of the SM and 100
+// more per slice (cluster barrier, exchange of partial tiles). Real constants fitted to 58 shapes of H_eff,
+// environment and split GEMMs at chi = 64 to 512, each measured in all 24 configurations: the choice
+// costs 3.9% over the best one on average (5.6% without the operands' term and with 1600 cycles
+// for any split); complex ones as first measured. Some of them, M x N x K: 1280 x 1024 x 256 (64 x 64
+// tiles: 2.16 CTAs an SM run as three, 35.2 us; 64 x 32 28.9; 32 x 32 26.9), 1024 x 256 x 1280 (64 x 64 in
+// 5 slices 37.1; 4 slices 29.8; 32 x 32 unsplit 30.5, in 4 slices 31.9), 512 x 128 x 640 (64 x 64 in 8
+// slices 11.3; 32 x 32 unsplit 13.9, in 4 slices 7.7), 320 x 256 x 64 (64 x 64 6.4; 32 x 32 4.3).
+//
+// Long real sums: a rounding error is made against the running value at each addition, and H_eff's
+// last step at chi = 256 (K = 1280) in one chain left a matvec 7.6e-16 from the exact result, where four
+// slices leave 5.4e-16 (J1-J2, 171 x 187, K = 1496: two slices 8.7e-16, eight 7.3e-16). So sums over more than
+// 512 values go in slices of at most 384, where the output has fewer 64 x 64 tiles than there are SMs
+// (a larger one loses up to 15% to the exchange: 1024^3 79.9 us unsplit, 91.8 in 4 slices). A
+// complex product keeps its chain: two slices would take the Josephson matvec at chi = 128 (K = 512)
+// from 7.0e-16 to 6.1e-16, and from 151 to 161 us.
 struct TileModel {
   int bm, bn;
   int occ;  // CTAs an SM holds (four warps each)
@@ -229,21 +240,17 @@ constexpr TileModel TILES_Z[] = {{64, 32, 4}, {32, 32, 6}};
 
 template <typename T>
 GemmChoice choose(const Gemm<T>& d) {
-  constexpr double share[] = {0.62, 0.82, 0.86, 0.90, 0.92, 0.92};
+  constexpr bool real = !ST<T>::cplx;
+  constexpr double share[] = {real ? 0.60 : 0.62, 0.82, 0.86, 0.90, 0.92, 0.92};
+  constexpr double move = real ? 0.05 : 0.0, split_cta = real ? 1200.0 : 1600.0, split_slice = real ? 100.0 : 0.0;
   const TileModel* tiles = ST<T>::cplx ? TILES_Z : TILES_D;
   const int nt = ST<T>::cplx ? 2 : 3;
   const double rate = ST<T>::cplx ? 16.0 : 64.0;
   const int bk = ST<T>::cplx ? 8 : 16;
-  // Real sums over more k than this go in slices: a rounding error is made against the running value at
-  // each addition, and H_eff's last step at chi = 256 (K = 1280) in one chain left a matvec 7.6e-16 from
-  // the exact result, four slices leave 5.4e-16 at 70.8 us for 69.5 (J1-J2, 171 x 187, K = 1496: 8.7e-16
-  // and 55.0 us in two slices, 7.3e-16 and 53.6 us in eight). A complex product keeps one chain: two
-  // slices would take the Josephson matvec at chi = 128 (K = 512) from 7.0e-16 to 6.1e-16, and from
-  // 151 to 161 us.
-  const int chain_max = ST<T>::cplx ? 1 << 30 : 384;
   const int nb = d.nb1 * d.nb2;
   const double narrow_a = rows16(d.A, d.lda, d.sA1, d.sA2) ? 0.0 : 8.0 / 32;
   const double narrow_b = rows16(d.B, d.ldb, d.sB1, d.sB2) ? 0.0 : 8.0 / 32;
+  const bool slices = real && nb == 1 && d.K > 512 && ceil_div(d.M, 64) * (ll)ceil_div(d.N, 64) < 148;
   GemmChoice best{0, 1};
   double best_t = 1e300;
   for (int t = 0; t < nt; ++t) {
@@ -252,11 +259,12 @@ GemmChoice choose(const Gemm<T>& d) {
       if (sk > 1 && ceil_div(d.K, sk) < 2 * bk) break;  // at least two k tiles per slice
       const int kc = ceil_div(ceil_div(d.K, sk), bk) * bk, ns = ceil_div(d.K, kc);
       if (ns < sk) continue;
-      if (nb == 1 && kc > chain_max && sk < 8) continue;
+      if (slices && kc > 384 && sk < 8) continue;
       const double q = std::ceil(out * ns / 148.0);
       const double f = share[std::min((int)std::min(q, 6.0), tiles[t].occ) - 1];
-      const double time = q * (tiles[t].bm * tiles[t].bn * (double)kc / rate / f + (ns > 1 ? 1600.0 : 0.0) +
-                               kc * (narrow_a * tiles[t].bm + narrow_b * tiles[t].bn));
+      const double time = q * (tiles[t].bm * tiles[t].bn * (double)kc / rate / f +
+                               (ns > 1 ? split_cta + split_slice * ns : 0.0) +
+                               kc * ((narrow_a + move) * tiles[t].bm + (narrow_b + move) * tiles[t].bn));
       if (time < best_t) {
         best_t = time;
         best = {t, ns};

@@ -43,7 +43,8 @@ def test_gemm_tiles(shape, ta, tb, cplx):
 @pytest.mark.parametrize("shape", [(1024, 256, 1280), (684, 187, 1496), (1000, 240, 1200), (700, 250, 1500)])
 def test_long_sums_are_split(shape):
     """H_eff's last step sums over D chi values. Against one chain of fused multiply-adds over them (formed
-    here, rounded at each addition), slices of at most 384 leave at most sqrt(384 / K) of its error."""
+    here, rounded at each addition), slices of at most 384 leave at most sqrt(384 / K) of its error (outputs
+    of fewer 64 x 64 tiles than SMs)."""
     M, N, K = shape
     rng = np.random.default_rng(9)
     A, B = rng.standard_normal((M, K)), rng.standard_normal((N, K))
