@@ -50,7 +50,7 @@ RESTARTS = 2
 CPU_BONDS = 14        # bonds of the oracle's sweep in the CPU baseline (edge shapes + full width)
 METRIC = "sweeps/s (two-site DMRG, Heisenberg L=100, chi=256, FP64 plain form)"
 # DRAM bytes of one H_eff application at chi = 256 (dram__bytes_read.sum + dram__bytes_write.sum over step 1's
-# GEMM 4.75, the MPO mixing 10.50 and step 3's GEMM 13.14 MB, nothing written), from an ncu capture of case
+# GEMM 4.75, the MPO mixing 10.50 and step 3's GEMM 13.15 MB, nothing written), from an ncu capture of case
 # matvec_xxz256 of perf/cases.py with its caches flushed; the algorithmic bytes are 9.4 MB
 HEFF_TRAFFIC_BYTES_CHI256 = 28.4e6
 
